@@ -623,10 +623,13 @@ static int run_rhs(dnsbox_ctx *c, const void *uin, int mode, void *out, void *st
   }
   CK(cudaGetLastError());
   const char *u = reinterpret_cast<const char *>(uin);
+  // pruned passes on the SIMT kernel keep the workspace in compact rows
+  const bool compact = pruned && strided_simt<T>(c);
+  const int wp = ws_pitch(c, compact);
   // pass A: inverse z
   StridedArgs<T> a = strided_base<T>(c, 2);
   a.njobs = 5;
-  strided_ws<T>(c, a, 2, false, true);   // state -> padded workspace
+  strided_ws<T>(c, a, 2, false, true, compact);   // state -> padded workspace
   set_job<T>(a, 0, cfield(u, c, 0), wfield(c->W1, c, 0));
   set_job<T>(a, 1, cfield(u, c, 1), wfield(c->W1, c, 1));
   set_job<T>(a, 2, cfield(u, c, 2), wfield(c->W1, c, 2));
@@ -640,7 +643,7 @@ static int run_rhs(dnsbox_ctx *c, const void *uin, int mode, void *out, void *st
   RET(run_strided<T>(c, 2, true, a, DNSBOX_PASS_Z_INV, true, uin, 3));
   // pass B: inverse y
   StridedArgs<T> b = strided_base<T>(c, 1);
-  strided_ws<T>(c, b, 1, true, true);
+  strided_ws<T>(c, b, 1, true, true, compact);
   b.njobs = 6;
   set_job<T>(b, 0, wfield(c->W1, c, 0), wfield(c->W2, c, 0));
   set_job<T>(b, 1, wfield(c->W1, c, 1), wfield(c->W2, c, 1));
@@ -666,7 +669,8 @@ static int run_rhs(dnsbox_ctx *c, const void *uin, int mode, void *out, void *st
   x.NX = reinterpret_cast<C *>(wfield(c->W1, c, 0));
   x.NY = reinterpret_cast<C *>(wfield(c->W1, c, 1));
   x.NZ = reinterpret_cast<C *>(wfield(c->W1, c, 2));
-  x.pin = x.pout = c->wp;
+  x.pin = x.pout = wp;
+  if (compact) x.nyq = c->keep[0].a;
   x.status = c->tc_status;
   x.tw = reinterpret_cast<const C *>(c->tw[0]);
   x.st = c->st;
@@ -692,7 +696,7 @@ static int run_rhs(dnsbox_ctx *c, const void *uin, int mode, void *out, void *st
   }
   // pass D: forward y
   StridedArgs<T> d = strided_base<T>(c, 1);
-  strided_ws<T>(c, d, 1, true, true);
+  strided_ws<T>(c, d, 1, true, true, compact);
   d.njobs = 3;
   for (int f = 0; f < 3; ++f) set_job<T>(d, f, wfield(c->W1, c, f), wfield(c->W2, c, f));
   if (pruned) {   // only kept kx columns; ky rows outside the kept set are masked by the finish
@@ -703,7 +707,7 @@ static int run_rhs(dnsbox_ctx *c, const void *uin, int mode, void *out, void *st
   // pass E1: forward z of the three components, in place (the SIMT kernel in
   // every form); pruned: kept kx columns and ky tiles, kept kz rows written
   StridedArgs<T> z = strided_base<T>(c, 2);
-  strided_ws<T>(c, z, 2, true, true);
+  strided_ws<T>(c, z, 2, true, true, compact);
   z.njobs = 3;
   for (int f = 0; f < 3; ++f) set_job<T>(z, f, wfield(c->W2, c, f), wfield(c->W2, c, f));
   if (pruned) {
@@ -715,9 +719,10 @@ static int run_rhs(dnsbox_ctx *c, const void *uin, int mode, void *out, void *st
   // pass E2: spectral finish, one warp per (kz, ky) row
   FinishArgs<T> e = finish_base<T>(c);
   e.n3 = reinterpret_cast<const C *>(c->W2);
-  e.n3_pitch = c->wp;
+  e.n3_pitch = wp;
+  e.n3_nyq = compact ? c->keep[0].a : 0;
   e.n3_nh = (long long)c->wstride;
-  e.n3_bstride = (long long)p.nz * p.ny * c->wp;
+  e.n3_bstride = (long long)p.nz * p.ny * wp;
   e.uin = reinterpret_cast<const C *>(uin);
   e.out = reinterpret_cast<C *>(out);
   e.state = reinterpret_cast<C *>(state);
@@ -1708,9 +1713,9 @@ extern "C" int dnsbox_upload_physical(dnsbox_ctx *ctx, const double *host, void 
   void *out[3];
   char *src = ctx->W2;
   if (!ctx->fp64) {
-    // convert to float into W1 slots 3-5 (each holds nh*8 B >= np*4 B)
+    // convert to float into W1's padded slots 3-5, past those the R2C writes (each holds nh*8 B >= np*4 B)
     for (int c = 0; c < 3; ++c) {
-      float *dst = reinterpret_cast<float *>(field(ctx->W1, ctx, 3 + c));
+      float *dst = reinterpret_cast<float *>(wfield(ctx->W1, ctx, 3 + c));
       k_convert<double, float><<<grid_for((long long)ctx->np), 256, 0, ctx->stream>>>(
           reinterpret_cast<const double *>(src + c * pbytes), dst, (long long)ctx->np);
       in[c] = dst;

@@ -268,13 +268,28 @@ static inline char *wfield(char *base, const dnsbox_ctx *c, int slot) {
   return base + (size_t)slot * c->wstride * c->cbytes;
 }
 
+// Whether a right-hand side runs its four strided passes on the SIMT kernel,
+// which reads and writes the workspace in compact rows when pruned.
+template <typename T> static bool strided_simt(const dnsbox_ctx *c);
+
+// Row pitch of the workspace fields: wp, or the compact pitch of pruned rows.
+static inline int ws_pitch(const dnsbox_ctx *c, bool compact) {
+  const int q = c->fp64 ? 8 : 16;   // complex elements per 128 bytes
+  return compact ? (c->keep[0].a + 1 + q - 1) / q * q : c->wp;
+}
+
 // Sets the input (in_ws) and output (out_ws) strides of a strided pass along
 // `axis` (2: z, 1: y) to the padded workspace layout; the other side keeps
-// the state layout of strided_base.
+// the state layout of strided_base.  compact: pruned columns only, the Nyquist
+// column in slot keep[0].a.
 template <typename T> static void strided_ws(const dnsbox_ctx *c, StridedArgs<T> &a, int axis, bool in_ws,
-                                             bool out_ws) {
-  const long long wp = c->wp, plane = (long long)c->p.ny * wp, box = plane * c->p.nz;
+                                             bool out_ws, bool compact = false) {
+  const long long wp = ws_pitch(c, compact), plane = (long long)c->p.ny * wp, box = plane * c->p.nz;
   const long long rs = axis == 2 ? plane : wp, os = axis == 2 ? wp : plane;
+  a.ws = (in_ws ? 1 : 0) | (out_ws ? 2 : 0);
+  a.compact = compact;
+  const int sec = 32 / (int)(2 * sizeof(T)), ns = compact ? c->keep[0].a + 1 : c->nxh;
+  a.nslot = (ns + sec - 1) / sec * sec;   // whole 32-byte sectors
   if (in_ws) {
     a.rowstride = rs;
     a.otherstride = os;
@@ -374,7 +389,10 @@ static int run_strided(dnsbox_ctx *c, int axis, bool inv, StridedArgs<T> a, int 
   const bool simt = si >= 0 && si < 3 && c->sched_tc[si] == 2;
   const bool tc = allow_tc && c->tc && Ops<T>::has_tc(n) && !simt;
   const int width = tc ? 4096 / n : TileCols<T>::v;
-  if (a.kcol.a) {
+  if (a.kcol.a && a.compact) {   // slots [0, kcol.a], the Nyquist column last
+    a.ntx_lo = (a.nslot + width - 1) / width;
+    a.nyq_tile = -1;
+  } else if (a.kcol.a) {
     a.ntx_lo = (a.kcol.a + width - 1) / width;
     const int nt = (c->p.nx / 2) / width;
     // 0: the Nyquist column lies in the low tiles; < 0: it takes the free slot
@@ -393,6 +411,14 @@ static int run_strided(dnsbox_ctx *c, int axis, bool inv, StridedArgs<T> a, int 
   }
   CK(Ops<T>::strided(n, a, inv, ntiles, c->stream));
   return DNSBOX_OK;
+}
+
+template <typename T> static bool strided_simt(const dnsbox_ctx *c) {
+  if (!c->tc) return true;
+  const int n[3] = {c->p.nz, c->p.ny, c->p.ny};   // passes A, B, D
+  for (int i = 0; i < 3; ++i)
+    if (c->sched_tc[i] != 2 && Ops<T>::has_tc(n[i])) return false;
+  return c->sched_tc[3] == 0;
 }
 
 // One output of a batched C2R: sum over terms of in * (a + i b k), with k
@@ -415,24 +441,27 @@ static int c2r_jobs(dnsbox_ctx *c, int nf, const SpecJob *jobs, void *const *out
   for (int f0 = 0; f0 < nf; f0 += 6) {
     const int m = nf - f0 < 6 ? nf - f0 : 6;
     StridedArgs<T> a = strided_base<T>(c, 2);
+    strided_ws<T>(c, a, 2, false, true);   // padded rows between the passes
     a.njobs = m;
     for (int j = 0; j < m; ++j) {
       const SpecJob &J = jobs[f0 + j];
-      set_job<T>(a, j, J.t[0].in, field(c->W1, c, j), J.t[0].a, J.t[0].b, J.t[0].ks,
+      set_job<T>(a, j, J.t[0].in, wfield(c->W1, c, j), J.t[0].a, J.t[0].b, J.t[0].ks,
                  J.nt > 1 ? J.t[1].in : nullptr, J.nt > 1 ? J.t[1].a : 1.0, J.nt > 1 ? J.t[1].b : 0.0,
                  J.nt > 1 ? J.t[1].ks : 0);
     }
     RET(run_strided<T>(c, 2, true, a));
     StridedArgs<T> b = strided_base<T>(c, 1);
+    strided_ws<T>(c, b, 1, true, true);
     b.njobs = m;
-    for (int j = 0; j < m; ++j) set_job<T>(b, j, field(c->W1, c, j), field(c->W2, c, j));
+    for (int j = 0; j < m; ++j) set_job<T>(b, j, wfield(c->W1, c, j), wfield(c->W2, c, j));
     RET(run_strided<T>(c, 1, true, b));
     XlineArgs<T> x;
     memset(&x, 0, sizeof(x));
     for (int j = 0; j < m; ++j) {
-      x.in[j] = field(c->W2, c, j);
+      x.in[j] = wfield(c->W2, c, j);
       x.out[j] = out[f0 + j];
     }
+    x.pitch = c->wp;
     x.tw = reinterpret_cast<const typename CT<T>::type *>(c->tw[0]);
     x.nlines = c->p.ny * c->p.nz;
     x.nxh = c->nxh;
@@ -461,8 +490,9 @@ static int r2c_fields(dnsbox_ctx *c, int nf, const void *const *in, void *const 
     memset(&x, 0, sizeof(x));
     for (int j = 0; j < m; ++j) {
       x.in[j] = in[f0 + j];
-      x.out[j] = field(c->W1, c, j);
+      x.out[j] = wfield(c->W1, c, j);
     }
+    x.pitch = c->wp;
     x.tw = reinterpret_cast<const typename CT<T>::type *>(c->tw[0]);
     x.nlines = c->p.ny * c->p.nz;
     x.nxh = c->nxh;
@@ -472,12 +502,14 @@ static int r2c_fields(dnsbox_ctx *c, int nf, const void *const *in, void *const 
       CK(Ops<T>::xline_r2c(c->p.nx, x, m, c->stream));
     }
     StridedArgs<T> b = strided_base<T>(c, 1);
+    strided_ws<T>(c, b, 1, true, true);
     b.njobs = m;
-    for (int j = 0; j < m; ++j) set_job<T>(b, j, field(c->W1, c, j), field(c->W2, c, j));
+    for (int j = 0; j < m; ++j) set_job<T>(b, j, wfield(c->W1, c, j), wfield(c->W2, c, j));
     RET(run_strided<T>(c, 1, false, b));
     StridedArgs<T> a = strided_base<T>(c, 2);
+    strided_ws<T>(c, a, 2, true, false);
     a.njobs = m;
-    for (int j = 0; j < m; ++j) set_job<T>(a, j, field(c->W2, c, j), out[f0 + j]);
+    for (int j = 0; j < m; ++j) set_job<T>(a, j, wfield(c->W2, c, j), out[f0 + j]);
     RET(run_strided<T>(c, 2, false, a));
   }
   return DNSBOX_OK;

@@ -19,6 +19,7 @@
 
 #include "common.cuh"
 #include "fft.cuh"
+#include "fftv.cuh"
 
 namespace dnsbox {
 
@@ -102,6 +103,10 @@ template <typename T> struct StridedArgs {
   // strides of the output when its row pitch differs from the input's (the
   // padded workspace fields of a right-hand side); 0: the input's
   long long rowstride_o, otherstride_o, bstride_o;
+  // which sides are padded workspace fields (1: input, 2: output), whose rows
+  // of nslot columns start on 128-byte boundaries; with column pruning the
+  // workspace is compact: slot kcol.a holds the Nyquist column (compact = 1)
+  int ws, compact, nslot, pad;
 };
 
 // Output strides of a strided launch (the input's where unset).
@@ -129,28 +134,25 @@ __host__ __device__ __forceinline__ int strided_col(const StridedArgs<T> &a, int
   return (a.nyq_tile < 0 && kx == a.kcol.a) ? (a.kcol.n >> 1) : kx;
 }
 
-// Columns per CTA of the SIMT strided kernel: the host's tile width, or at
-// N >= 512 (plans of 64 threads per column) half a tile, so that a CTA has
-// 512 (FP32) or 256 (FP64) threads and several CTAs share an SM, each with
-// its own barriers; in FP32 at every size (at 256: 128-thread CTAs, eight per
-// SM, 5% off the inverse y pass at 256^3; at 96 the pruned 34-column grid
-// wastes 6 columns instead of 14, 3% off the 96^3 strided passes; the FP64
-// kernel below 512 keeps its tile).
-template <typename T, int N> struct StridedCols {
-  static constexpr int v = (N >= 512 || sizeof(T) == 4) ? TileCols<T>::v / 2 : TileCols<T>::v;
-};
-
-// Resident CTAs of a strided launch to ask the register allocator for: FP32
-// blocks of up to 256 threads whose plans hold at most 16 values a thread
-// are held to 64 registers a thread (the load-latency-bound passes gain more
-// from the extra warps than they lose to the tighter allocation), 512-thread
-// FP32 blocks to two per SM and the 256-thread FP64 blocks of N = 512 to
-// three (80 registers, a few spills: 24% off the inverse y pass at 512^3);
-// 0 leaves the choice to the compiler.
-template <typename T, int N> struct StridedMinCtas {
-  static constexpr int NT = round32(StridedCols<T, N>::v * (N / FftPlan<N>::E));
-  static constexpr int v = (sizeof(T) == 4 && NT <= 256 && FftPlan<N>::E <= 16) ? 1024 / NT
-                         : (sizeof(T) == 4 && NT == 512) ? 2 : (sizeof(T) == 8 && N == 512) ? 3 : 0;
+// Shape of a strided block: 8 threads across the columns, each with one 16-byte
+// element per row (a complex double, or two neighbouring single-precision
+// columns), so a row segment of a tile is 128 bytes; P threads along the rows.
+template <typename T, int N> struct StridedShape {
+  using PL = VPlan<N>;
+  static constexpr int W = 8;
+  static constexpr int NT = W * PL::P;
+  static constexpr size_t tile = PL::NST > 1 ? (size_t)N * W * 16 : 0;
+  static constexpr size_t smem(bool inv) {   // tile, twiddles and (inverse) row multipliers
+    return tile + (size_t)vtw_size<PL>() * 16 + (inv ? 2 * N * sizeof(T) : 0);
+  }
+  // Resident CTAs asked of the register allocator: 16 warps per SM where a
+  // thread holds 16 values (128 registers), 20 at 12 (96), 24 at 8 (80), 32 in
+  // the 512-thread blocks of N = 512 (64).  The 256-row pass with 8 values,
+  // three stages and 32 warps measured the same (57.7 against 56.7 us for pass
+  // D): the loads in flight per SM are equal.
+  static constexpr int warps = PL::E >= 16 ? 16 : PL::E == 12 ? 20 : N >= 512 ? 32 : 24;
+  static constexpr int wcta = round32(NT) / 32;
+  static constexpr int minb = warps / wcta < 1 ? 1 : warps / wcta;
 };
 
 // Column origin and other-axis index of tile t of the (possibly pruned) grid.
@@ -162,114 +164,216 @@ __device__ __forceinline__ void strided_tile(const StridedArgs<T> &a, int tile, 
   other = a.koth.map(o);
 }
 
-template <typename T, typename C>
-__device__ __forceinline__ C apply_mult(C v, double a, double b, double k) {
-  // v * (a + i b k)
-  const T bk = T(b * k), aa = T(a);
-  return mkc<C>(v.x * aa - v.y * bk, v.y * aa + v.x * bk);
+// Tile addressing: rows of 8 elements of 16 bytes (128 bytes), so the eight
+// lanes of a quarter warp, one row's columns, cover all banks once.
+struct AddrRows8 {
+  __device__ static __forceinline__ int at(int row, int col) { return row * 8 + col; }
+};
+
+// One 16-byte element from / to memory (zero where !on): an aligned 16-byte
+// word, or (single precision) two columns one by one.  The loads are volatile,
+// so that a thread's rows are all requested before the first is used.
+template <typename C> struct StridedIO;
+template <> struct StridedIO<double2> {
+  using Raw = VC<double>;
+  __device__ static __forceinline__ Raw load(const double2 *p, bool on) {
+    Raw x{0.0, 0.0};
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q ld.global.v2.f64 {%0, %1}, [%2];\n\t}"
+                 : "+d"(x.re), "+d"(x.im)
+                 : "l"(p), "r"((unsigned)on));
+    return x;
+  }
+  __device__ static __forceinline__ void store(double2 *p, Raw v) { *p = make_double2(v.re, v.im); }
+  // x (a + i b)
+  __device__ static __forceinline__ Raw mul(Raw x, double a, double b, double) {
+    return Raw{x.re * a - x.im * b, x.im * a + x.re * b};
+  }
+  __device__ static __forceinline__ Raw add(Raw x, Raw y) { return Raw{x.re + y.re, x.im + y.im}; }
+};
+template <> struct StridedIO<float2> {
+  using Raw = Raw2;
+  __device__ static __forceinline__ Raw load(const float2 *p, bool on) {
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t@q ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+        : "+f"(x.x), "+f"(x.y), "+f"(x.z), "+f"(x.w)
+        : "l"(p), "r"((unsigned)on));
+    return Raw{x};
+  }
+  __device__ static __forceinline__ Raw load2(const float2 *p0, const float2 *p1, bool v0, bool v1) {
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q ld.global.v2.f32 {%0, %1}, [%2];\n\t}"
+                 : "+f"(x.x), "+f"(x.y)
+                 : "l"(p0), "r"((unsigned)v0));
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q ld.global.v2.f32 {%0, %1}, [%2];\n\t}"
+                 : "+f"(x.z), "+f"(x.w)
+                 : "l"(p1), "r"((unsigned)v1));
+    return Raw{x};
+  }
+  __device__ static __forceinline__ void store(float2 *p, Raw v) { *reinterpret_cast<float4 *>(p) = v.q; }
+  __device__ static __forceinline__ void store2(float2 *p0, float2 *p1, Raw v, bool v0, bool v1) {
+    if (v0) *p0 = make_float2(v.q.x, v.q.y);
+    if (v1) *p1 = make_float2(v.q.z, v.q.w);
+  }
+  // x (a + i b0), y (a + i b1) of the two columns
+  __device__ static __forceinline__ Raw mul(Raw x, float a, float b0, float b1) {
+    return Raw{make_float4(x.q.x * a - x.q.y * b0, x.q.y * a + x.q.x * b0, x.q.z * a - x.q.w * b1, x.q.w * a + x.q.z * b1)};
+  }
+  __device__ static __forceinline__ Raw add(Raw x, Raw y) {
+    return Raw{make_float4(x.q.x + y.q.x, x.q.y + y.q.y, x.q.z + y.q.z, x.q.w + y.q.w)};
+  }
+};
+
+// Bit q is set when row p + P q of the axis is kept (q < E).
+template <class PL> __device__ __forceinline__ unsigned keep_mask(const AxisKeep &k, int p) {
+  constexpr int P = PL::P, E = PL::E, N = PL::N;
+  constexpr unsigned all = E == 32 ? 0xffffffffu : (1u << E) - 1u;
+  if (k.a == 0) return all;
+  const int lo = (k.a - p + P - 1) / P;                    // rows below a: q < lo (a >= 1, p < P)
+  unsigned m = lo >= E ? all : (1u << lo) - 1u;
+  if (k.full) {
+    const int t = N - k.a - p;                             // rows above N - a: P q > t
+    const int hi = t < 0 ? 0 : t / P + 1;
+    if (hi < E) m |= all & ~((1u << hi) - 1u);
+  }
+  if ((N / 2 - p) % P == 0 && N / 2 >= p) m |= 1u << ((N / 2 - p) / P);   // the Nyquist row
+  return m;
 }
 
-template <typename T, int N, bool INV>
-__global__ void __launch_bounds__(round32(StridedCols<T, N>::v *(N / FftPlan<N>::E)), StridedMinCtas<T, N>::v)
+// Layouts of a strided pass's two sides.  A workspace side is read and
+// written in whole 16-byte elements over its nslot columns, padding included,
+// so that every 32-byte sector is written whole (a sector written in part
+// costs a read of it when it leaves L2: 57 MB of 219 in pass B at 256^3 FP32);
+// a state side column by column, kept columns only.
+enum StridedMode : int {
+  ST_ANY = 0,      // columns of any layout, one by one
+  ST_TO_WS = 1,    // state -> workspace
+  ST_WS = 2,       // workspace -> workspace
+  ST_FROM_WS = 3,  // workspace -> state
+};
+
+// One strided pass.  A thread holds E rows of one 16-byte element (VPlan), so
+// a row segment of 8 threads is 128 bytes, loads, stores and exchanges are
+// 16-byte instructions, and in single precision the transform runs on packed
+// pairs (fftv.cuh).  Row pruning and the jobs' multipliers concern the inputs
+// of the inverse passes and the outputs of the forward ones only.  With its
+// instructions halved the pass is bound by DRAM and its latency: without the
+// FFT the same loads and stores take 67 / 125 / 56 / 35 us (A, B, D, E1,
+// 256^3 FP32, padded rows with the kept columns first) and the pass takes
+// 76 / 135 / 57 / 39; compact rows, written in whole sectors, bring it to
+// 63 / 111 / 48 / 32 (one 8-byte column per thread: 77 / 148 / 63 / 43), FP64
+// from 111 / 248 / 94 / 67 to 101 / 197 / 75 / 54.
+template <typename T, int N, bool INV, int MODE>
+__global__ void __launch_bounds__(StridedShape<T, N>::NT, StridedShape<T, N>::minb)
     k_strided(const __grid_constant__ StridedArgs<T> a) {
   using C = typename CT<T>::type;
-  using EN = FftEnds<N>;
-  constexpr int TC = StridedCols<T, N>::v;    // columns of this CTA
-  constexpr int SPLIT = TileCols<T>::v / TC;  // CTAs per tile of the host's grid
-  constexpr int E = EN::E;
-  constexpr int NF = TC * (N / E);   // FFT threads: column fastest
+  using SH = StridedShape<T, N>;
+  using PL = typename SH::PL;
+  using EN = VEnds<PL>;
+  using IO = StridedIO<C>;
+  using Raw = typename IO::Raw;
+  using V = VC<typename VecOf<T>::R>;
+  constexpr int E = PL::E, P = PL::P, CPT = VecOf<T>::cols;
+  constexpr bool PAIR = CPT == 2;
+  constexpr bool WSI = MODE == ST_WS || MODE == ST_FROM_WS, WSO = MODE == ST_WS || MODE == ST_TO_WS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C *s = reinterpret_cast<C *>(smem_raw);
-  // block (tile, job, part): the parts of a tile are adjacent blocks, so they
-  // read the two halves of the same 128-byte row segments at about one time
-  const int part = blockIdx.x % SPLIT, tj = blockIdx.x / SPLIT;
-  const int job = tj % a.njobs;
-  const int tile = tj / a.njobs;
+  V *s = reinterpret_cast<V *>(smem_raw);
+  V *twt = reinterpret_cast<V *>(smem_raw + SH::tile);
+  T *bks = reinterpret_cast<T *>(smem_raw + SH::tile + (size_t)vtw_size<PL>() * 16);
+  const int job = blockIdx.x % a.njobs;
+  const int tile = blockIdx.x / a.njobs;
   int kx0, other;
   strided_tile(a, tile, TileCols<T>::v, kx0, other);
-  kx0 += part * TC;
-  // the job's fields, read from the parameter bank once (an indexed
-  // parameter read each time they are used measured as a busy ADU pipe)
-  const C *const in1p = a.job[job].in1, *const in2p = a.job[job].in2;
-  C *const outp = a.job[job].out;
-  const double ja1 = a.job[job].a1, jb1 = a.job[job].b1, ja2 = a.job[job].a2, jb2 = a.job[job].b2;
-  const int ks1 = a.job[job].ks1, ks2 = a.job[job].ks2;
-  const bool act = threadIdx.x < NF;
-  const int col = threadIdx.x % TC, p = threadIdx.x / TC;
-  const int kx = strided_col(a, kx0 + col);
-  const bool valid = act && kx < a.ncols && a.kcol.keep(kx);
-  const long long base = (long long)other * a.otherstride + kx + (long long)blockIdx.y * a.bstride;
-  // FP32: the job's row multipliers T(b k_row(n)) (ks == 1), once per block
-  // instead of once per element (the same values as apply_mult forms; FP64
-  // evaluates them per element, which keeps its kernel at 128 registers)
-  constexpr bool TAB = sizeof(T) == 4;
-  __shared__ T bks[2][TAB ? N : 1];
-  const bool mult1 = !(ja1 == 1.0 && jb1 == 0.0);
-  if (TAB && ((mult1 && ks1 == 1) || (in2p && ks2 == 1))) {
-    for (int n = threadIdx.x; n < N; n += blockDim.x) {
-      const double k = k_full(n, N, a.alpha_row);
-      bks[0][n] = T(jb1 * k);
-      bks[1][n] = T(jb2 * k);
+  const StridedJob<T> &jb = a.job[job];
+  const int col = threadIdx.x % SH::W, p = threadIdx.x / SH::W;
+  // the thread's slot(s) and the modes they hold; v0, v1: kept columns
+  const int s0 = kx0 + CPT * col;
+  const int c0 = strided_col(a, s0), c1 = PAIR ? strided_col(a, s0 + 1) : c0;
+  const bool v0 = c0 < a.ncols && a.kcol.keep(c0);
+  const bool v1 = PAIR && c1 < a.ncols && a.kcol.keep(c1);
+  const bool vs = s0 < a.nslot;
+  const long long base = (long long)other * a.otherstride + (long long)blockIdx.y * a.bstride + (long long)p * a.rowstride +
+                         (WSI ? s0 : c0);
+  const long long step = (long long)P * a.rowstride;
+  const unsigned rin = INV ? keep_mask<PL>(a.krin, p) : 0u;
+  // rows p + P q, q in [Q0, Q0 + QN), of one input into x[0 .. QN)
+  auto load = [&](const C *in, Raw *x, int Q0, int QN) {
+    const C *q0 = in + base + Q0 * step;
+#pragma unroll
+    for (int q = Q0; q < Q0 + QN; ++q, q0 += step) {
+      const bool k = INV ? (rin >> q & 1) : true;
+      if constexpr (WSI || !PAIR) x[q - Q0] = IO::load(q0, (WSI ? vs : v0) && k);
+      else x[q - Q0] = IO::load2(q0, q0 + (c1 - c0), v0 && k, v1 && k);
     }
-    __syncthreads();
+  };
+  Raw v[E];   // row p + P q in v[in_i(q)]
+  {
+    Raw x[E];
+    load(jb.in1, x, 0, E);
+#pragma unroll
+    for (int q = 0; q < E; ++q) v[EN::in_i(q)] = x[q];
   }
-  C v[E];
-  if (valid) {
-    // all E loads of the first stage are independent and issued together
-    const C *in1 = in1p + base;
+  // second inputs: a part of the rows at a time, so that their loads in flight
+  // fit beside the first input's values; the first part right away
+  // (at 512, held to 64 registers, a quarter: all eight rows spill 290 bytes)
+  constexpr int QN = N == 512 ? 2 : E <= 8 ? E : E / 2;
+  const C *const in2p = INV ? jb.in2 : nullptr;
+  Raw w[INV ? QN : 1];
+  if (INV && in2p) load(in2p, w, 0, QN);
+  // with the rows on their way: the twiddle tables (read after the exchange's
+  // barrier) and the job's row multipliers T(b k_row(n)) (ks == 1)
+  vtw_fill<PL, V>(twt, a.tw, threadIdx.x, SH::NT);
+  if constexpr (INV) {
+    const bool mult1 = !(jb.a1 == 1.0 && jb.b1 == 0.0);
+    const bool rows1 = mult1 && jb.ks1 == 1, rows2 = in2p && jb.ks2 == 1;
+    if (rows1 || rows2) {
+      for (int n = threadIdx.x; n < N; n += SH::NT) {
+        const double k = k_full(n, N, a.alpha_row);
+        bks[n] = T(jb.b1 * k);
+        bks[N + n] = T(jb.b2 * k);
+      }
+      __syncthreads();
+    }
+    // the factor b k of a column (ks 0) or of the tile's other-axis index (ks 2)
+    auto colmul = [&](int ks, double b, int c) {
+      return T(b * (ks == 2 ? (a.n_other ? k_full(other, a.n_other, a.alpha_other) : 0.0) : k_half(c, a.nx, a.alpha_x)));
+    };
+    if (mult1) {   // v (a + i b k)
+      const T aa = T(jb.a1), m0 = colmul(jb.ks1, jb.b1, c0), m1 = colmul(jb.ks1, jb.b1, c1);
 #pragma unroll
-    for (int i = 0; i < E; ++i)
-      v[i] = a.krin.keep(EN::in_row(p, i)) ? in1[(long long)EN::in_row(p, i) * a.rowstride] : mkc<C>(0, 0);
-    // wavenumber of the column (0) or of the tile's other-axis index (2)
-    const double kcol = k_half(kx, a.nx, a.alpha_x);
-    const double koth = a.n_other ? k_full(other, a.n_other, a.alpha_other) : 0.0;
-    if constexpr (TAB) {
-      if (mult1) {
-        const T aa = T(ja1), bkc = T(jb1 * (ks1 == 2 ? koth : kcol));
+      for (int q = 0; q < E; ++q) {
+        const T br = rows1 ? bks[p + P * q] : m0;
+        v[EN::in_i(q)] = IO::mul(v[EN::in_i(q)], aa, br, rows1 ? br : m1);
+      }
+    }
+    if (in2p) {
+      const T aa = T(jb.a2), m0 = colmul(jb.ks2, jb.b2, c0), m1 = colmul(jb.ks2, jb.b2, c1);
 #pragma unroll
-        for (int i = 0; i < E; ++i) {
-          const T bk = ks1 == 1 ? bks[0][EN::in_row(p, i)] : bkc;
-          v[i] = mkc<C>(v[i].x * aa - v[i].y * bk, v[i].y * aa + v[i].x * bk);
+      for (int h = 0; h < E / QN; ++h) {
+        if (h) load(in2p, w, h * QN, QN);
+#pragma unroll
+        for (int i = 0; i < QN; ++i) {
+          const T br = rows2 ? bks[N + p + P * (h * QN + i)] : m0;
+          Raw &x = v[EN::in_i(h * QN + i)];
+          x = IO::add(x, IO::mul(w[i], aa, br, rows2 ? br : m1));
         }
       }
-      if (in2p) {
-        const C *in2 = in2p + base;
-        const T aa = T(ja2), bkc = T(jb2 * (ks2 == 2 ? koth : kcol));
+    }
+  }
+  Raw x[E];   // row p + P q in x[out_i(q)]
+  vfft<PL, INV, AddrRows8>(v, x, s, col, p, twt, []() { __syncthreads(); });
+  const unsigned rout = INV ? 0u : keep_mask<PL>(a.krout, p);
+  const long long rso = out_rowstride(a), so = (long long)P * rso;
+  C *o0 = jb.out + (long long)other * out_otherstride(a) + (long long)blockIdx.y * out_bstride(a) + (long long)p * rso +
+          (WSO ? s0 : c0);
 #pragma unroll
-        for (int i = 0; i < E; ++i) {
-          const C w = a.krin.keep(EN::in_row(p, i)) ? in2[(long long)EN::in_row(p, i) * a.rowstride] : mkc<C>(0, 0);
-          const T bk = ks2 == 1 ? bks[1][EN::in_row(p, i)] : bkc;
-          v[i] = cadd(v[i], mkc<C>(w.x * aa - w.y * bk, w.y * aa + w.x * bk));
-        }
-      }
+  for (int q = 0; q < E; ++q, o0 += so) {
+    const bool k = INV ? true : (rout >> q & 1);
+    if constexpr (WSO || !PAIR) {
+      if ((WSO ? vs : v0) && k) IO::store(o0, x[EN::out_i(q)]);
     } else {
-      if (mult1) {
-        const double kc = ks1 == 2 ? koth : kcol;
-#pragma unroll
-        for (int i = 0; i < E; ++i)
-          v[i] = apply_mult<T>(v[i], ja1, jb1, ks1 == 1 ? k_full(EN::in_row(p, i), N, a.alpha_row) : kc);
-      }
-      if (in2p) {
-        const C *in2 = in2p + base;
-        const double kc = ks2 == 2 ? koth : kcol;
-#pragma unroll
-        for (int i = 0; i < E; ++i) {
-          const C w = a.krin.keep(EN::in_row(p, i)) ? in2[(long long)EN::in_row(p, i) * a.rowstride] : mkc<C>(0, 0);
-          v[i] = cadd(v[i], apply_mult<T>(w, ja2, jb2, ks2 == 1 ? k_full(EN::in_row(p, i), N, a.alpha_row) : kc));
-        }
-      }
+      IO::store2(o0, o0 + (c1 - c0), x[EN::out_i(q)], v0 && k, v1 && k);
     }
-  } else {
-#pragma unroll
-    for (int i = 0; i < E; ++i) v[i] = mkc<C>(0, 0);
-  }
-  fft_regs<C, N, INV>(v, s, TC, col, p, act, a.tw);
-  if (valid) {
-    const long long rso = out_rowstride(a);
-    C *out = outp + ((long long)other * out_otherstride(a) + kx + (long long)blockIdx.y * out_bstride(a));
-#pragma unroll
-    for (int i = 0; i < E; ++i)
-      if (a.krout.keep(EN::out_row(p, i))) out[(long long)EN::out_row(p, i) * rso] = v[i];
   }
 }
 
@@ -284,6 +388,7 @@ template <typename T> struct XlineNLArgs {
   int lines_per_box;                   // ny * nz
   int kxa;                             // pruning: only kx < kxa and kx = N/2 are read and written (0: all)
   int pin, pout;                       // row pitch (complex elements) of the inputs / outputs; 0: nxh
+  int nyq;                             // slot of the Nyquist column in a row (kxa in compact workspace rows); 0: N/2
   int *status;                         // set to 1 when a bounded wait of a staged kernel gives up (or null)
   double alpha_x;
   double s;                            // scalemodes
@@ -291,6 +396,9 @@ template <typename T> struct XlineNLArgs {
 
 // kept half-axis index under the x-line pruning rule
 __device__ __forceinline__ bool xkeep(int kxa, int k, int n) { return kxa == 0 || k < kxa || k == (n >> 1); }
+
+// Slot of half-axis index k in a row whose Nyquist column lies at nyq (0: N/2).
+__device__ __forceinline__ int xslot(int nyq, int k, int n) { return nyq && k == (n >> 1) ? nyq : k; }
 
 // Lines per CTA of the fused x pass (even; 3B columns in shared memory).  In
 // FP32 below 256, 8 where 16 lines would make 384-thread blocks (N = 64, 96,
@@ -368,8 +476,9 @@ __global__ void __launch_bounds__(round32(3 * XlineB<T, N>::v *(N / FftPlan<N>::
       const int n = EN::in_row(p, i);
       const int kk = n <= N / 2 ? n : N - n;
       const bool kp = xkeep(a.kxa, kk, N);
-      const C X1 = (v1 && kp) ? r1[kk] : mkc<C>(0, 0);
-      const C X2 = (v2 && kp) ? r2[kk] : mkc<C>(0, 0);
+      const int sl = xslot(a.nyq, kk, N);
+      const C X1 = (v1 && kp) ? r1[sl] : mkc<C>(0, 0);
+      const C X2 = (v2 && kp) ? r2[sl] : mkc<C>(0, 0);
       v[i] = pack_pair<C, N>(n, X1, X2);
     }
     fft_regs<C, N, true>(v, s, LD, col, p, act, a.tw);
@@ -433,18 +542,19 @@ __global__ void __launch_bounds__(round32(3 * XlineB<T, N>::v *(N / FftPlan<N>::
     const C X2 = mkc<C>(T(0.5) * (zk.y + zn.y), T(-0.5) * (zk.x - zn.x));
     const int la = line0 + 2 * j, lb = la + 1;
     if (!xkeep(a.kxa, k, N)) continue;
+    const int sl = xslot(a.nyq, k, N);
     if (c == 0) {
       if (la < a.nlines) {
-        a.NX[(long long)la * pout + k] = X1;
-        a.NY[(long long)la * pout + k] = X2;
+        a.NX[(long long)la * pout + sl] = X1;
+        a.NY[(long long)la * pout + sl] = X2;
       }
     } else if (c == 1) {
-      if (la < a.nlines) a.NZ[(long long)la * pout + k] = X1;
-      if (lb < a.nlines) a.NZ[(long long)lb * pout + k] = X2;
+      if (la < a.nlines) a.NZ[(long long)la * pout + sl] = X1;
+      if (lb < a.nlines) a.NZ[(long long)lb * pout + sl] = X2;
     } else {
       if (lb < a.nlines) {
-        a.NX[(long long)lb * pout + k] = X1;
-        a.NY[(long long)lb * pout + k] = X2;
+        a.NX[(long long)lb * pout + sl] = X1;
+        a.NY[(long long)lb * pout + sl] = X2;
       }
     }
   }
@@ -602,20 +712,21 @@ __device__ __forceinline__ void xline_w_tail(typename CT<T>::type *s, const Xlin
   // unpack two real transforms per sequence and store
   for (int k = lane; k < H; k += 32) {
     if (!xkeep(a.kxa, k, N)) continue;
+    const int sl = xslot(a.nyq, k, N);
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
       const C zk = s[AD::at(k, q, LDC)], zn = s[AD::at((N - k) % N, q, LDC)];
       const C X1 = mkc<C>(T(0.5) * (zk.x + zn.x), T(0.5) * (zk.y - zn.y));
       const C X2 = mkc<C>(T(0.5) * (zk.y + zn.y), T(-0.5) * (zk.x - zn.x));
       if (q == 0) {
-        a.NX[la * pout + k] = X1;
-        a.NY[la * pout + k] = X2;
+        a.NX[la * pout + sl] = X1;
+        a.NY[la * pout + sl] = X2;
       } else if (q == 1) {
-        a.NZ[la * pout + k] = X1;
-        a.NZ[lb * pout + k] = X2;
+        a.NZ[la * pout + sl] = X1;
+        a.NZ[lb * pout + sl] = X2;
       } else {
-        a.NX[lb * pout + k] = X1;
-        a.NY[lb * pout + k] = X2;
+        a.NX[lb * pout + sl] = X1;
+        a.NY[lb * pout + sl] = X2;
       }
     }
   }
@@ -668,8 +779,9 @@ __global__ void __launch_bounds__(32 * XlineWarp<T, N>::wpb)
     for (int i = 0; i <= E / 2; ++i) {
       const int n = p + P * i;   // <= N / 2 for i < E / 2 and for p = 0
       const bool kp = (i < E / 2 || p == 0) && xkeep(a.kxa, n, N);
-      x1[i] = kp ? g1[n] : mkc<C>(0, 0);
-      x2[i] = kp ? g2[n] : mkc<C>(0, 0);
+      const int sl = xslot(a.nyq, n, N);
+      x1[i] = kp ? g1[sl] : mkc<C>(0, 0);
+      x2[i] = kp ? g2[sl] : mkc<C>(0, 0);
     }
   };
   const int mirror = (lane & ~(P - 1)) | ((P - p) & (P - 1));   // lane of the mirror rows
@@ -753,8 +865,9 @@ __global__ void __launch_bounds__(32 * XlineWarp<T, 256>::wpb, MINB)
     for (int i = 0; i <= E / 2; ++i) {
       const int n = p + P * i;
       const bool kp = (i < E / 2 || p == 0) && xkeep(a.kxa, n, N);
-      x1[i] = kp ? g1[n] : mkc<C>(0, 0);
-      x2[i] = kp ? g2[n] : mkc<C>(0, 0);
+      const int sl = xslot(a.nyq, n, N);
+      x1[i] = kp ? g1[sl] : mkc<C>(0, 0);
+      x2[i] = kp ? g2[sl] : mkc<C>(0, 0);
     }
   };
   // value at row N - (p + 16 i) of a lane's rows from w (own rows): the partner
@@ -840,8 +953,9 @@ __global__ void __launch_bounds__(32 * XlineWarp<T, 256>::wpb, MINB)
       if (p == 0) zn = z[(E - i) & (E - 1)];
       const C zk = z[i];
       if ((i < E / 2 || p == 0) && xkeep(a.kxa, k, N)) {
-        if (d1) d1[k] = mkc<C>(T(0.5) * (zk.x + zn.x), T(0.5) * (zk.y - zn.y));
-        if (d2) d2[k] = mkc<C>(T(0.5) * (zk.y + zn.y), T(-0.5) * (zk.x - zn.x));
+        const int sl = xslot(a.nyq, k, N);
+        if (d1) d1[sl] = mkc<C>(T(0.5) * (zk.x + zn.x), T(0.5) * (zk.y - zn.y));
+        if (d2) d2[sl] = mkc<C>(T(0.5) * (zk.y + zn.y), T(-0.5) * (zk.x - zn.x));
       }
     }
   };
@@ -873,6 +987,7 @@ template <typename T> struct XlineArgs {
   void *out[6];
   const C *tw;
   int nlines, nxh;
+  int pitch;               // row pitch (complex elements) of the half lines; 0: nxh
   double scale;            // multiplies the output
 };
 
@@ -896,6 +1011,7 @@ __global__ void __launch_bounds__(round32((XlinePlainB<T, N>::v / 2) * (N / FftP
   C *s = reinterpret_cast<C *>(smem_raw);
   const C *in = reinterpret_cast<const C *>(a.in[blockIdx.y]);
   T *out = reinterpret_cast<T *>(a.out[blockIdx.y]);
+  const int pitch = a.pitch ? a.pitch : a.nxh;
   const bool act = threadIdx.x < NF;
   const int p = threadIdx.x % P, j = threadIdx.x / P;
   const int la = blockIdx.x * B + 2 * j, lb = la + 1;
@@ -905,8 +1021,8 @@ __global__ void __launch_bounds__(round32((XlinePlainB<T, N>::v / 2) * (N / FftP
   for (int i = 0; i < E; ++i) {
     const int n = EN::in_row(p, i);
     const int kk = n <= N / 2 ? n : N - n;
-    const C X1 = va ? in[(long long)la * a.nxh + kk] : mkc<C>(0, 0);
-    const C X2 = vb ? in[(long long)lb * a.nxh + kk] : mkc<C>(0, 0);
+    const C X1 = va ? in[(long long)la * pitch + kk] : mkc<C>(0, 0);
+    const C X2 = vb ? in[(long long)lb * pitch + kk] : mkc<C>(0, 0);
     v[i] = pack_pair<C, N>(n, X1, X2);
   }
   fft_regs<C, N, true>(v, s, LD, j, p, act, a.tw);
@@ -936,6 +1052,7 @@ __global__ void __launch_bounds__(round32((XlinePlainB<T, N>::v / 2) * (N / FftP
   C *s = reinterpret_cast<C *>(smem_raw);
   const T *in = reinterpret_cast<const T *>(a.in[blockIdx.y]);
   C *out = reinterpret_cast<C *>(a.out[blockIdx.y]);
+  const int pitch = a.pitch ? a.pitch : a.nxh;
   const int NT = blockDim.x;
   const bool act = threadIdx.x < NF;
   const int p = threadIdx.x % P, j = threadIdx.x / P;
@@ -963,8 +1080,8 @@ __global__ void __launch_bounds__(round32((XlinePlainB<T, N>::v / 2) * (N / FftP
     const C zk = s[k * LD + jj], zn = s[((N - k) % N) * LD + jj];
     const C X1 = mkc<C>(T(0.5) * (zk.x + zn.x) * sc, T(0.5) * (zk.y - zn.y) * sc);
     const C X2 = mkc<C>(T(0.5) * (zk.y + zn.y) * sc, T(-0.5) * (zk.x - zn.x) * sc);
-    if (la < a.nlines) out[(long long)la * a.nxh + k] = X1;
-    if (lb < a.nlines) out[(long long)lb * a.nxh + k] = X2;
+    if (la < a.nlines) out[(long long)la * pitch + k] = X1;
+    if (lb < a.nlines) out[(long long)lb * pitch + k] = X2;
   }
 }
 
@@ -999,7 +1116,7 @@ template <typename T> struct FinishArgs {
   AxisKeep kx, ky, kz;     // pruning: only kept (kz, ky) rows and kept kx modes are visited
   // layout of n3 when it is a padded workspace field: row pitch, elements
   // between components and between boxes; 0: the state's (nxh, nh, bstride)
-  int n3_pitch;
+  int n3_pitch, n3_nyq;    // n3_nyq: slot of the Nyquist column (0: nx / 2)
   long long n3_nh, n3_bstride;
   // a ky slab of a box split over ranks: row ky of this launch is ky0 + ky of
   // an axis of ny_k rows (0, 0: the box's own rows)
@@ -1070,7 +1187,7 @@ __global__ void __launch_bounds__(256, FinishMinB<T, MODE>::v)
       const long long idx = rowbase + kx;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        nn[h][c] = ok[h] ? a.n3[c * n3nh + n3row + kx] : mkc<C>(0, 0);
+        nn[h][c] = ok[h] ? a.n3[c * n3nh + n3row + xslot(a.n3_nyq, kx, a.nx)] : mkc<C>(0, 0);
         uu[h][c] = ok[h] && need_u ? a.uin[c * a.nh + idx] : mkc<C>(0, 0);
         ss[h][c] = ok[h] && MODE == FIN_CORR ? a.state[c * a.nh + idx] : mkc<C>(0, 0);
         no[h][c] = ok[h] && MODE == FIN_AB2 ? a.nold[c * a.nh + idx] : mkc<C>(0, 0);

@@ -29,41 +29,45 @@ template <typename T, int N> struct Launcher {
   static bool has_xline_warp();
   static cudaError_t xline_c2r(const XlineArgs<T> &a, int nf, cudaStream_t st);
   static cudaError_t xline_r2c(const XlineArgs<T> &a, int nf, cudaStream_t st);
-  static int strided_threads();
 };
 
 #define DNSBOX_SIZES(X) X(8) X(12) X(16) X(24) X(32) X(48) X(64) X(96) X(128) X(192) X(256) X(512) X(1024)
 
 #ifdef DNSBOX_LAUNCH_IMPL
-// Opts the kernel in to `bytes` of dynamic shared memory (the 48 KB default
-// covers static + dynamic, so it is set for every size); refuses sizes over
-// the 227 KB per-CTA limit.
+// Opts the kernel in to `bytes` of dynamic shared memory where the 48 KB every
+// kernel may use (static + dynamic; no kernel here has 4 KB of static) does
+// not cover them; refuses sizes over the 227 KB per-CTA limit.
 template <typename K>
 static cudaError_t set_smem(K kernel, size_t bytes) {
   if (bytes > 227 * 1024) return cudaErrorInvalidConfiguration;
+  if (bytes <= 44 * 1024) return cudaSuccess;
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-template <typename T, int N> int Launcher<T, N>::strided_threads() {
-  return round32(StridedCols<T, N>::v * (N / FftPlan<N>::E));
+template <typename T, int N, bool INV, int MODE>
+static cudaError_t strided_launch(const StridedArgs<T> &a, dim3 nb, cudaStream_t st) {
+  using SH = StridedShape<T, N>;
+  const cudaError_t e = set_smem(k_strided<T, N, INV, MODE>, SH::smem(INV));
+  if (e != cudaSuccess) return e;
+  k_strided<T, N, INV, MODE><<<nb, SH::NT, SH::smem(INV), st>>>(a);
+  return cudaGetLastError();
 }
 
 template <typename T, int N>
 cudaError_t Launcher<T, N>::strided(const StridedArgs<T> &a, bool inv, int ntiles, cudaStream_t st) {
-  using C = typename CT<T>::type;
-  const size_t smem = (size_t)N * StridedCols<T, N>::v * sizeof(C);
-  const int nt = strided_threads();
-  const dim3 nb((unsigned)ntiles * a.njobs * (TileCols<T>::v / StridedCols<T, N>::v),
-                (unsigned)(a.nbatch > 0 ? a.nbatch : 1));
-  cudaError_t e;
+  const dim3 nb((unsigned)ntiles * a.njobs, (unsigned)(a.nbatch > 0 ? a.nbatch : 1));
+  // the workspace modes of the passes that use them (inverse: state or
+  // workspace to workspace, forward: workspace to either); pruned columns need
+  // the compact workspace
+  const int ws = a.kcol.a && !a.compact ? 0 : a.ws;
   if (inv) {
-    if ((e = set_smem(k_strided<T, N, true>, smem)) != cudaSuccess) return e;
-    k_strided<T, N, true><<<nb, nt, smem, st>>>(a);
-  } else {
-    if ((e = set_smem(k_strided<T, N, false>, smem)) != cudaSuccess) return e;
-    k_strided<T, N, false><<<nb, nt, smem, st>>>(a);
+    if (ws == 3) return strided_launch<T, N, true, ST_WS>(a, nb, st);
+    if (ws == 2) return strided_launch<T, N, true, ST_TO_WS>(a, nb, st);
+    return strided_launch<T, N, true, ST_ANY>(a, nb, st);
   }
-  return cudaGetLastError();
+  if (ws == 3) return strided_launch<T, N, false, ST_WS>(a, nb, st);
+  if (ws == 1) return strided_launch<T, N, false, ST_FROM_WS>(a, nb, st);
+  return strided_launch<T, N, false, ST_ANY>(a, nb, st);
 }
 
 template <typename T, int N> bool Launcher<T, N>::has_tc() {
