@@ -670,7 +670,10 @@ static int run_rhs(dnsbox_ctx *c, const void *uin, int mode, void *out, void *st
   x.NY = reinterpret_cast<C *>(wfield(c->W1, c, 1));
   x.NZ = reinterpret_cast<C *>(wfield(c->W1, c, 2));
   x.pin = x.pout = wp;
-  if (compact) x.nyq = c->keep[0].a;
+  if (compact) {
+    x.nyq = c->keep[0].a;
+    x.npad = a.nslot - x.nyq - 1;
+  }
   x.status = c->tc_status;
   x.tw = reinterpret_cast<const C *>(c->tw[0]);
   x.st = c->st;

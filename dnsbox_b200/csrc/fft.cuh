@@ -53,9 +53,7 @@ template <int N> struct WarpPlan;
     static constexpr int NST = sizeof(R) / sizeof(int);                        \
     __host__ __device__ static constexpr int ns(int s) { int p = 1; for (int i = 0; i < s; ++i) p *= R[i]; return p; } \
   };
-DNSBOX_WPLAN(256, 8, 8, 8, 4)
 DNSBOX_WPLAN(512, 16, 16, 8, 4)
-DNSBOX_WPLAN(1024, 32, 16, 16, 4)
 #undef DNSBOX_WPLAN
 
 // Shared-memory addressing of element (row, col) of a tile.  Row-major tiles

@@ -305,6 +305,22 @@ DNSBOX_VPLAN(512, 8, 8, 8, 8)
 DNSBOX_VPLAN(1024, 16, 16, 16, 4)
 #undef DNSBOX_VPLAN
 
+// Plans of the x lines, at most 32 threads per line (a warp synchronises
+// itself): 16 values in single precision, 8 in double precision (three
+// sequences of a line are held at once) where the length allows it.
+template <typename T, int N> struct XPlan : VPlan<N> {};
+#define DNSBOX_XPLAN(TT, NN, EE, ...)                                                                                \
+  template <> struct XPlan<TT, NN> {                                                                                 \
+    static constexpr int N = NN, E = EE, P = NN / EE;                                                                \
+    static constexpr int R[] = {__VA_ARGS__};                                                                        \
+    static constexpr int NST = sizeof(R) / sizeof(int);                                                              \
+    __host__ __device__ static constexpr int ns(int s) { int q = 1; for (int i = 0; i < s; ++i) q *= R[i]; return q; } \
+  };
+DNSBOX_XPLAN(float, 512, 16, 16, 8, 4)
+DNSBOX_XPLAN(double, 128, 8, 8, 4, 4)
+DNSBOX_XPLAN(double, 256, 8, 8, 8, 4)
+#undef DNSBOX_XPLAN
+
 // Register i of a thread holds row p + P in_q(i) before and p + P out_q(i)
 // after the transform; in_i / out_i are the inverse maps.
 template <class PL> struct VEnds {
@@ -323,14 +339,22 @@ template <class PL, int S> __host__ __device__ constexpr int vtw_off() {
 }
 template <class PL> __host__ __device__ constexpr int vtw_size() { return vtw_off<PL, PL::NST>(); }
 
-__device__ __forceinline__ VC<double> vtw_of(double2 w) { return VC<double>{w.x, w.y}; }
-__device__ __forceinline__ VC<f2> vtw_of(float2 w) { return VC<f2>{mkf2(w.x, w.x), mkf2(w.y, w.y)}; }
+template <typename V> struct VtwOf;
+template <> struct VtwOf<VC<double>> {
+  __device__ static __forceinline__ VC<double> of(double2 w) { return VC<double>{w.x, w.y}; }
+};
+template <> struct VtwOf<VC<float>> {
+  __device__ static __forceinline__ VC<float> of(float2 w) { return VC<float>{w.x, w.y}; }
+};
+template <> struct VtwOf<VC<f2>> {
+  __device__ static __forceinline__ VC<f2> of(float2 w) { return VC<f2>{mkf2(w.x, w.x), mkf2(w.y, w.y)}; }
+};
 // from the N-point table exp(-2 pi i k / N); all threads of the block
 template <class PL, typename V, typename C, int S = 1>
 __device__ __forceinline__ void vtw_fill(V *t, const C *__restrict__ tw, int tid, int nthreads) {
   if constexpr (S < PL::NST) {
     constexpr int NS = PL::ns(S), R = PL::R[S], TS = PL::N / (NS * R);
-    for (int i = tid; i < (R - 1) * NS; i += nthreads) t[vtw_off<PL, S>() + i] = vtw_of(tw[(1 + i / NS) * (i % NS) * TS]);
+    for (int i = tid; i < (R - 1) * NS; i += nthreads) t[vtw_off<PL, S>() + i] = VtwOf<V>::of(tw[(1 + i / NS) * (i % NS) * TS]);
     vtw_fill<PL, V, C, S + 1>(t, tw, tid, nthreads);
   }
 }
@@ -344,13 +368,18 @@ template <bool INV, typename V> __device__ __forceinline__ V vtwmul(V a, V w) {
   return r;
 }
 
+// a pair with one twiddle for both transforms
+template <bool INV> __device__ __forceinline__ VC<f2> vtwmul(VC<f2> a, VC<float> w) {
+  return vtwmul<INV>(a, VC<f2>{mkf2(w.re, w.re), mkf2(w.im, w.im)});
+}
+
 // ---------------------------------------------------------------------- stages
 // Whole transform of the values v (first-stage order) into x (last-stage
 // order), exchanged through the tile s; AD::at(row, col) gives an element's
 // place.  sync() separates the phases (a block or a warp barrier).  The tile
 // may be reused after the caller's next barrier.
-template <class PL, bool INV, class AD, int S, typename O, typename V, typename SYNC>
-__device__ __forceinline__ void vfft_stage(O *x, V *s, int col, int p, const V *tw, SYNC sync) {
+template <class PL, bool INV, class AD, int S, typename O, typename V, typename W, typename SYNC>
+__device__ __forceinline__ void vfft_stage(O *x, V *s, int col, int p, const W *tw, SYNC sync) {
   constexpr int R = PL::R[S], NS = PL::ns(S), E = PL::E, M = E / R, P = PL::P, NB = PL::N / R;
   constexpr bool last = S + 1 == PL::NST;
   V y[last ? 1 : E];
@@ -378,8 +407,8 @@ __device__ __forceinline__ void vfft_stage(O *x, V *s, int col, int p, const V *
     vfft_stage<PL, INV, AD, S + 1>(x, s, col, p, tw, sync);
   }
 }
-template <class PL, bool INV, class AD, typename O, typename A, typename V, typename SYNC>
-__device__ __forceinline__ void vfft(const A *v, O *x, V *s, int col, int p, const V *tw, SYNC sync) {
+template <class PL, bool INV, class AD, typename O, typename A, typename V, typename W, typename SYNC>
+__device__ __forceinline__ void vfft(const A *v, O *x, V *s, int col, int p, const W *tw, SYNC sync) {
   constexpr int R = PL::R[0], M = PL::E / R, P = PL::P;
   if constexpr (PL::NST == 1) {
     vdft<R, INV>(v, x);

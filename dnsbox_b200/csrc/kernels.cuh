@@ -388,6 +388,7 @@ template <typename T> struct XlineNLArgs {
   int lines_per_box;                   // ny * nz
   int kxa;                             // pruning: only kx < kxa and kx = N/2 are read and written (0: all)
   int pin, pout;                       // row pitch (complex elements) of the inputs / outputs; 0: nxh
+  int npad;                            // compact rows: slots after nyq that complete its 32-byte sector (written as 0)
   int nyq;                             // slot of the Nyquist column in a row (kxa in compact workspace rows); 0: N/2
   int *status;                         // set to 1 when a bounded wait of a staged kernel gives up (or null)
   double alpha_x;
@@ -400,15 +401,9 @@ __device__ __forceinline__ bool xkeep(int kxa, int k, int n) { return kxa == 0 |
 // Slot of half-axis index k in a row whose Nyquist column lies at nyq (0: N/2).
 __device__ __forceinline__ int xslot(int nyq, int k, int n) { return nyq && k == (n >> 1) ? nyq : k; }
 
-// Lines per CTA of the fused x pass (even; 3B columns in shared memory).  In
-// FP32 below 256, 8 where 16 lines would make 384-thread blocks (N = 64, 96,
-// 128): four 192-thread CTAs per SM instead of two of 384, each with its own
-// barriers (x pass 10-13% faster at 64^3 and 96^3).
+// Lines per CTA of the block x kernel (even; 3B columns in shared memory).
 template <typename T, int N> struct XlineB {
-  static constexpr int v = (N >= 512) ? 2
-                         : (sizeof(T) == 8 ? (N >= 256 ? 4 : 8)
-                                           : (N >= 256 || (FftPlan<N>::E <= 16 && 3 * 16 * (N / FftPlan<N>::E) > 256)
-                                                  ? 8 : 16));
+  static constexpr int v = 2;
 };
 
 // Full-length sequence value at row n of Z = X1 + i X2, where X1, X2 are the
@@ -422,9 +417,10 @@ __device__ __forceinline__ C pack_pair(int n, C X1, C X2) {
   return mkc<C>(X1.x + X2.y, X2.x - X1.y);   // conj(X1) + i conj(X2) at N - n
 }
 
-// Resident CTAs of the block x-line kernel to ask the register allocator
-// for: 3 for blocks of up to 256 threads; 2 for the 384-thread FP32 blocks of
-// N = 1024 (80 registers instead of 123, two CTAs per SM instead of one).
+// The block x kernel: lines of 1024 points (and, by choice, double-precision
+// lines of 512).  Resident CTAs to ask the register allocator for: 3 for
+// blocks of up to 256 threads; 2 for the 384-thread FP32 blocks of N = 1024
+// (80 registers instead of 123, two CTAs per SM instead of one).
 template <typename T, int N> struct XlineMinCtas {
   static constexpr int NT = round32(3 * XlineB<T, N>::v * (N / FftPlan<N>::E));
   static constexpr int v = (sizeof(T) == 4 && N >= 1024) ? 2 : min_ctas(NT, 3);
@@ -586,48 +582,19 @@ __global__ void __launch_bounds__(round32(3 * XlineB<T, N>::v *(N / FftPlan<N>::
   }
 }
 
-// Warp-granular variant of the fused x pass for N >= 256: each warp owns one
+// Warp-granular variant of the fused x pass for double-precision lines of 512
+// points (whose fields do not fit a warp's registers): each warp owns one
 // line pair from its loads to its stores and synchronises only with
 // __syncwarp, so the SM overlaps one warp's memory phases with another's
 // transforms (the block-wide barriers of k_xline_nl serialise them).  Columns
 // of a warp's tile are the six sequences of k_xline_nl, stored column-major
-// with the row / R0 skew (conflict-free for both plans below).  At N = 256 a
-// sequence runs the two-stage radix-16 plan on 16 threads, so a warp
-// transforms two sequences at once with one shared-memory exchange each; at
-// N = 512 a sequence runs the three-stage plan on all 32 threads.
-// In FP32 the twiddles come from per-stage tables in shared memory (one
-// wavefront per lane-varying read instead of a scatter of L1 sectors, which
-// left the kernel bound by L1 throughput); FP64 keeps the global table, whose
-// shared copy would cost a resident block.
+// with the row / R0 skew; a sequence runs the three-stage plan on all 32
+// threads.
 template <typename T, int N> struct XlineWarp {
-  static constexpr bool on = N == 256 || N == 512;
-  static constexpr int wpb = sizeof(T) == 8 ? (N >= 512 ? 1 : 2) : (N >= 1024 ? 1 : (N >= 512 ? 2 : 4));
-  using Plan = typename std::conditional<N == 256, FftPlan<256>, WarpPlan<N>>::type;
-  static constexpr bool full3 = 32 / (N / Plan::E) == 2 && sizeof(T) == 4;   // see xline_w_tail
-  static constexpr bool smtw = on && sizeof(T) == 4;
-  static constexpr int twn = smtw ? tw_size<Plan>() + (full3 ? tw_size<WarpPlan<N>>() : 0) : 0;
-  // twiddle tables of the block after its warps' tiles; all threads fill them
-  __device__ static __forceinline__ typename CT<T>::type *tables(unsigned char *smem, const typename CT<T>::type *tw,
-                                                                  int cols = 6) {
-    using C = typename CT<T>::type;
-    C *t = reinterpret_cast<C *>(smem) + (size_t)wpb * cols * (N + N / Plan::R[0]);
-    if constexpr (smtw) {
-      tw_fill<C, Plan>(t, tw, threadIdx.x, blockDim.x);
-      if constexpr (full3) tw_fill<C, WarpPlan<N>>(t + tw_size<Plan>(), tw, threadIdx.x, blockDim.x);
-      __syncthreads();
-    }
-    return t;
-  }
+  static constexpr bool on = N == 512 && sizeof(T) == 8;
+  static constexpr int wpb = 1;
+  using Plan = WarpPlan<512>;
 };
-
-// The x pass's transform of `v` on column `col` with the kernel's twiddle source.
-template <typename T, class PL, bool INV, class AD, int N>
-__device__ __forceinline__ void xw_fft(typename CT<T>::type *v, typename CT<T>::type *s, int LD, int col, int p,
-                                       bool active, const typename CT<T>::type *tw, const typename CT<T>::type *twt) {
-  using C = typename CT<T>::type;
-  if constexpr (XlineWarp<T, N>::smtw) fft_regs_t<C, PL, INV, true, AD>(v, s, LD, col, p, active, TwShared<C>{twt});
-  else fft_regs_p<C, PL, INV, true, AD>(v, s, LD, col, p, active, tw);
-}
 
 // Second half of the warp-granular fused x pass for one line pair (la, lb):
 // the inverse transforms are in the warp's tile s (column-major, skewed);
@@ -635,18 +602,14 @@ __device__ __forceinline__ void xw_fft(typename CT<T>::type *v, typename CT<T>::
 // output half lines and the CFL maxima of the pair.
 template <typename T, int N>
 __device__ __forceinline__ void xline_w_tail(typename CT<T>::type *s, const XlineNLArgs<T> &a, long long la,
-                                             long long lb, int lane, long long pout,
-                                             const typename CT<T>::type *twt) {
+                                             long long lb, int lane, long long pout) {
   using C = typename CT<T>::type;
   using PL = typename XlineWarp<T, N>::Plan;
   using EN = FftEndsP<PL>;
   using AD = AddrSkew<PL::R[0]>;
   constexpr int E = PL::E;
-  constexpr int P = N / E;
-  constexpr int SPW = 32 / P;
   constexpr int H = N / 2 + 1;
   constexpr int LDC = N + N / PL::R[0];
-  const int p = lane % P, h = lane / P;
   const T sc = T(a.s);
   __syncwarp();
   // (omega x u) * s, written back as (px_a,py_a) (pz_a,pz_b) (px_b,py_b) in
@@ -673,40 +636,16 @@ __device__ __forceinline__ void xline_w_tail(typename CT<T>::type *s, const Xlin
     s[AD::at(n, 2, LDC)] = mkc<C>(px[1], py[1]);
   }
   __syncwarp();
-  // forward transforms of the three product sequences, SPW at a time.  In
-  // FP32 with two per warp, sequence 2 runs on all 32 lanes with the 32-thread
-  // plan (same column, skew and twiddle table) instead of on one half-warp
-  // (in FP64 that form measured slower)
-  constexpr bool FULL3 = XlineWarp<T, N>::full3;
-  constexpr int RF = FULL3 ? 1 : (3 + SPW - 1) / SPW;
+  // forward transforms of the three product sequences
 #pragma unroll 1
-  for (int r = 0; r < RF; ++r) {
-    const int q = SPW * r + h;
-    const bool act = q < 3;
-    const int qc = act ? q : 0;
+  for (int q = 0; q < 3; ++q) {
     C v[E];
-    if (act) {
 #pragma unroll
-      for (int i = 0; i < E; ++i) v[i] = s[AD::at(EN::in_row(p, i), qc, LDC)];
-    }
+    for (int i = 0; i < E; ++i) v[i] = s[AD::at(EN::in_row(lane, i), q, LDC)];
     __syncwarp();
-    xw_fft<T, PL, false, AD, N>(v, s, LDC, qc, p, act, a.tw, twt);
-    if (act) {
+    fft_regs_p<C, PL, false, true, AD>(v, s, LDC, q, lane, true, a.tw);
 #pragma unroll
-      for (int i = 0; i < E; ++i) s[AD::at(EN::out_row(p, i), qc, LDC)] = v[i];
-    }
-  }
-  if constexpr (FULL3) {
-    using WP = WarpPlan<N>;
-    using EW = FftEndsP<WP>;
-    static_assert(N + (N - 1) / PL::R[0] < LDC, "the 32-thread plan stays inside its column");
-    C w[WP::E];
-#pragma unroll
-    for (int i = 0; i < WP::E; ++i) w[i] = s[AD::at(EW::in_row(lane, i), 2, LDC)];
-    __syncwarp();
-    xw_fft<T, WP, false, AD, N>(w, s, LDC, 2, lane, true, a.tw, twt + tw_size<PL>());
-#pragma unroll
-    for (int i = 0; i < WP::E; ++i) s[AD::at(EW::out_row(lane, i), 2, LDC)] = w[i];
+    for (int i = 0; i < E; ++i) s[AD::at(EN::out_row(lane, i), q, LDC)] = v[i];
   }
   __syncwarp();
   // unpack two real transforms per sequence and store
@@ -751,23 +690,22 @@ __global__ void __launch_bounds__(32 * XlineWarp<T, N>::wpb)
   using AD = AddrSkew<PL::R[0]>;
   constexpr int E = PL::E;
   constexpr int P = N / E;                // threads per sequence
-  constexpr int SPW = 32 / P;             // sequences a warp transforms at once
+  static_assert(P == 32, "a sequence on all lanes");
   constexpr int LDC = N + N / PL::R[0];   // column length with the skew
   constexpr int WPB = XlineWarp<T, N>::wpb;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   C *s = reinterpret_cast<C *>(smem_raw) + (size_t)warp * 6 * LDC;
-  const C *twt = XlineWarp<T, N>::tables(smem_raw, a.tw);   // (a block barrier in FP32)
   const long long la = 2 * ((long long)blockIdx.x * WPB + warp), lb = la + 1;
   if (la >= a.nlines) return;
   const C *f1s[6] = {a.U, a.U, a.W, a.OX, a.OX, a.OZ};
   const C *f2s[6] = {a.V, a.V, a.W, a.OY, a.OY, a.OZ};
   const long long l1s[6] = {la, lb, la, la, lb, la};
   const long long l2s[6] = {la, lb, lb, la, lb, lb};
-  const int p = lane % P, h = lane / P;   // position in the sequence, sequence slot
+  const int p = lane;   // position in the sequence
   const long long pin = a.pin ? a.pin : a.nxh, pout = a.pout ? a.pout : a.nxh;
-  // inverse transforms: round r transforms sequences SPW r + h; the loads of
-  // the next round are issued before this round's transform.  A lane loads
+  // inverse transforms: round r transforms sequence r; the loads of the next
+  // round are issued before this round's transform.  A lane loads
   // only its rows n = p + P i <= N/2 (i < E/2, and i = E/2 at p = 0); row
   // N - n of the Hermitian mirror is row n' = (P - p) + P (E - 1 - i) of lane
   // P - p (lane p = 0: its own row P (E - i)), taken by a shuffle, so every
@@ -799,185 +737,300 @@ __global__ void __launch_bounds__(32 * XlineWarp<T, N>::wpb)
       x2[i] = m2;
     }
   };
-  load(f1s[h] + l1s[h] * pin, f2s[h] + l2s[h] * pin);
+  load(f1s[0] + l1s[0] * pin, f2s[0] + l2s[0] * pin);
 #pragma unroll 1
-  for (int r = 0; r < 6 / SPW; ++r) {
-    const int q = SPW * r + h;
+  for (int q = 0; q < 6; ++q) {
     C v[E];
     mirror_fill();
 #pragma unroll
     for (int i = 0; i < E; ++i) v[i] = pack_pair<C, N>(EN::in_row(p, i), x1[i], x2[i]);
-    if (r + 1 < 6 / SPW) {
-      const int qn = q + SPW;
+    if (q + 1 < 6) {
+      const int qn = q + 1;
       load(f1s[qn] + l1s[qn] * pin, f2s[qn] + l2s[qn] * pin);
     }
-    xw_fft<T, PL, true, AD, N>(v, s, LDC, q, p, true, a.tw, twt);
+    fft_regs_p<C, PL, true, true, AD>(v, s, LDC, q, p, true, a.tw);
 #pragma unroll
     for (int i = 0; i < E; ++i) s[AD::at(EN::out_row(p, i), q, LDC)] = v[i];
   }
-  xline_w_tail<T, N>(s, a, la, lb, lane, pout, twt);
+  xline_w_tail<T, N>(s, a, la, lb, lane, pout);
 }
 
-// Plain x-line transforms of nf fields (blockIdx.y = field).
-// Fused x pass at N = 256 with the fields of a line in registers (FP32).
-// Half-warp h owns line la + h and packs its six real lines as three
-// sequences, U + iV, W + i 2^e OZ and OX + i OY, transformed one per round on
-// its 16 lanes.  With the two-stage radix-16 plan a lane's first-stage
-// input rows and last-stage output rows are the same, n = p + 16 i, so after
-// the three rounds every lane holds u, v, w and the vorticity at its 16
-// rows: the cross product and the CFL maxima need no shared memory, and the
-// products px + i py are already the forward transform's inputs.  The third
-// forward sequence, pz(a) + i pz(b), is formed by one shuffle across the
-// halves and transformed by both (each stores its line's half).  Shared
-// memory holds only each sequence's one exchange (two columns per warp) and
-// the twiddle tables.  Hermitian-mirror rows, on input and output, come from
-// the partner lane by shuffle.
-// MINB > 0: that many resident blocks per SM asked of the register allocator.
-template <typename T, int MINB = 0>
-__global__ void __launch_bounds__(32 * XlineWarp<T, 256>::wpb, MINB)
-    k_xline_nl_r(const __grid_constant__ XlineNLArgs<T> a) {
-  constexpr int N = 256;
+// ------------------------------------------------ fused x pass, fields in registers
+// One complex value, zero where !on; volatile, so that loads stay where they
+// are issued, ahead of the transforms that hide them.
+__device__ __forceinline__ float2 ld_on(const float2 *p, bool on) {
+  float2 x = make_float2(0.f, 0.f);
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q ld.global.v2.f32 {%0, %1}, [%2];\n\t}"
+               : "+f"(x.x), "+f"(x.y)
+               : "l"(p), "r"((unsigned)on));
+  return x;
+}
+__device__ __forceinline__ double2 ld_on(const double2 *p, bool on) {
+  double2 x = make_double2(0.0, 0.0);
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q ld.global.v2.f64 {%0, %1}, [%2];\n\t}"
+               : "+d"(x.x), "+d"(x.y)
+               : "l"(p), "r"((unsigned)on));
+  return x;
+}
+// Exchange tile of one line: rows skewed by row / R0, or for the 4 x 4 x ..
+// plans of 96 and 192 exchanged by an exclusive or within 16, so that the
+// strided writes of a stage and the consecutive reads of the next fall in
+// distinct banks for 8- and 16-byte elements (counted for every access of
+// every plan).
+template <typename PL> struct XTile {
+  static constexpr int N = PL::N, R0 = PL::R[0];
+  static constexpr int SK = (R0 == 8 || R0 == 16) ? R0 : 4;
+  static constexpr bool XOR = N == 96 || N == 192;
+  static constexpr int pitch = PL::NST == 1 ? 0 : XOR ? N + (N == 96 ? 8 : 0) : N + N / SK;
+  __device__ static __forceinline__ int at(int row, int) { return XOR ? row ^ (row >> 2 & 15) : row + row / SK; }
+};
+template <typename T, int N> struct XReg {
+  using PL = XPlan<T, N>;
+  // up to 48 (FP32) or 36 (FP64) held values per thread, a line within a warp
+  static constexpr bool on = PL::P <= 32 && PL::E <= (sizeof(T) == 8 ? 12 : 16);
+  static constexpr int NT = 128;                      // threads of a full block
+  static constexpr size_t tw = ((size_t)vtw_size<PL>() * 2 * sizeof(T) + 15) / 16 * 16;
+  static constexpr size_t line = (size_t)XTile<PL>::pitch * 16;
+  static constexpr size_t smem(int threads) { return tw + threads / PL::P * line; }
+  static constexpr int minb = sizeof(T) == 8 ? (PL::E <= 8 ? 3 : 2) : (PL::E <= 8 ? 5 : PL::E == 12 ? 4 : 3);
+};
+
+// Fused x pass: P lanes own one line from its loads to its stores.  Every plan
+// gives a lane the rows p + P q at both ends of a transform, so u, v, w and the
+// vorticity of a row meet in one lane's registers after the inverse
+// transforms, the cross product is formed there and is the forward
+// transforms' input; shared memory carries only each transform's exchanges.
+// A line's six real lines are three sequences: U + iV and OX + i OY, in single
+// precision transformed together as pairs, and W + i 2^e OZ, whose parts are
+// brought to one magnitude first (the transform rounds them relative to each
+// other; e is the difference of the half lines' exponents, exact both ways).
+// Forward, px + i py and pz + i 0 (its transform is the half line itself).
+// A lane loads its rows up to N/2 and forms both that row's value and its
+// Hermitian mirror's, which goes to the lane that holds row N - n by shuffle.
+// Against the block kernel (fields in shared memory, 45% bank conflicts at 96)
+// and the warp kernels it replaces, us: 32 boxes of 96^3 FP32 625 -> 287, of
+// 64^3 152 -> 82, of 32^3 29 -> 19, 128^3 55 -> 27, 192^3 191 -> 78, 256^3 162 ->
+// 138 (FP64 397 -> 352), 512^3 1698 -> 1335.  At 256 in FP32 it is balanced:
+// issue 57%, FMA pipe 50%, L1 60%, 12 warps by registers; FP64 (78%) and 96
+// (87%) are bound by L1, the exchanges.  All loads of a line up front (the
+// third sequence's during the pair's transform) brought 179 -> 140 at 256.
+template <typename T, int N>
+__global__ void __launch_bounds__(XReg<T, N>::NT, XReg<T, N>::minb)
+    k_xline_nl_g(const __grid_constant__ XlineNLArgs<T> a) {
   using C = typename CT<T>::type;
-  using PL = typename XlineWarp<T, N>::Plan;
-  using EN = FftEndsP<PL>;
-  using AD = AddrSkew<PL::R[0]>;
-  constexpr int E = PL::E;
-  constexpr int P = N / E;
-  static_assert(P == 16 && E == 16 && PL::NST == 2 && PL::R[0] == 16 && PL::R[1] == 16,
-                "rows n = p + 16 i at both ends of the transform");
-  constexpr int LDC = N + N / PL::R[0];
-  constexpr int WPB = XlineWarp<T, N>::wpb;
+  using SH = XReg<T, N>;
+  using PL = typename SH::PL;
+  using EN = VEnds<PL>;
+  using AD = XTile<PL>;
+  using V1 = VC<T>;
+  constexpr int E = PL::E, P = PL::P, H = E / 2;
+  constexpr bool PAIR = sizeof(T) == 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int p = lane & 15, h = lane >> 4;
-  C *s = reinterpret_cast<C *>(smem_raw) + (size_t)warp * 2 * LDC;
-  const C *twt = XlineWarp<T, N>::tables(smem_raw, a.tw, 2);   // (a block barrier in FP32)
-  const long long la = 2 * ((long long)blockIdx.x * WPB + warp);
-  if (la >= a.nlines) return;
-  const long long line = la + h;
+  V1 *twt = reinterpret_cast<V1 *>(smem_raw);
+  vtw_fill<PL, V1>(twt, a.tw, threadIdx.x, blockDim.x);
+  __syncthreads();
+  const int g = threadIdx.x / P, p = threadIdx.x % P, lane = threadIdx.x & 31;
+  unsigned char *tile = smem_raw + SH::tw + (size_t)g * SH::line;
+  V1 *s1 = reinterpret_cast<V1 *>(tile);
   const long long pin = a.pin ? a.pin : a.nxh, pout = a.pout ? a.pout : a.nxh;
-  const T sc = T(a.s);
-  const int mirror = (lane & 16) | ((16 - p) & 15);
-  // rows n = p + 16 i <= N / 2 of the two half lines of a sequence
-  C x1[E / 2 + 1], x2[E / 2 + 1];
-  auto load = [&](const C *g1, const C *g2) {
+  // last lines first: what pass B wrote last is still in L2
+  const unsigned blk = gridDim.x - 1 - blockIdx.x;
+  const long long line = (long long)blk * (blockDim.x / P) + g;
+  const bool on = line < a.nlines;
+  const int mirror = (lane & ~(P - 1)) | ((P - p) & (P - 1));   // lane of rows N - n
+  auto sync = []() { __syncwarp(); };
+  // own rows n = p + P i, i <= H (i = H: the Nyquist row of lane 0), bit i of own
+  unsigned own = 0;
 #pragma unroll
-    for (int i = 0; i <= E / 2; ++i) {
-      const int n = p + P * i;
-      const bool kp = (i < E / 2 || p == 0) && xkeep(a.kxa, n, N);
-      const int sl = xslot(a.nyq, n, N);
-      x1[i] = kp ? g1[sl] : mkc<C>(0, 0);
-      x2[i] = kp ? g2[sl] : mkc<C>(0, 0);
+  for (int i = 0; i <= H; ++i)
+    if (on && (i < H || p == 0) && xkeep(a.kxa, p + P * i, N)) own |= 1u << i;
+  const int nyq = a.nyq ? a.nyq : N / 2;
+  auto load = [&](const C *f, C *x) {
+    const C *r = f + line * pin;
+#pragma unroll
+    for (int i = 0; i <= H; ++i) {
+      x[i] = ld_on(r + (i == H ? nyq : p + P * i), own >> i & 1);
+    }
+    if (p == 0) x[0].y = x[H].y = 0;   // a C2R drops these imaginary parts
+  };
+  auto shfl = [&](T v) { return __shfl_sync(0xffffffffu, v, mirror); };
+  // X1 + i X2 at the own rows and the mirror rows from the half lines x1, x2:
+  // put(q, re, im) with the value of row p + P q
+  auto pack = [&](const C *x1, const C *x2, auto put) {
+#pragma unroll
+    for (int i = 0; i < H; ++i) put(i, x1[i].x - x2[i].y, x1[i].y + x2[i].x);
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+      // lane p sends the mirror of its row i, lane 0 (its own partner) that of row i + 1
+      const int j = i + 1;
+      T re = x1[i].x + x2[i].y, im = x2[i].x - x1[i].y;
+      const T re0 = x1[j].x + x2[j].y, im0 = x2[j].x - x1[j].y;   // row N/2: imaginary parts are 0
+      re = p == 0 ? re0 : re;
+      im = p == 0 ? im0 : im;
+      put(E - 1 - i, shfl(re), shfl(im));
     }
   };
-  // value at row N - (p + 16 i) of a lane's rows from w (own rows): the partner
-  // lane's row p' + 16 (15 - i), or (p = 0) its own row 16 (16 - i)
-  auto shfl_c = [&](C c, int src) {
-    return mkc<C>(__shfl_sync(0xffffffffu, c.x, src), __shfl_sync(0xffffffffu, c.y, src));
-  };
-  const C *f1s[3] = {a.U, a.W, a.OX};
-  const C *f2s[3] = {a.V, a.OZ, a.OY};
-  // W and OZ share a sequence, and the vorticity is larger than the velocity
-  // by the factor s of the spectral curl and by the wavenumbers of the field:
-  // the transform would round OZ's part relative to W's, so each line's OZ is
-  // first brought to its W's magnitude by a power of two (exact both ways),
-  // the exponent difference of the two half lines' largest components.
   T up = 1, down = 1;
-  C o[3][E];   // inverse transforms: (u, v), (w, 2^e oz), (ox, oy) at rows p + 16 i
-  load(f1s[0] + line * pin, f2s[0] + line * pin);
+  V1 w[E];   // (w, 2^e oz) at row p + P q in w[out_i(q)]
+  T u_[E], v_[E], ox_[E], oy_[E];
+  C xw[H + 1], xo[H + 1];
+  if constexpr (PAIR) {
+    using V2 = VC<f2>;
+    V2 z[E], x[E];
+    {
+      C x1[H + 1], x2[H + 1], x3[H + 1], x4[H + 1];
+      load(a.U, x1);
+      load(a.V, x2);
+      load(a.OX, x3);
+      load(a.OY, x4);
+      load(a.W, xw);   // on their way during the pair's transform
+      load(a.OZ, xo);
+      T re[E], im[E];
+      pack(x1, x2, [&](int q, T r, T i) { re[q] = r, im[q] = i; });
+      pack(x3, x4, [&](int q, T r, T i) { z[EN::in_i(q)] = V2{mkf2(re[q], r), mkf2(im[q], i)}; });
+    }
+    vfft<PL, true, AD>(z, x, reinterpret_cast<V2 *>(tile), 0, p, twt, sync);
 #pragma unroll
-  for (int r = 0; r < 3; ++r) {
-    C v[E];
-    if (r == 1) {
-      T mw = 0, mo = 0;
+    for (int i = 0; i < E; ++i) u_[i] = f2_lo(x[i].re), v_[i] = f2_lo(x[i].im), ox_[i] = f2_hi(x[i].re), oy_[i] = f2_hi(x[i].im);
+  } else {
+    load(a.U, xw);
+    load(a.V, xo);
 #pragma unroll
-      for (int i = 0; i <= E / 2; ++i) {
-        mw = fmax(mw, fmax(fabs(x1[i].x), fabs(x1[i].y)));
-        mo = fmax(mo, fmax(fabs(x2[i].x), fabs(x2[i].y)));
-      }
+    for (int k = 0; k < 2; ++k) {
+      V1 z[E], x[E];
+      pack(xw, xo, [&](int q, T r, T i) { z[EN::in_i(q)] = V1{r, i}; });
+      load(k == 0 ? a.OX : a.W, xw);   // the next sequence's rows
+      load(k == 0 ? a.OY : a.OZ, xo);
+      vfft<PL, true, AD>(z, x, s1, 0, p, twt, sync);
+      sync();
 #pragma unroll
-      for (int o = 8; o; o >>= 1) {   // the 16 lanes of this line
-        mw = fmax(mw, __shfl_xor_sync(0xffffffffu, mw, o));
-        mo = fmax(mo, __shfl_xor_sync(0xffffffffu, mo, o));
-      }
-      int ew = 0, eo = 0;
-      frexp(mw, &ew);
-      frexp(mo, &eo);
-      const int d = mw > 0 && mo > 0 ? max(-96, min(96, ew - eo)) : 0;
-      up = ldexp(T(1), d);
-      down = ldexp(T(1), -d);
+      for (int i = 0; i < E; ++i) (k == 0 ? u_ : ox_)[i] = x[i].re, (k == 0 ? v_ : oy_)[i] = x[i].im;
+    }
+  }
+  {
+    T mw = 0, mo = 0;
 #pragma unroll
-      for (int i = 0; i <= E / 2; ++i) x2[i] = mkc<C>(x2[i].x * up, x2[i].y * up);
+    for (int i = 0; i <= H; ++i) {
+      mw = fmax(mw, fmax(fabs(xw[i].x), fabs(xw[i].y)));
+      mo = fmax(mo, fmax(fabs(xo[i].x), fabs(xo[i].y)));
     }
 #pragma unroll
-    for (int i = 0; i < E; ++i) {
-      const int n = p + P * i;
-      C y1, y2;
-      if (i < E / 2) {
-        y1 = x1[i], y2 = x2[i];
-      } else {
-        y1 = shfl_c(x1[E - 1 - i], mirror);
-        y2 = shfl_c(x2[E - 1 - i], mirror);
-        if (p == 0) {
-          y1 = i == E / 2 ? x1[E / 2] : x1[E - i];
-          y2 = i == E / 2 ? x2[E / 2] : x2[E - i];
-        }
-      }
-      v[i] = pack_pair<C, N>(n, y1, y2);
+    for (int o = P / 2; o; o >>= 1) {
+      mw = fmax(mw, __shfl_xor_sync(0xffffffffu, mw, o));
+      mo = fmax(mo, __shfl_xor_sync(0xffffffffu, mo, o));
     }
-    if (r < 2) load(f1s[r + 1] + line * pin, f2s[r + 1] + line * pin);
-    xw_fft<T, PL, true, AD, N>(v, s, LDC, h, p, true, a.tw, twt);
+    int ew = 0, eo = 0;
+    frexp(mw, &ew);
+    frexp(mo, &eo);
+    const int d = mw > 0 && mo > 0 ? max(-96, min(96, ew - eo)) : 0;
+    up = ldexp(T(1), d);
+    down = ldexp(T(1), -d);
 #pragma unroll
-    for (int i = 0; i < E; ++i) o[r][i] = v[i];
+    for (int i = 0; i <= H; ++i) xo[i] = mkc<C>(xo[i].x * up, xo[i].y * up);
+    V1 z[E];
+    pack(xw, xo, [&](int q, T r, T i) { z[EN::in_i(q)] = V1{r, i}; });
+    sync();
+    vfft<PL, true, AD>(z, w, s1, 0, p, twt, sync);
+    sync();
   }
   // (omega x u) s at the lane's rows, and the CFL maxima
+  const T sc = T(a.s);
   T m0 = 0, m1 = 0, m2 = 0;
-  C f[E];
-  T pz[E];
+  T px[E], py[E], pz[E];
 #pragma unroll
   for (int i = 0; i < E; ++i) {
-    const T u = o[0][i].x, v = o[0][i].y, w = o[1][i].x, oz = o[1][i].y * down, ox = o[2][i].x, oy = o[2][i].y;
-    f[i] = mkc<C>((oy * w - oz * v) * sc, (oz * u - ox * w) * sc);
+    const T u = u_[i], v = v_[i], ww = w[i].re, oz = w[i].im * down, ox = ox_[i], oy = oy_[i];
+    px[i] = (oy * ww - oz * v) * sc;
+    py[i] = (oz * u - ox * ww) * sc;
     pz[i] = (ox * v - oy * u) * sc;
     m0 = fmax(m0, fabs(u));
     m1 = fmax(m1, fabs(v));
-    m2 = fmax(m2, fabs(w));
+    m2 = fmax(m2, fabs(ww));
   }
-  // forward transforms and the unpacking of two real transforms per sequence:
-  // X1[k] = (Z[k] + conj Z[N-k]) / 2, X2[k] = (Z[k] - conj Z[N-k]) / 2i at k = p + 16 i <= N/2
-  auto unpack_store = [&](const C *z, C *d1, C *d2) {
+  // forward; rows k = p + P i <= N/2 of the half lines: of px + i py by
+  // X1 = (Z[k] + conj Z[N-k]) / 2, X2 = (Z[k] - conj Z[N-k]) / 2i, of pz its transform
+  C *const dx = a.NX + line * pout, *const dy = a.NY + line * pout, *const dz = a.NZ + line * pout;
+  auto store = [&](int i, T zr, T zi, T nr, T ni, bool xy, T fr, T fi, bool z) {
+    if (!(own >> i & 1)) return;
+    const int sl = i == H ? nyq : p + P * i;
+    if (xy) {
+      dx[sl] = mkc<C>(T(0.5) * (zr + nr), T(0.5) * (zi - ni));
+      dy[sl] = mkc<C>(T(0.5) * (zi + ni), T(0.5) * (nr - zr));
+    }
+    if (z) dz[sl] = mkc<C>(fr, fi);
+  };
+  if constexpr (PAIR) {
+    using V2 = VC<f2>;
+    V2 z[E], x[E];
 #pragma unroll
-    for (int i = 0; i <= E / 2; ++i) {
-      const int k = p + P * i;
-      C zn = shfl_c(z[(E - 1 - i) & (E - 1)], mirror);
-      if (p == 0) zn = z[(E - i) & (E - 1)];
-      const C zk = z[i];
-      if ((i < E / 2 || p == 0) && xkeep(a.kxa, k, N)) {
-        const int sl = xslot(a.nyq, k, N);
-        if (d1) d1[sl] = mkc<C>(T(0.5) * (zk.x + zn.x), T(0.5) * (zk.y - zn.y));
-        if (d2) d2[sl] = mkc<C>(T(0.5) * (zk.y + zn.y), T(-0.5) * (zk.x - zn.x));
+    for (int q = 0; q < E; ++q) {
+      const int i = EN::out_i(q);
+      z[EN::in_i(q)] = V2{mkf2(px[i], pz[i]), mkf2(py[i], T(0))};
+    }
+    vfft<PL, false, AD>(z, x, reinterpret_cast<V2 *>(tile), 0, p, twt, sync);
+#pragma unroll
+    for (int i = 0; i <= H; ++i) {
+      const V2 zk = x[EN::out_i(i)];
+      T nr = f2_lo(zk.re), ni = f2_lo(zk.im);   // i = H: row N/2, its own mirror
+      if (i < H) {
+        const V2 b = x[EN::out_i(E - 1 - i)], b0 = x[EN::out_i((E - i) % E)];
+        nr = shfl(p == 0 ? f2_lo(b0.re) : f2_lo(b.re));
+        ni = shfl(p == 0 ? f2_lo(b0.im) : f2_lo(b.im));
+      }
+      store(i, f2_lo(zk.re), f2_lo(zk.im), nr, ni, true, f2_hi(zk.re), f2_hi(zk.im), true);
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      V1 z[E], x[E];
+#pragma unroll
+      for (int q = 0; q < E; ++q) {
+        const int i = EN::out_i(q);
+        z[EN::in_i(q)] = k == 0 ? V1{px[i], py[i]} : V1{pz[i], T(0)};
+      }
+      if (k) sync();
+      vfft<PL, false, AD>(z, x, s1, 0, p, twt, sync);
+#pragma unroll
+      for (int i = 0; i <= H; ++i) {
+        const V1 zk = x[EN::out_i(i)];
+        T nr = zk.re, ni = zk.im;
+        if (k == 0 && i < H) {
+          const V1 b = x[EN::out_i(E - 1 - i)], b0 = x[EN::out_i((E - i) % E)];
+          nr = shfl(p == 0 ? b0.re : b.re);
+          ni = shfl(p == 0 ? b0.im : b.im);
+        }
+        store(i, zk.re, zk.im, nr, ni, k == 0, zk.re, zk.im, k == 1);
       }
     }
-  };
-  xw_fft<T, PL, false, AD, N>(f, s, LDC, h, p, true, a.tw, twt);
-  unpack_store(f, a.NX + line * pout, a.NY + line * pout);
-  // pz(a) + i pz(b) on both halves (the same sequence)
-#pragma unroll
-  for (int i = 0; i < E; ++i) {
-    const T other = __shfl_xor_sync(0xffffffffu, pz[i], 16);
-    f[i] = h == 0 ? mkc<C>(pz[i], other) : mkc<C>(other, pz[i]);
   }
-  xw_fft<T, PL, false, AD, N>(f, s, LDC, h, p, true, a.tw, twt);
-  unpack_store(f, h == 0 ? a.NZ + line * pout : nullptr, h == 1 ? a.NZ + line * pout : nullptr);
-  // CFL maxima of the pair (both lines lie in one box: ny*nz is even)
-  m0 = warp_max(m0);
-  m1 = warp_max(m1);
-  m2 = warp_max(m2);
-  if (lane == 0 && a.st) {
-    double *um = a.st[la / a.lines_per_box].umax;
-    atomic_max_nonneg(um + 0, (double)m0 * a.s);
-    atomic_max_nonneg(um + 1, (double)m1 * a.s);
-    atomic_max_nonneg(um + 2, (double)m2 * a.s);
+  if (on)
+    for (int j = p; j < a.npad; j += P) dx[nyq + 1 + j] = dy[nyq + 1 + j] = dz[nyq + 1 + j] = mkc<C>(0, 0);
+  // CFL maxima: of the lane's line, then of the warp's lines where they share a box
+  if (!a.st) return;
+#pragma unroll
+  for (int o = P / 2; o; o >>= 1) {
+    m0 = fmax(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+    m1 = fmax(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+    m2 = fmax(m2, __shfl_xor_sync(0xffffffffu, m2, o));
+  }
+  const int box = (int)((on ? line : (long long)a.nlines - 1) / a.lines_per_box);
+  bool lead = p == 0 && on;
+  if (P < 32 && __all_sync(0xffffffffu, box == __shfl_sync(0xffffffffu, box, 0))) {
+#pragma unroll
+    for (int o = 16; o >= P; o >>= 1) {
+      m0 = fmax(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+      m1 = fmax(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+      m2 = fmax(m2, __shfl_xor_sync(0xffffffffu, m2, o));
+    }
+    lead = lane == 0 && on;
+  }
+  if (lead) {
+    // only a larger value needs the atomic (the stored one never decreases)
+    double *um = a.st[box].umax;
+    const double x[3] = {(double)m0 * a.s, (double)m1 * a.s, (double)m2 * a.s};
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      if (!(x[c] <= __ldcg(um + c))) atomic_max_nonneg(um + c, x[c]);
   }
 }
 

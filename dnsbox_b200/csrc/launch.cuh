@@ -22,9 +22,8 @@ template <typename T, int N> struct Launcher {
   static cudaError_t strided_tma(const TmaArgs &a, bool inv, const void *adft, int *status, int nctas,
                                  cudaStream_t st);
   static bool has_tma();
-  // variant: 0 the default kernel for N, 1 the block kernel, 2 the warp kernel, 3 the warp kernel with
-  // each line's fields in registers (N = 256, FP32), 4 the same held to the registers of four resident
-  // blocks per SM; 3 and 4 run the warp kernel at other sizes
+  // variant: at lines whose fields fit a warp's registers (XReg) there is one kernel; at 512 in FP64
+  // 1 is the block kernel and anything else the warp kernel; at 1024 the block kernel
   static cudaError_t xline_nl(const XlineNLArgs<T> &a, int variant, cudaStream_t st);
   static bool has_xline_warp();
   static cudaError_t xline_c2r(const XlineArgs<T> &a, int nf, cudaStream_t st);
@@ -148,38 +147,33 @@ template <typename T, int N> bool Launcher<T, N>::has_xline_warp() { return Xlin
 template <typename T, int N>
 cudaError_t Launcher<T, N>::xline_nl(const XlineNLArgs<T> &a, int variant, cudaStream_t st) {
   using C = typename CT<T>::type;
-  if constexpr (XlineWarp<T, N>::on) {
-    if (variant != 1) {
-    // warp-granular kernel: one warp per line pair
-    constexpr int WPB = XlineWarp<T, N>::wpb;
-    constexpr int LDC = N + N / XlineWarp<T, N>::Plan::R[0];
-    const size_t smem = ((size_t)WPB * 6 * LDC + XlineWarp<T, N>::twn) * sizeof(C);
-    cudaError_t e;
-    const long long pairs = (a.nlines + 1) / 2;
-    const unsigned nb = (unsigned)((pairs + WPB - 1) / WPB);
-    if constexpr (N == 256 && sizeof(T) == 4) {
-      if (variant == 3 || variant == 4) {
-        // fields of a line in registers: two exchange columns per warp (4: held to
-        // 128 registers for four blocks per SM)
-        const size_t smem_r = ((size_t)WPB * 2 * LDC + XlineWarp<T, N>::twn) * sizeof(C);
-        auto kern = variant == 3 ? k_xline_nl_r<T> : k_xline_nl_r<T, 4>;
-        if ((e = set_smem(kern, smem_r)) != cudaSuccess) return e;
-        kern<<<nb, 32 * WPB, smem_r, st>>>(a);
+  cudaError_t e;
+  if constexpr (XReg<T, N>::on) {   // the only kernel for these lines, whatever the choice
+    using SH = XReg<T, N>;
+    // few lines: smaller blocks, so that every SM gets some
+    int nt = SH::NT;
+    while (nt > 32 && (long long)a.nlines * SH::PL::P < 148LL * 4 * nt) nt >>= 1;
+    const int lpb = nt / SH::PL::P;
+    if ((e = set_smem(k_xline_nl_g<T, N>, SH::smem(nt))) != cudaSuccess) return e;
+    k_xline_nl_g<T, N><<<(unsigned)((a.nlines + lpb - 1) / lpb), nt, SH::smem(nt), st>>>(a);
+  } else {
+    if constexpr (XlineWarp<T, N>::on) {
+      if (variant != 1) {   // one warp per line pair
+        constexpr int WPB = XlineWarp<T, N>::wpb;
+        constexpr int LDC = N + N / XlineWarp<T, N>::Plan::R[0];
+        const size_t smem = (size_t)WPB * 6 * LDC * sizeof(C);
+        const long long pairs = (a.nlines + 1) / 2;
+        if ((e = set_smem(k_xline_nl_w<T, N>, smem)) != cudaSuccess) return e;
+        k_xline_nl_w<T, N><<<(unsigned)((pairs + WPB - 1) / WPB), 32 * WPB, smem, st>>>(a);
         return cudaGetLastError();
       }
     }
-    if ((e = set_smem(k_xline_nl_w<T, N>, smem)) != cudaSuccess) return e;
-    k_xline_nl_w<T, N><<<nb, 32 * WPB, smem, st>>>(a);
-    return cudaGetLastError();
-    }
+    constexpr int B = XlineB<T, N>::v;
+    const size_t smem = (size_t)N * (3 * B + 1) * sizeof(C);
+    const int nt = round32(3 * B * (N / FftPlan<N>::E));
+    if ((e = set_smem(k_xline_nl<T, N>, smem)) != cudaSuccess) return e;
+    k_xline_nl<T, N><<<(unsigned)((a.nlines + B - 1) / B), nt, smem, st>>>(a);
   }
-  constexpr int B = XlineB<T, N>::v;
-  const size_t smem = (size_t)N * (3 * B + 1) * sizeof(C);
-  const int nt = round32(3 * B * (N / FftPlan<N>::E));
-  cudaError_t e;
-  if ((e = set_smem(k_xline_nl<T, N>, smem)) != cudaSuccess) return e;
-  const unsigned nb = (unsigned)((a.nlines + B - 1) / B);
-  k_xline_nl<T, N><<<nb, nt, smem, st>>>(a);
   return cudaGetLastError();
 }
 

@@ -7,9 +7,9 @@
 // differently across sizes are made by timing: for each of the tensor-core
 // strided passes (A inverse z, B inverse y, D forward y) of the tensor-core
 // form the cp.async-fed tensor-core kernel or the FP32 SIMT kernel (the
-// form's accuracy bars hold for both), and for the fused x pass the block
-// kernel or the warp kernel, and at 256 in FP32 the warp kernel that keeps each line's fields in
-// registers.  The TMA-staged tensor-core kernels (passes A, B, D and
+// form's accuracy bars hold for both), and for the fused x pass of 512-point
+// FP64 lines the block kernel or the warp kernel (other lines have one
+// kernel).  The TMA-staged tensor-core kernels (passes A, B, D and
 // E1) stay selectable by dnsbox_set_schedule but are not candidates: they
 // measured slower than both others at every size.  Each uniform candidate schedule advances a copy of the caller's
 // state for a few steps with pass timing on (CUDA events on the context's
@@ -152,7 +152,6 @@ extern "C" int dnsbox_autotune(dnsbox_ctx *ctx, const void *uh, int nsteps, dnsb
     tc_opts.push_back(2);   // the FP32 SIMT kernel
   std::vector<int> x_opts = {0};
   if (fp64 ? Ops<double>::has_xline_warp(p.nx) : Ops<float>::has_xline_warp(p.nx)) x_opts = {2, 1};
-  if (!fp64 && p.nx == 256) x_opts.insert(x_opts.end(), {3, 4});
   const dnsbox_schedule saved_sched = current(ctx);
   Saved sv;
   RET(save(ctx, sv));

@@ -382,10 +382,8 @@ typedef struct dnsbox_schedule {
   int32_t tc_kernel[4];   /* passes A (inverse z), B (inverse y), D (forward y): 0 TMA-staged tensor-core
                              kernel, 1 cp.async-fed one (the default), 2 FP32 SIMT kernel; [3] pass E1
                              (forward z): 0 SIMT (the default), 1 TMA-staged tensor-core kernel */
-  int32_t x_kernel;       /* fused x pass: 0 default for the size, 1 block kernel, 2 warp kernel,
-                             3 (N = 256, FP32) warp kernel with each line's fields in registers,
-                             4 the same held to 128 registers (four blocks per SM); 3 and 4 run the
-                             warp kernel at other sizes */
+  int32_t x_kernel;       /* fused x pass, 0 .. 4: a choice only at FP64 lines of 512 points, 1 the block
+                             kernel, any other the warp kernel; other lines have one kernel */
   int32_t tuned;          /* 1 when chosen by dnsbox_autotune */
   double ms_default;      /* step time of the default schedule in the tuning run (ms) */
   double ms_tuned;        /* step time of the chosen schedule (ms) */

@@ -1,0 +1,62 @@
+"""Every line length on each axis and layout of the right-hand side's passes: the x kernel's plans and its ragged last
+block, the strided kernel's plans, and the pruned (compact) workspace rows against the full ones."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import dnsbox_oracle as O
+
+pytestmark = pytest.mark.gpu
+SIZES = (8, 12, 16, 24, 32, 48, 64, 96, 128, 192, 256, 512, 1024)
+# the bars of the other right-hand-side tests: FP64 round-off of a transform chain, FP32 likewise
+TOL = {"fp64": 1e-12, "fp32": 2e-6}
+
+
+def rel(a, b):
+    return float(np.linalg.norm(np.asarray(a) - np.asarray(b)) / np.linalg.norm(np.asarray(b)))
+
+
+def rough(g, nx, ny, nz, seed):
+    rng = np.random.default_rng(seed)
+    return O.state_dealias(g, O.state_project(g, O.state_u2uhat(g, rng.standard_normal((3, nz, ny, nx)))))
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("axis", ["x", "y", "z"])
+@pytest.mark.parametrize("n", SIZES)
+def test_line_length(n, axis, prec):
+    from dnsbox_b200.ops import Box
+    nx, ny, nz = {"x": (n, 12, 8), "y": (12, n, 8), "z": (24, 8, n)}[axis]
+    kw = dict(nu=2e-3, kCutOff=2.5, Pin=0.1, bandlim=True)
+    g = O.Grid(O.Params(nx=nx, ny=ny, nz=nz, tstep_fix=True, **kw))
+    uh = rough(g, nx, ny, nz, seed=n)
+    b = Box(nx=nx, ny=ny, nz=nz, precision=prec, tstep_fix=True, dt=1e-3, **kw)
+    u = b.from_numpy(uh)
+    got, _ = b.rhs_nonlinear(u)   # the full passes
+    assert rel(got.cpu().numpy(), O.rhs_nonlinear(g, uh)) < TOL[prec]
+    b.step(u, 1)                  # the pruned passes
+    assert b.step_pruned()
+    assert rel(u.cpu().numpy(), O.heun_step(g, uh, 1e-3)) < 2 * TOL[prec]   # two right-hand sides
+    b.close()
+
+
+@pytest.mark.parametrize("nx", [8, 12, 24, 32])
+def test_maxima_of_boxes_sharing_a_warp(nx):
+    """144 lines a box: a warp's lines (32 P-lane groups at most) cross box boundaries."""
+    from dnsbox_b200.ops import Box
+    ny = nz = 12
+    kw = dict(nx=nx, ny=ny, nz=nz, nu=2e-3, bandlim=False, tstep_fix=True, dt=1e-3)
+    g = O.Grid(O.Params(nx=nx, ny=ny, nz=nz, bandlim=False))
+    fields = [rough(g, nx, ny, nz, seed=s) * (s + 1) for s in range(3)]
+    batch = Box(nbatch=3, **kw)
+    u = batch.zeros()
+    for i, f in enumerate(fields):
+        u[:, i] = torch.from_numpy(f).to(u.device)
+    recs = batch.step(u, 1)[0]
+    for i, f in enumerate(fields):
+        one = Box(**kw)
+        v = one.from_numpy(f)
+        assert one.step(v, 1)[0]["umax"] == recs[i]["umax"]
+        assert torch.equal(v, u[:, i])
+        one.close()
+    batch.close()
