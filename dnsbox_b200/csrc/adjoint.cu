@@ -478,8 +478,7 @@ int vjp_impl(dnsbox_ctx *c, const void *uh, const void *g, void *out) {
                                               reinterpret_cast<C *>(out), nh, gr, s);
   CK(cudaGetLastError());
   if (p.bandlim && c->nband) {
-    k_eband<C><<<1, 256, 0, c->stream>>>(reinterpret_cast<const C *>(uh), nh, c->band, c->nband, p.nx, c->st,
-                                         s * s, 0);
+    k_eband<C><<<1, 256, 0, c->stream>>>(band_args(c, uh), p.nx, 0);
     k_vjp_band<C><<<1, 256, 0, c->stream>>>(reinterpret_cast<const C *>(uh), reinterpret_cast<const C *>(g),
                                             reinterpret_cast<C *>(out), nh, c->band, c->nband, gr, c->st, p.Pin,
                                             s * s);

@@ -66,45 +66,32 @@ extern "C" void dnsbox_default_params(dnsbox_params *p) {
 }
 
 // ------------------------------------------------------------ small kernels
-// io_Courant (io.f90:664-676) on the fused max|u_i| and, when control is on,
-// set_time_step (dnsboxheun.f90:153-157, 227-246).
-__global__ void k_cfl(StepState *sts, int nbatch, double dx, double dy, double dz, int control, int force,
-                      double cmin, double cmax, double dtmax, dnsbox_diag *ring, int ring_cap) {
+// The CFL update of every box as a launch of its own (a pass D that does not
+// run the SIMT kernel on workspace rows).
+__global__ void k_cfl(StepState *sts, int nbatch, CflArgs cfl) {
+  pdl_launch();
+  pdl_wait();
   const int box = blockIdx.x * blockDim.x + threadIdx.x;
   if (box >= nbatch) return;
-  StepState *st = sts + box;
-  dnsbox_diag *drec = ring ? ring + ((long long)st->step % ring_cap) * nbatch + box : nullptr;
-  double dt = st->dt;
-  double C = st->umax[0] * dt / dx + st->umax[1] * dt / dy + st->umax[2] * dt / dz;
-  if (control && (force || C > cmax || (C < cmin && dt < dtmax))) {
-    double nd = ((cmax + cmin) / (2.0 * C)) * dt;
-    if (nd > dtmax) nd = dtmax;
-    C = C * nd / dt;
-    st->dt = nd;
-    dt = nd;
-  }
-  st->courant = C;
-  st->eband1 = st->eband;
-  if (drec) {
-    drec->courant = C;
-    drec->umax[0] = st->umax[0];
-    drec->umax[1] = st->umax[1];
-    drec->umax[2] = st->umax[2];
-    drec->eband = st->eband;
-    drec->dt = dt;
-  }
+  cfl_update(cfl, sts + box, box, nbatch);
 }
 
-// Sums the finish-kernel partials (fixed order), writes the step record and
-// advances the clock.
-// Per-plane sums of the spectral finish's row partials: block (kz, box) adds
-// the (E, D) pairs of the ny rows of plane kz in a fixed order.  Rows and
-// planes outside the kept ky / kz sets of a pruned step were not visited and
-// count as zero.
-__global__ void k_plane_sums(const double *rows, double *planes, int nz, int ny, AxisKeep ky, AxisKeep kz) {
+// The step record from the finish kernel's row partials.  Block (kz, box) adds
+// the (E, D) pairs of the ny rows of plane kz in a fixed order; the last block
+// of a box adds the planes in a fixed order, writes the record and advances
+// the clock.  Rows and planes outside the kept ky / kz sets of a pruned step
+// were not visited and count as zero.
+__global__ void k_step_record(StepState *sts, const double *rows, double *planes, int nz, int ny, AxisKeep ky,
+                              AxisKeep kz, double s2, double nu, const double *nu_box, double Q, double Pin,
+                              int bandlim, dnsbox_diag *ring, int ring_cap) {
   __shared__ double red[2 * 32];
-  const int iz = blockIdx.x, box = blockIdx.y;
+  __shared__ bool last;
+  pdl_launch();
+  pdl_wait();
+  const int iz = blockIdx.x, box = blockIdx.y, nbatch = gridDim.y;
+  StepState *st = sts + box;
   const double *r = rows + 2 * ((long long)box * nz + iz) * ny;
+  planes += 2 * (long long)box * nz;
   double e = 0.0, d = 0.0;
   if (kz.keep(iz))
     for (int j = threadIdx.x; j < ny; j += blockDim.x)
@@ -115,29 +102,24 @@ __global__ void k_plane_sums(const double *rows, double *planes, int nz, int ny,
   double v[2] = {e, d};
   block_sum<2>(v, red);
   if (threadIdx.x == 0) {
-    planes[2 * ((long long)box * nz + iz)] = v[0];
-    planes[2 * ((long long)box * nz + iz) + 1] = v[1];
+    planes[2 * iz] = v[0];
+    planes[2 * iz + 1] = v[1];
+    __threadfence();
+    last = atomicAdd(&st->rec_done, 1u) == (unsigned)nz - 1;
   }
-}
-
-// one block per box; partials: np (E, D) pairs per box (the plane sums)
-__global__ void k_finalize(StepState *sts, const double *partials, int np, double s2, double nu,
-                           const double *nu_box, double Q, double Pin, int bandlim, dnsbox_diag *ring,
-                           int ring_cap) {
-  __shared__ double red[2 * 32];
-  const int box = blockIdx.x, nbatch = gridDim.x;
-  StepState *st = sts + box;
-  partials += 2 * (long long)box * np;
-  if (nu_box) nu = nu_box[box];
-  dnsbox_diag *drec = ring ? ring + ((long long)st->step % ring_cap) * nbatch + box : nullptr;
-  double e = 0.0, d = 0.0;
-  for (int i = threadIdx.x; i < np; i += blockDim.x) {
-    e += partials[2 * i];
-    d += partials[2 * i + 1];
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  e = d = 0.0;
+  for (int i = threadIdx.x; i < nz; i += blockDim.x) {
+    e += __ldcg(planes + 2 * i);
+    d += __ldcg(planes + 2 * i + 1);
   }
-  double v[2] = {e, d};
+  v[0] = e, v[1] = d;
   block_sum<2>(v, red);
   if (threadIdx.x == 0) {
+    if (nu_box) nu = nu_box[box];
+    dnsbox_diag *drec = ring ? ring + ((long long)st->step % ring_cap) * nbatch + box : nullptr;
     const double E = v[0] * s2, D = nu * v[1] * s2;
     const double dt = st->dt;
     if (drec) {
@@ -153,12 +135,8 @@ __global__ void k_finalize(StepState *sts, const double *partials, int np, doubl
     st->t_prev = st->t;
     st->t = st->t + dt;
     st->step += 1.0;
+    st->rec_done = 0;
   }
-}
-
-__global__ void k_reset_umax(StepState *st, int nbatch) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b < nbatch) st[b].umax[0] = st[b].umax[1] = st[b].umax[2] = 0.0;
 }
 
 // sets the double at byte offset `off` of every box's StepState
@@ -590,7 +568,7 @@ template <typename T> static FinishArgs<T> finish_base(const dnsbox_ctx *c) {
   f.nu = p.nu;
   f.Q = p.Q;
   f.Pin = p.Pin;
-  f.kcut = p.kCutOff;
+  f.kcut2 = kcut2_of(p.kCutOff);
   // rhs.f90:74-88
   f.cutx = (p.nx / 2.0) * (2.0 * p.alpha_x / 3.0);
   f.cuty = (p.ny / 2.0) * (2.0 * p.alpha_y / 3.0);
@@ -612,20 +590,20 @@ static int run_rhs(dnsbox_ctx *c, const void *uin, int mode, void *out, void *st
   using C = typename CT<T>::type;
   const dnsbox_params &p = c->p;
   const double s = 1.0 / ((double)p.nx * p.ny * p.nz);
-  // rhs_Eband (rhs.f90:22-24) and reset of the CFL maxima
-  if (p.bandlim) {
-    Prof pr(c, DNSBOX_PASS_SMALL);
-    k_eband<C><<<c->nbatch, 256, 0, c->stream>>>(reinterpret_cast<const C *>(uin), (long long)c->fstride, c->band,
-                                                 c->nband, p.nx, c->st, s * s, 1, (long long)c->nh);
-  } else {
-    Prof pr(c, DNSBOX_PASS_SMALL);
-    k_reset_umax<<<(c->nbatch + 127) / 128, 128, 0, c->stream>>>(c->st, c->nbatch);
-  }
-  CK(cudaGetLastError());
   const char *u = reinterpret_cast<const char *>(uin);
   // pruned passes on the SIMT kernel keep the workspace in compact rows
   const bool compact = pruned && strided_simt<T>(c);
   const int wp = ws_pitch(c, compact);
+  // rhs_Eband (rhs.f90:22-24): a block of pass A where that runs the SIMT
+  // kernel on workspace rows, else a launch
+  auto simt = [&](int i, int n) {
+    return (!c->tc || !Ops<T>::has_tc(n) || c->sched_tc[i] == 2) && (!pruned || compact);
+  };
+  const bool band = p.bandlim && c->nband, band_in_a = band && simt(0, p.nz);
+  if (band && !band_in_a) {
+    Prof pr(c, DNSBOX_PASS_SMALL);
+    CK(launch_pdl(k_eband<C>, c->nbatch, 256, 0, c->stream, band_args(c, uin), p.nx, 0));
+  }
   // pass A: inverse z
   StridedArgs<T> a = strided_base<T>(c, 2);
   a.njobs = 5;
@@ -640,6 +618,7 @@ static int run_rhs(dnsbox_ctx *c, const void *uin, int mode, void *out, void *st
     a.koth = c->keep[1];
     a.krin = c->keep[2];
   }
+  if (band_in_a) a.band = band_args(c, uin);
   RET(run_strided<T>(c, 2, true, a, DNSBOX_PASS_Z_INV, true, uin, 3));
   // pass B: inverse y
   StridedArgs<T> b = strided_base<T>(c, 1);
@@ -676,7 +655,7 @@ static int run_rhs(dnsbox_ctx *c, const void *uin, int mode, void *out, void *st
   }
   x.status = c->tc_status;
   x.tw = reinterpret_cast<const C *>(c->tw[0]);
-  x.st = c->st;
+  x.st = cfl ? c->st : nullptr;   // the CFL maxima, where they are used
   x.lines_per_box = p.ny * p.nz;
   x.nlines = c->nbatch * p.ny * p.nz;
   x.nxh = c->nxh;
@@ -687,16 +666,6 @@ static int run_rhs(dnsbox_ctx *c, const void *uin, int mode, void *out, void *st
     Prof pr(c, DNSBOX_PASS_X_NL);
     CK(Ops<T>::xline_nl(p.nx, x, c->sched_x, c->stream));
   }
-  if (cfl) {
-    const double dx = (2 * M_PI / p.alpha_x) / p.nx, dy = (2 * M_PI / p.alpha_y) / p.ny,
-                 dz = (2 * M_PI / p.alpha_z) / p.nz;
-    Prof pr(c, DNSBOX_PASS_SMALL);
-    k_cfl<<<(c->nbatch + 127) / 128, 128, 0, c->stream>>>(c->st, c->nbatch, dx, dy, dz, !p.tstep_fix,
-                                                          c->cfl_first, p.courant_min, p.courant_max, p.dt_max,
-                                                          c->ddiag, c->ring_cap);
-    CK(cudaGetLastError());
-    c->cfl_first = 0;
-  }
   // pass D: forward y
   StridedArgs<T> d = strided_base<T>(c, 1);
   strided_ws<T>(c, d, 1, true, true, compact);
@@ -705,6 +674,19 @@ static int run_rhs(dnsbox_ctx *c, const void *uin, int mode, void *out, void *st
   if (pruned) {   // only kept kx columns; ky rows outside the kept set are masked by the finish
     d.kcol = c->keep[0];
     d.krout = c->keep[1];
+  }
+  if (cfl) {   // the CFL update: a block of pass D on the SIMT kernel, else a launch
+    const CflArgs g{1, !p.tstep_fix, c->cfl_first, c->ring_cap, (2 * M_PI / p.alpha_x) / p.nx,
+                    (2 * M_PI / p.alpha_y) / p.ny, (2 * M_PI / p.alpha_z) / p.nz, p.courant_min, p.courant_max,
+                    p.dt_max, c->ddiag};
+    if (simt(2, p.ny)) {
+      d.cfl = g;
+      d.st = c->st;
+    } else {
+      Prof pr(c, DNSBOX_PASS_SMALL);
+      CK(launch_pdl(k_cfl, (c->nbatch + 127) / 128, 128, 0, c->stream, c->st, c->nbatch, g));
+    }
+    c->cfl_first = 0;
   }
   RET(run_strided<T>(c, 1, false, d, DNSBOX_PASS_Y_FWD, true, c->W1, 6));
   // pass E1: forward z of the three components, in place (the SIMT kernel in
@@ -743,10 +725,10 @@ static int run_rhs(dnsbox_ctx *c, const void *uin, int mode, void *out, void *st
   Prof pr(c, DNSBOX_PASS_Z_FIN);
   const dim3 grid((unsigned)((nrows + 7) / 8), (unsigned)c->nbatch);
   switch (mode) {
-    case FIN_RHS: k_finish_rows<T, FIN_RHS><<<grid, 256, 0, c->stream>>>(e, nrows); break;
-    case FIN_PRED: k_finish_rows<T, FIN_PRED><<<grid, 256, 0, c->stream>>>(e, nrows); break;
-    case FIN_CORR: k_finish_rows<T, FIN_CORR><<<grid, 256, 0, c->stream>>>(e, nrows); break;
-    default: k_finish_rows<T, FIN_AB2><<<grid, 256, 0, c->stream>>>(e, nrows); break;
+    case FIN_RHS: CK(launch_pdl(k_finish_rows<T, FIN_RHS>, grid, 256, 0, c->stream, e, nrows)); break;
+    case FIN_PRED: CK(launch_pdl(k_finish_rows<T, FIN_PRED>, grid, 256, 0, c->stream, e, nrows)); break;
+    case FIN_CORR: CK(launch_pdl(k_finish_rows<T, FIN_CORR>, grid, 256, 0, c->stream, e, nrows)); break;
+    default: CK(launch_pdl(k_finish_rows<T, FIN_AB2>, grid, 256, 0, c->stream, e, nrows)); break;
   }
   CK(cudaGetLastError());
   return DNSBOX_OK;
@@ -1031,13 +1013,9 @@ template <typename T> static int step_once(dnsbox_ctx *c, void *uh) {
   const AxisKeep ky = rows_pruned ? c->keep[1] : AxisKeep{0, p.ny, 1};
   const AxisKeep kz = rows_pruned ? c->keep[2] : AxisKeep{0, p.nz, 1};
   double *planes = c->partials + 2 * (size_t)c->npartials * c->nbatch;
-  Prof pr(c, DNSBOX_PASS_SMALL, 2);
-  k_plane_sums<<<dim3((unsigned)p.nz, (unsigned)c->nbatch), 256, 0, c->stream>>>(c->partials, planes, p.nz, p.ny, ky,
-                                                                                 kz);
-  CK(cudaGetLastError());
-  k_finalize<<<c->nbatch, 1024, 0, c->stream>>>(c->st, planes, p.nz, s * s, p.nu, c->d_nu, p.Q, p.Pin, p.bandlim,
-                                                 c->ddiag, c->ring_cap);
-  CK(cudaGetLastError());
+  Prof pr(c, DNSBOX_PASS_SMALL);
+  CK(launch_pdl(k_step_record, dim3((unsigned)p.nz, (unsigned)c->nbatch), 256, 0, c->stream, c->st, c->partials, planes,
+                p.nz, p.ny, ky, kz, s * s, p.nu, c->d_nu, p.Q, p.Pin, p.bandlim, c->ddiag, c->ring_cap));
   c->host_step += 1;
   return DNSBOX_OK;
 }
@@ -1565,12 +1543,8 @@ extern "C" int dnsbox_eband(dnsbox_ctx *ctx, const void *uh, double *eband) {
     *eband = 0.0;
     return DNSBOX_OK;
   }
-  if (ctx->fp64)
-    k_eband<double2><<<1, 256, 0, ctx->stream>>>((const double2 *)uh, (long long)ctx->nh, ctx->band,
-                                                 ctx->nband, p.nx, ctx->st, s * s, 0);
-  else
-    k_eband<float2><<<1, 256, 0, ctx->stream>>>((const float2 *)uh, (long long)ctx->nh, ctx->band, ctx->nband,
-                                                p.nx, ctx->st, s * s, 0);
+  if (ctx->fp64) k_eband<double2><<<1, 256, 0, ctx->stream>>>(band_args(ctx, uh), p.nx, 0);
+  else k_eband<float2><<<1, 256, 0, ctx->stream>>>(band_args(ctx, uh), p.nx, 0);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(ctx->hstage, &ctx->st->eband, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));

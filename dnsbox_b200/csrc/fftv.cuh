@@ -349,14 +349,20 @@ template <> struct VtwOf<VC<float>> {
 template <> struct VtwOf<VC<f2>> {
   __device__ static __forceinline__ VC<f2> of(float2 w) { return VC<f2>{mkf2(w.x, w.x), mkf2(w.y, w.y)}; }
 };
-// from the N-point table exp(-2 pi i k / N); all threads of the block
-template <class PL, typename V, typename C, int S = 1>
-__device__ __forceinline__ void vtw_fill(V *t, const C *__restrict__ tw, int tid, int nthreads) {
-  if constexpr (S < PL::NST) {
-    constexpr int NS = PL::ns(S), R = PL::R[S], TS = PL::N / (NS * R);
-    for (int i = tid; i < (R - 1) * NS; i += nthreads) t[vtw_off<PL, S>() + i] = VtwOf<V>::of(tw[(1 + i / NS) * (i % NS) * TS]);
-    vtw_fill<PL, V, C, S + 1>(t, tw, tid, nthreads);
+// Entry i of the tables, from the N-point table exp(-2 pi i k / N).
+template <class PL, int S = 1, typename C> __device__ __forceinline__ C vtw_entry(const C *__restrict__ tw, int i) {
+  static_assert(S < PL::NST, "a plan of one stage has no twiddles");
+  constexpr int NS = PL::ns(S), R = PL::R[S], TS = PL::N / (NS * R);
+  if constexpr (S + 1 < PL::NST) {
+    if (i >= (R - 1) * NS) return vtw_entry<PL, S + 1>(tw, i - (R - 1) * NS);
   }
+  return __ldg(tw + (1 + i / NS) * (i % NS) * TS);
+}
+// All tables, by all threads of the block.
+template <class PL, typename V, typename C>
+__device__ __forceinline__ void vtw_fill(V *t, const C *__restrict__ tw, int tid, int nthreads) {
+  if constexpr (PL::NST > 1)
+    for (int i = tid; i < vtw_size<PL>(); i += nthreads) t[i] = VtwOf<V>::of(vtw_entry<PL>(tw, i));
 }
 
 template <bool INV, typename V> __device__ __forceinline__ V vtwmul(V a, V w) {

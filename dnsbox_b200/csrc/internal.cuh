@@ -149,33 +149,13 @@ struct Prof {
 };
 
 // ------------------------------------------------------------ shared kernels
-// rhs_Eband (rhs.f90:137-168) over the precomputed band-mode list, stored as
-// (offset lo, offset hi, kx) triples; optionally resets the CFL maxima.
-// One block per box: u + box * bstride, components fstride apart.
-template <typename C>
-__global__ void k_eband(const C *u, long long nh, const int *band, int nband, int nx, StepState *st, double s2,
-                        int reset_umax, long long bstride = 0) {
+// rhs_Eband (rhs.f90:137-168) over the precomputed band-mode list; optionally
+// resets the CFL maxima.  One block per box.
+template <typename C> __global__ void k_eband(BandArgs b, int nx, int reset_umax) {
   __shared__ double red[32];
-  u += (long long)blockIdx.x * bstride;
-  st += blockIdx.x;
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < nband; i += blockDim.x) {
-    const long long off = (long long)(unsigned)band[3 * i] | ((long long)band[3 * i + 1] << 32);
-    const int kx = band[3 * i + 2];
-    const double w = (k_half(kx, nx, 1.0) == 0.0) ? 0.5 : 1.0;   // rhs.f90:151-155
-    double e = 0.0;
-    for (int c = 0; c < 3; ++c) {
-      const C v = u[c * nh + off];
-      e += ((double)v.x * v.x + (double)v.y * v.y) * w;
-    }
-    acc += e;
-  }
-  double v[1] = {acc};
-  block_sum<1>(v, red);
-  if (threadIdx.x == 0) {
-    st->eband = v[0] * s2;
-    if (reset_umax) st->umax[0] = st->umax[1] = st->umax[2] = 0.0;
-  }
+  pdl_launch();
+  pdl_wait();
+  eband_block<C>(b, nx, blockIdx.x, reset_umax, red);
 }
 
 // Sum of n doubles in a fixed order (one block).
@@ -419,6 +399,12 @@ template <typename T> static bool strided_simt(const dnsbox_ctx *c) {
   for (int i = 0; i < 3; ++i)
     if (c->sched_tc[i] != 2 && Ops<T>::has_tc(n[i])) return false;
   return c->sched_tc[3] == 0;
+}
+
+// The band-energy arguments of a state (boxes nh apart, components fstride).
+static inline BandArgs band_args(const dnsbox_ctx *c, const void *u) {
+  const double s = 1.0 / ((double)c->p.nx * c->p.ny * c->p.nz);
+  return BandArgs{c->band, c->nband, s * s, c->st, u, (long long)c->fstride, (long long)c->nh};
 }
 
 // One output of a batched C2R: sum over terms of in * (a + i b k), with k

@@ -15,8 +15,10 @@
 // stepper and the energy/dissipation row sums (k_finish_rows).
 #pragma once
 
+#include <cmath>
 #include <type_traits>
 
+#include "../../include/dnsbox.h"
 #include "common.cuh"
 #include "fft.cuh"
 #include "fftv.cuh"
@@ -41,8 +43,86 @@ struct StepState {
   double courant;   // io_Courant of the step's initial state with dt
   double eband1;    // eband of the step's first RHS (for the diagnostics)
   double step;      // step counter
-  double pad[6];
+  unsigned rec_done, pad0;   // planes of the step record that are through (0 between launches)
+  double pad[5];
 };
+
+// Programmatic dependent launch: a kernel launched with launch_pdl may start
+// while its predecessor's last blocks run, so its launch and its prologue
+// (indices, twiddle tables) are hidden; it waits for the predecessor's end
+// before it touches memory any kernel writes.  Every kernel so launched lets
+// its own successor start early too, and waits before anything else it does
+// on global memory but read constant tables.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// io_Courant (io.f90:664-676) on the fused max|u_i| of one box and, when
+// control is on, set_time_step (dnsboxheun.f90:153-157, 227-246).  The maxima
+// are consumed: they start the next right-hand side at zero.
+struct CflArgs {
+  int on, control, force, ring_cap;
+  double dx, dy, dz, cmin, cmax, dtmax;
+  dnsbox_diag *ring;
+};
+__device__ __forceinline__ void cfl_update(const CflArgs &c, StepState *st, int box, int nbatch) {
+  const double umax[3] = {st->umax[0], st->umax[1], st->umax[2]};
+  dnsbox_diag *drec = c.ring ? c.ring + ((long long)st->step % c.ring_cap) * nbatch + box : nullptr;
+  double dt = st->dt;
+  double C = umax[0] * dt / c.dx + umax[1] * dt / c.dy + umax[2] * dt / c.dz;
+  if (c.control && (c.force || C > c.cmax || (C < c.cmin && dt < c.dtmax))) {
+    double nd = ((c.cmax + c.cmin) / (2.0 * C)) * dt;
+    if (nd > c.dtmax) nd = c.dtmax;
+    C = C * nd / dt;
+    st->dt = nd;
+    dt = nd;
+  }
+  st->courant = C;
+  st->eband1 = st->eband;
+  if (drec) {
+    drec->courant = C;
+    drec->umax[0] = umax[0];
+    drec->umax[1] = umax[1];
+    drec->umax[2] = umax[2];
+    drec->eband = st->eband;
+    drec->dt = dt;
+  }
+  st->umax[0] = st->umax[1] = st->umax[2] = 0.0;   // for the next right-hand side that takes the maxima
+}
+
+// The band modes of rhs_Eband, (offset lo, offset hi, kx) triples.
+struct BandArgs {
+  const int *modes;
+  int n;            // 0: none
+  double s2;
+  StepState *st;
+  const void *u;    // the right-hand side's input, components nh apart, boxes bstride apart
+  long long nh, bstride;
+};
+// rhs_Eband (rhs.f90:137-168) of box `box` by one block (red: 32 doubles);
+// optionally resets the CFL maxima.
+template <typename C>
+__device__ __forceinline__ void eband_block(const BandArgs &b, int nx, int box, bool reset_umax, double *red) {
+  const C *u = reinterpret_cast<const C *>(b.u) + (long long)box * b.bstride;
+  StepState *st = b.st + box;
+  double acc = 0.0;
+  for (int i = threadIdx.x; i < b.n; i += blockDim.x) {
+    const long long off = (long long)(unsigned)b.modes[3 * i] | ((long long)b.modes[3 * i + 1] << 32);
+    const int kx = b.modes[3 * i + 2];
+    const double w = (k_half(kx, nx, 1.0) == 0.0) ? 0.5 : 1.0;   // rhs.f90:151-155
+    double e = 0.0;
+    for (int c = 0; c < 3; ++c) {
+      const C v = u[c * b.nh + off];
+      e += ((double)v.x * v.x + (double)v.y * v.y) * w;
+    }
+    acc += e;
+  }
+  double v[1] = {acc};
+  block_sum<1>(v, red);
+  if (threadIdx.x == 0) {
+    st->eband = v[0] * b.s2;
+    if (reset_umax) st->umax[0] = st->umax[1] = st->umax[2] = 0.0;
+  }
+}
 
 // Pruning of the 2/3-rule zeros.  On an axis of length n the dealiasing mask
 // (rhs.f90:74-88) keeps index i when |k_i| < (n/2)(2/3) alpha, i.e. i < a, the
@@ -107,6 +187,9 @@ template <typename T> struct StridedArgs {
   // of nslot columns start on 128-byte boundaries; with column pruning the
   // workspace is compact: slot kcol.a holds the Nyquist column (compact = 1)
   int ws, compact, nslot, pad;
+  BandArgs band;   // band.n: one more block per box (the last) computes the band energy
+  CflArgs cfl;     // cfl.on: likewise (forward passes), the CFL update of the box
+  StepState *st;   // step states, with cfl.on
 };
 
 // Output strides of a strided launch (the input's where unset).
@@ -143,7 +226,8 @@ template <typename T, int N> struct StridedShape {
   static constexpr int NT = W * PL::P;
   static constexpr size_t tile = PL::NST > 1 ? (size_t)N * W * 16 : 0;
   static constexpr size_t smem(bool inv) {   // tile, twiddles and (inverse) row multipliers
-    return tile + (size_t)vtw_size<PL>() * 16 + (inv ? 2 * N * sizeof(T) : 0);
+    const size_t n = tile + (size_t)vtw_size<PL>() * 16 + (inv ? 2 * N * sizeof(T) : 0);
+    return n < 256 ? 256 : n;   // 32 doubles for the band block
   }
   // Resident CTAs asked of the register allocator: 16 warps per SM where a
   // thread holds 16 values (128 registers), 20 at 12 (96), 24 at 8 (80), 32 in
@@ -280,6 +364,21 @@ __global__ void __launch_bounds__(StridedShape<T, N>::NT, StridedShape<T, N>::mi
   V *s = reinterpret_cast<V *>(smem_raw);
   V *twt = reinterpret_cast<V *>(smem_raw + SH::tile);
   T *bks = reinterpret_cast<T *>(smem_raw + SH::tile + (size_t)vtw_size<PL>() * 16);
+  pdl_launch();
+  if constexpr (INV && MODE == ST_TO_WS) {
+    if (a.band.n && blockIdx.x == gridDim.x - 1) {
+      pdl_wait();
+      eband_block<C>(a.band, a.nx, blockIdx.y, false, reinterpret_cast<double *>(smem_raw));
+      return;
+    }
+  }
+  if constexpr (!INV && MODE == ST_WS) {
+    if (a.cfl.on && blockIdx.x == gridDim.x - 1) {
+      pdl_wait();
+      if (threadIdx.x == 0) cfl_update(a.cfl, a.st + blockIdx.y, blockIdx.y, gridDim.y);
+      return;
+    }
+  }
   const int job = blockIdx.x % a.njobs;
   const int tile = blockIdx.x / a.njobs;
   int kx0, other;
@@ -306,6 +405,15 @@ __global__ void __launch_bounds__(StridedShape<T, N>::NT, StridedShape<T, N>::mi
       else x[q - Q0] = IO::load2(q0, q0 + (c1 - c0), v0 && k, v1 && k);
     }
   };
+  // twiddles: read before the wait, stored once the rows are on their way
+  constexpr int NTW = (vtw_size<PL>() + SH::NT - 1) / SH::NT;
+  C tws[NTW > 0 ? NTW : 1];
+  if constexpr (NTW > 0) {
+#pragma unroll
+    for (int i = 0; i < NTW; ++i)
+      if ((int)threadIdx.x + i * SH::NT < vtw_size<PL>()) tws[i] = vtw_entry<PL>(a.tw, threadIdx.x + i * SH::NT);
+  }
+  pdl_wait();
   Raw v[E];   // row p + P q in v[in_i(q)]
   {
     Raw x[E];
@@ -322,7 +430,11 @@ __global__ void __launch_bounds__(StridedShape<T, N>::NT, StridedShape<T, N>::mi
   if (INV && in2p) load(in2p, w, 0, QN);
   // with the rows on their way: the twiddle tables (read after the exchange's
   // barrier) and the job's row multipliers T(b k_row(n)) (ks == 1)
-  vtw_fill<PL, V>(twt, a.tw, threadIdx.x, SH::NT);
+  if constexpr (NTW > 0) {
+#pragma unroll
+    for (int i = 0; i < NTW; ++i)
+      if ((int)threadIdx.x + i * SH::NT < vtw_size<PL>()) twt[threadIdx.x + i * SH::NT] = VtwOf<V>::of(tws[i]);
+  }
   if constexpr (INV) {
     const bool mult1 = !(jb.a1 == 1.0 && jb.b1 == 0.0);
     const bool rows1 = mult1 && jb.ks1 == 1, rows2 = in2p && jb.ks2 == 1;
@@ -827,8 +939,10 @@ __global__ void __launch_bounds__(XReg<T, N>::NT, XReg<T, N>::minb)
   constexpr bool PAIR = sizeof(T) == 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V1 *twt = reinterpret_cast<V1 *>(smem_raw);
+  pdl_launch();
   vtw_fill<PL, V1>(twt, a.tw, threadIdx.x, blockDim.x);
   __syncthreads();
+  pdl_wait();
   const int g = threadIdx.x / P, p = threadIdx.x % P, lane = threadIdx.x & 31;
   unsigned char *tile = smem_raw + SH::tw + (size_t)g * SH::line;
   V1 *s1 = reinterpret_cast<V1 *>(tile);
@@ -1162,7 +1276,8 @@ template <typename T> struct FinishArgs {
   long long bstride;       // elements between boxes
   int nx, ny, nz, nxh;
   double ax, ay, az;
-  double nu, Q, Pin, kcut;
+  double nu, Q, Pin;
+  double kcut2;            // largest k.k whose root is at most kCutOff (kcut2_of)
   double cutx, cuty, cutz, sph2;
   int bandlim, spherical, mode, ab2_standard;
   double s;                // scalemodes
@@ -1175,6 +1290,17 @@ template <typename T> struct FinishArgs {
   // an axis of ny_k rows (0, 0: the box's own rows)
   int ky0, ny_k;
 };
+
+// The largest double whose square root is at most kcut (both roundings are
+// IEEE), so that k.k <= kcut2_of(kcut) decides sqrt(k.k) <= kcut without a
+// double-precision root per mode; -1 for a negative cut-off.
+inline double kcut2_of(double kcut) {
+  if (!(kcut >= 0.0)) return -1.0;
+  double t = kcut * kcut;
+  while (std::sqrt(t) > kcut) t = std::nextafter(t, 0.0);
+  while (std::isfinite(t) && std::sqrt(std::nextafter(t, HUGE_VAL)) <= kcut) t = std::nextafter(t, HUGE_VAL);
+  return t;
+}
 
 // Spectral finish after the forward z transform (the second half of one
 // right-hand side's pass E): per mode the 2/3 mask, the pressure projection,
@@ -1198,18 +1324,38 @@ __global__ void __launch_bounds__(256, FinishMinB<T, MODE>::v)
     k_finish_rows(const __grid_constant__ FinishArgs<T> a, int nrows) {
   using C = typename CT<T>::type;
   constexpr int CH = 2;
+  pdl_launch();
   const int lane = threadIdx.x & 31;
   const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= nrows) return;   // whole warps: no block-level synchronisation below
-  const int nky = a.ky.count();
-  const int oz = w / nky;
-  const int kz = a.kz.map(oz), ky = a.ky.map(w - oz * nky);
+  // rows by ky, last ky first (the order in which pass E1 wrote them, the
+  // newest still in L2), kz within
+  const int nkz = a.kz.count();
+  const int oy = w / nkz;
+  const int ky = a.ky.map(a.ky.count() - 1 - oy), kz = a.kz.map(w - oy * nkz);
   const int box = blockIdx.y;
   const long long rowbase = ((long long)kz * a.ny + ky) * a.nxh + (long long)box * a.bstride;
   const long long n3nh = a.n3_nh ? a.n3_nh : a.nh;
   const long long n3row = ((long long)kz * a.ny + ky) * (a.n3_pitch ? a.n3_pitch : a.nxh) +
                           (long long)box * (a.n3_bstride ? a.n3_bstride : a.bstride);
+  const double kyr = k_full(a.ky0 + ky, a.ny_k ? a.ny_k : a.ny, a.ay);
+  const double kzr = k_full(kz, a.nz, a.az);
+  const bool rowcut = fabs(kyr) >= a.cuty || fabs(kzr) >= a.cutz;
+  const bool need_u = a.bandlim || MODE != FIN_RHS;
+  // kept kx, ascending per lane as in a full launch (so that the sums agree bit
+  // for bit): lane, lane + 32, .. below lim, then in its lane the Nyquist column
+  const int lim = a.kx.a ? a.kx.a : a.nxh, end = a.kx.a ? lim + 32 : lim;
+  const int nql = a.kx.a ? (a.nx >> 1) & 31 : -1;
+  auto column = [&](int s, bool &ok) {   // s = lane + 32 j
+    ok = s < lim;
+    if (s >= lim && s < lim + 32 && lane == nql) {
+      ok = true;
+      return a.nx >> 1;
+    }
+    return s;
+  };
   const StepState *st = a.st + box;
+  pdl_wait();
   const double nu = a.nu_box ? a.nu_box[box] : a.nu;
   const double dt = st->dt;
   const double fc = a.bandlim ? a.Pin / (2.0 * st->eband) : 0.0;
@@ -1226,21 +1372,18 @@ __global__ void __launch_bounds__(256, FinishMinB<T, MODE>::v)
     }
     tau2 = dt + tn - tm;
   }
-  const double kyr = k_full(a.ky0 + ky, a.ny_k ? a.ny_k : a.ny, a.ay);
-  const double kzr = k_full(kz, a.nz, a.az);
-  const bool need_u = a.bandlim || MODE != FIN_RHS;
   double esum = 0.0, dsum = 0.0;
-  for (int kx0 = lane; kx0 < a.nxh; kx0 += 32 * CH) {
+  for (int s0 = lane; s0 - lane < end; s0 += 32 * CH) {
     C nn[CH][3], uu[CH][3], ss[CH][3], no[CH][3];
     bool ok[CH];
 #pragma unroll
     for (int h = 0; h < CH; ++h) {
-      const int kx = kx0 + 32 * h;
-      ok[h] = kx < a.nxh && a.kx.keep(kx);
+      const int kx = column(s0 + 32 * h, ok[h]);
+      const C *n3 = a.n3 + n3row + xslot(a.n3_nyq, kx, a.nx);
       const long long idx = rowbase + kx;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        nn[h][c] = ok[h] ? a.n3[c * n3nh + n3row + xslot(a.n3_nyq, kx, a.nx)] : mkc<C>(0, 0);
+        nn[h][c] = ok[h] ? n3[c * n3nh] : mkc<C>(0, 0);
         uu[h][c] = ok[h] && need_u ? a.uin[c * a.nh + idx] : mkc<C>(0, 0);
         ss[h][c] = ok[h] && MODE == FIN_CORR ? a.state[c * a.nh + idx] : mkc<C>(0, 0);
         no[h][c] = ok[h] && MODE == FIN_AB2 ? a.nold[c * a.nh + idx] : mkc<C>(0, 0);
@@ -1249,14 +1392,14 @@ __global__ void __launch_bounds__(256, FinishMinB<T, MODE>::v)
 #pragma unroll
     for (int h = 0; h < CH; ++h) {
       if (!ok[h]) continue;
-      const int kx = kx0 + 32 * h;
+      bool unused;
+      const int kx = column(s0 + 32 * h, unused);
       const long long idx = rowbase + kx;
       const double kxr = k_half(kx, a.nx, a.ax);
-      const double wk = (kxr == 0.0) ? 0.5 : 1.0;   // state.f90:436-440
+    const double wk = (kxr == 0.0) ? 0.5 : 1.0;   // state.f90:436-440
       const double k2 = kxr * kxr + kyr * kyr + kzr * kzr;
       const bool zero = (kxr == 0.0) && (kyr == 0.0) && (kzr == 0.0);
-      const bool cut = (a.spherical && k2 >= a.sph2) || fabs(kxr) >= a.cutx || fabs(kyr) >= a.cuty ||
-                       fabs(kzr) >= a.cutz || zero;
+      const bool cut = (a.spherical && k2 >= a.sph2) || fabs(kxr) >= a.cutx || rowcut || zero;
       C Nc[3];
       if (cut) {
         Nc[0] = Nc[1] = Nc[2] = mkc<C>(0, 0);
@@ -1268,7 +1411,7 @@ __global__ void __launch_bounds__(256, FinishMinB<T, MODE>::v)
         const T knre = kr[0] * nn[h][0].x + kr[1] * nn[h][1].x + kr[2] * nn[h][2].x;
         const T knim = kr[0] * nn[h][0].y + kr[1] * nn[h][1].y + kr[2] * nn[h][2].y;
         const T pre = -knim / k2t, pim = knre / k2t;
-        const bool forced = a.bandlim && sqrt(k2) <= a.kcut;
+        const bool forced = a.bandlim && k2 <= a.kcut2;
         const T fct = T(fc);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {

@@ -11,6 +11,23 @@
 
 namespace dnsbox {
 
+// Launches a kernel that begins with pdl_launch / pdl_wait so that it may start
+// while its predecessor in the stream ends.
+template <typename... KA, typename... A>
+static inline cudaError_t launch_pdl(void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, KA(args)...);
+}
+
 template <typename T, int N> struct Launcher {
   static cudaError_t strided(const StridedArgs<T> &a, bool inv, int ntiles, cudaStream_t st);
   // tensor-core split-precision form of `strided` (FP32, N = 128 .. 1024);
@@ -48,17 +65,18 @@ static cudaError_t strided_launch(const StridedArgs<T> &a, dim3 nb, cudaStream_t
   using SH = StridedShape<T, N>;
   const cudaError_t e = set_smem(k_strided<T, N, INV, MODE>, SH::smem(INV));
   if (e != cudaSuccess) return e;
-  k_strided<T, N, INV, MODE><<<nb, SH::NT, SH::smem(INV), st>>>(a);
-  return cudaGetLastError();
+  return launch_pdl(k_strided<T, N, INV, MODE>, nb, SH::NT, SH::smem(INV), st, a);
 }
 
 template <typename T, int N>
 cudaError_t Launcher<T, N>::strided(const StridedArgs<T> &a, bool inv, int ntiles, cudaStream_t st) {
-  const dim3 nb((unsigned)ntiles * a.njobs, (unsigned)(a.nbatch > 0 ? a.nbatch : 1));
+  const bool tail = a.band.n || a.cfl.on;   // one more block per box
+  const dim3 nb((unsigned)ntiles * a.njobs + (tail ? 1 : 0), (unsigned)(a.nbatch > 0 ? a.nbatch : 1));
   // the workspace modes of the passes that use them (inverse: state or
   // workspace to workspace, forward: workspace to either); pruned columns need
   // the compact workspace
   const int ws = a.kcol.a && !a.compact ? 0 : a.ws;
+  if ((a.band.n && !(inv && ws == 2)) || (a.cfl.on && (inv || ws != 3))) return cudaErrorInvalidValue;
   if (inv) {
     if (ws == 3) return strided_launch<T, N, true, ST_WS>(a, nb, st);
     if (ws == 2) return strided_launch<T, N, true, ST_TO_WS>(a, nb, st);
@@ -155,7 +173,7 @@ cudaError_t Launcher<T, N>::xline_nl(const XlineNLArgs<T> &a, int variant, cudaS
     while (nt > 32 && (long long)a.nlines * SH::PL::P < 148LL * 4 * nt) nt >>= 1;
     const int lpb = nt / SH::PL::P;
     if ((e = set_smem(k_xline_nl_g<T, N>, SH::smem(nt))) != cudaSuccess) return e;
-    k_xline_nl_g<T, N><<<(unsigned)((a.nlines + lpb - 1) / lpb), nt, SH::smem(nt), st>>>(a);
+    return launch_pdl(k_xline_nl_g<T, N>, (unsigned)((a.nlines + lpb - 1) / lpb), nt, SH::smem(nt), st, a);
   } else {
     if constexpr (XlineWarp<T, N>::on) {
       if (variant != 1) {   // one warp per line pair

@@ -336,8 +336,7 @@ int rhs_begin(dnsbox_slab *s, const void *uh, double *eband, void *send5, cudaSt
   using C = typename CT<T>::type;
   const double sc = 1.0 / ((double)s->nx * s->ny * s->nz);
   const size_t F = slab_field(s);   // = nz * nyl * nxh, the ky-slab's field
-  k_eband<C><<<1, 256, 0, st>>>(reinterpret_cast<const C *>(uh), (long long)F, s->band, s->nband, s->nx, s->st,
-                                sc * sc, 1, 0);
+  k_eband<C><<<1, 256, 0, st>>>(BandArgs{s->band, s->nband, sc * sc, s->st, uh, (long long)F, 0}, s->nx, 1);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(eband, &s->st->eband, sizeof(double), cudaMemcpyDeviceToDevice, st));
   // pass A: state -> send buffers (rhs.f90:39-65: the spectral curl as multipliers)
@@ -441,7 +440,7 @@ int rhs_finish(dnsbox_slab *s, const void *recv3, const void *uh, const double *
   f.nu = p.nu;
   f.Q = p.Q;
   f.Pin = p.Pin;
-  f.kcut = p.kCutOff;
+  f.kcut2 = kcut2_of(p.kCutOff);
   f.cutx = (s->nx / 2.0) * (2.0 * p.alpha_x / 3.0);   // rhs.f90:74-88
   f.cuty = (s->ny / 2.0) * (2.0 * p.alpha_y / 3.0);
   f.cutz = (s->nz / 2.0) * (2.0 * p.alpha_z / 3.0);
