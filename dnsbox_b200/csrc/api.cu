@@ -148,97 +148,98 @@ __global__ void k_set_state(StepState *st, int nbatch, int off, double v) {
 // Spectral diagnostics over the half spectrum: shell spectrum (state.f90:350-411
 // or single/state.f90:191-230), EZero/EOne/Esqrt2, kinetic energy
 // (state.f90:429-454) and the Parseval dissipation sum.  Per-block partials
-// [gridDim][NV], NV = nspec + 5.
-template <typename C>
-__global__ void k_specdiag(const C *u, long long nh, int nx, int ny, int nz, double ax, double ay,
-                           double az, int nspec, double deltak, int single, double s2,
-                           double *partials) {
+// [gridDim][NV], NV = nspec + 5 (HIST) or 5.  One warp per (kz, ky) row: the
+// row's wavenumbers are formed once and its shells do not decrease with kx, so
+// the lanes of one shell are neighbours and are summed by shuffles before one
+// of them adds to the warp's copy of the histogram (`copies` of them fit).
+template <typename C, bool HIST>
+__global__ void __launch_bounds__(256)
+    k_specdiag(const C *u, long long nh, int nx, int ny, int nz, double ax, double ay, double az, int nspec,
+               double deltak, int single, double s2, int copies, double *partials) {
   extern __shared__ double hist[];
-  const int NV = nspec + 5;
-  for (int i = threadIdx.x; i < NV; i += blockDim.x) hist[i] = 0.0;
-  __syncthreads();
+  pdl_launch();
+  const int NV = (HIST ? nspec : 0) + 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if (HIST) {
+    for (int i = threadIdx.x; i < nspec * copies; i += blockDim.x) hist[i] = 0.0;
+    __syncthreads();
+  }
+  double *h = hist + (size_t)(warp % copies) * nspec;
+  pdl_wait();
   const int nxh = nx / 2 + 1;
   const double sq2 = sqrt(2.0);
   double ez = 0, e1 = 0, es = 0, ek = 0, dk = 0;
-  for (long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x; m < nh;
-       m += (long long)gridDim.x * blockDim.x) {
-    const int kx = (int)(m % nxh);
-    const int ky = (int)((m / nxh) % ny);
-    const int kz = (int)(m / ((long long)nxh * ny));
-    const double kxr = k_half(kx, nx, ax), kyr = k_full(ky, ny, ay), kzr = k_full(kz, nz, az);
-    const double k2 = kxr * kxr + kyr * kyr + kzr * kzr;
-    const double absk = sqrt(k2);
-    double e2 = 0.0;
-    for (int c = 0; c < 3; ++c) {
-      const C v = u[c * nh + m];
-      e2 += (double)v.x * v.x + (double)v.y * v.y;
-    }
-    const double w = (kxr == 0.0) ? 0.5 : 1.0;
-    ek += w * e2;
-    dk += 2.0 * w * k2 * e2;
-    const double base = floor(absk / deltak);
-    const int nk = (absk < base + 0.5 * deltak) ? (int)base : (int)base + 1;
-    if (!single) {
-      if (absk == 0.0) ez += e2;
-      if (absk == 1.0) e1 += e2;
-      if (absk - sq2 < 1.0e-9) es += e2;
-      if (nk < nspec && nk != 0) atomicAdd(&hist[nk - 1], e2 * s2 / deltak);
-    } else {
-      if (absk == 0.0) ez += w * e2;
-      if (nk <= nspec && nk != 0) atomicAdd(&hist[nk - 1], w * e2 * s2 / deltak);
+  for (int row = blockIdx.x * nw + warp; row < ny * nz; row += gridDim.x * nw) {
+    const int kz = row / ny, ky = row - kz * ny;
+    const double kyr = k_full(ky, ny, ay), kzr = k_full(kz, nz, az);
+    const C *r = u + (long long)row * nxh;
+    for (int k0 = 0; k0 < nxh; k0 += 32) {
+      const int kx = k0 + lane;
+      const bool in = kx < nxh;
+      const double kxr = k_half(kx, nx, ax);
+      const double k2 = kxr * kxr + kyr * kyr + kzr * kzr;
+      double e2 = 0.0;
+      if (in)
+        for (int c = 0; c < 3; ++c) {
+          const C v = r[c * nh + kx];
+          e2 += (double)v.x * v.x + (double)v.y * v.y;
+        }
+      const double w = (kxr == 0.0) ? 0.5 : 1.0;
+      ek += w * e2;
+      dk += 2.0 * w * k2 * e2;
+      if (HIST) {
+        const double absk = sqrt(k2), q = deltak == 1.0 ? absk : absk / deltak;
+        const double base = floor(q);
+        int nk = (absk < base + 0.5 * deltak) ? (int)base : (int)base + 1;
+        if (!single) {
+          if (absk == 0.0) ez += e2;
+          if (absk == 1.0) e1 += e2;
+          if (absk - sq2 < 1.0e-9) es += e2;
+          if (nk >= nspec) nk = 0;
+        } else {
+          if (absk == 0.0) ez += w * e2;
+          if (nk > nspec) nk = 0;
+        }
+        if (!in) nk = 0;
+        double v = single ? w * e2 : e2;
+        // sums over runs of equal neighbours (from lane `start` on), whole at a run's last lane
+        const int prev = __shfl_up_sync(0xffffffffu, nk, 1);
+        const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || prev != nk);
+        const int start = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const double y = __shfl_up_sync(0xffffffffu, v, o);
+          if (lane - o >= start) v += y;
+        }
+        const int nxt = __shfl_down_sync(0xffffffffu, nk, 1);
+        if (nk && (lane == 31 || nxt != nk)) atomicAdd(h + nk - 1, v);
+      }
     }
   }
   __shared__ double red[5 * 32];
   double v[5] = {ez, e1, es, ek, dk};
-  block_sum<5>(v, red);
+  block_sum<5>(v, red);   // (its barriers also close the histograms)
+  double *out = partials + (long long)blockIdx.x * NV;
   if (threadIdx.x == 0)
-    for (int i = 0; i < 5; ++i) hist[nspec + i] = v[i];
-  __syncthreads();
-  for (int i = threadIdx.x; i < NV; i += blockDim.x) partials[(long long)blockIdx.x * NV + i] = hist[i];
+    for (int i = 0; i < 5; ++i) out[NV - 5 + i] = v[i];
+  if (HIST)
+    for (int i = threadIdx.x; i < nspec; i += blockDim.x) {
+      double t = 0.0;
+      for (int c = 0; c < copies; ++c) t += hist[(size_t)c * nspec + i];
+      out[i] = t * s2 / deltak;
+    }
 }
 
+// One warp per value: the blocks' partials in a fixed order.
 __global__ void k_sum_partials(const double *partials, int nblk, int nv, double *out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int b = 0; b < nblk; ++b) s += partials[(long long)b * nv + i];
-    out[i] = s;
-  }
-}
-
-// max (signed or |.|) of a real array: per-block partials
-template <typename T>
-__global__ void k_max(const T *f, long long n, int absval, double *partials) {
-  __shared__ double red[32];
-  double m = -INFINITY;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    double x = (double)f[i];
-    m = fmax(m, absval ? fabs(x) : x);
-  }
-  m = warp_max(m);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) red[wid] = m;
-  __syncthreads();
-  if (wid == 0) {
-    double x = lane < (int)(blockDim.x >> 5) ? red[lane] : -INFINITY;
-    x = warp_max(x);
-    if (lane == 0) partials[blockIdx.x] = x;
-  }
-}
-
-__global__ void k_max_partials(const double *partials, int nblk, double *out) {
-  __shared__ double red[32];
-  double m = -INFINITY;
-  for (int i = threadIdx.x; i < nblk; i += blockDim.x) m = fmax(m, partials[i]);
-  m = warp_max(m);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) red[wid] = m;
-  __syncthreads();
-  if (wid == 0) {
-    double x = lane < (int)(blockDim.x >> 5) ? red[lane] : -INFINITY;
-    x = warp_max(x);
-    if (lane == 0) *out = x;
-  }
+  pdl_launch();
+  pdl_wait();
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (i >= nv) return;
+  double s = 0.0;
+  for (int b = lane; b < nblk; b += 32) s += partials[(long long)b * nv + i];
+  s = warp_sum(s);
+  if (lane == 0) out[i] = s;
 }
 
 // state_project (state.f90:120-179), in place
@@ -463,16 +464,21 @@ __global__ void k_dealias(C *u, long long nh, int nx, int ny, int nz, double ax,
   }
 }
 
-// (i k . u) * s for one field (divergence)
+// (i k . u) * s for one field (divergence), one warp per (kz, ky) row
 template <typename C>
 __global__ void k_divhat(const C *u, C *out, long long nh, int nx, int ny, int nz, double ax, double ay,
                          double az, double s) {
   using T = decltype(C{}.x);
+  pdl_launch();
   const int nxh = nx / 2 + 1;
-  for (long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x; m < nh;
-       m += (long long)gridDim.x * blockDim.x) {
-    const int kx = (int)(m % nxh), ky = (int)((m / nxh) % ny), kz = (int)(m / ((long long)nxh * ny));
-    const double kr[3] = {k_half(kx, nx, ax), k_full(ky, ny, ay), k_full(kz, nz, az)};
+  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= ny * nz) return;
+  const int kz = row / ny, ky = row - kz * ny;
+  const double kyr = k_full(ky, ny, ay), kzr = k_full(kz, nz, az);
+  pdl_wait();
+  for (int kx = threadIdx.x & 31; kx < nxh; kx += 32) {
+    const long long m = (long long)row * nxh + kx;
+    const double kr[3] = {k_half(kx, nx, ax), kyr, kzr};
     double re = 0, im = 0;
     for (int c = 0; c < 3; ++c) {
       const C v = u[c * nh + m];
@@ -889,6 +895,10 @@ int run_strided_tma(dnsbox_ctx *c, int axis, bool inv, const StridedArgs<float> 
 // synchronises before returning ends with it; asynchronous entries leave the
 // flag to the next such call or to dnsbox_sync.
 int tc_check(dnsbox_ctx *c) {
+  if (!c->tc) {   // no kernel with a bounded wait
+    CK(cudaStreamSynchronize(c->stream));
+    return DNSBOX_OK;
+  }
   int *flag = reinterpret_cast<int *>(c->hstage + 63);
   *flag = 0;
   if (c->tc_status) CK(cudaMemcpyAsync(flag, c->tc_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
@@ -1468,29 +1478,39 @@ extern "C" int dnsbox_dealias(dnsbox_ctx *ctx, void *uh) {
   return DNSBOX_OK;
 }
 
-// shared spectral diagnostics: out[0..nspec) spectrum, then ezero, eone, esqrt2, E-sum, D-sum
-static int specdiag(dnsbox_ctx *ctx, const void *uh, int single, std::vector<double> &out) {
+// shared spectral diagnostics: (hist) out[0..nspec) spectrum, then ezero, eone, esqrt2, E-sum, D-sum
+template <typename C, bool HIST>
+static int specdiag_t(dnsbox_ctx *ctx, const void *uh, int single, std::vector<double> &out) {
   const dnsbox_params &p = ctx->p;
-  const int nv = ctx->nspec + 5;
-  const int nblk = 148 * 2;
+  const int nv = (HIST ? ctx->nspec : 0) + 5;
+  int nblk = (p.ny * p.nz + 7) / 8;
+  if (nblk > 148 * 4) nblk = 148 * 4;
   RET(ensure_red(ctx, (size_t)nblk * nv + nv));
   const double s = 1.0 / ((double)p.nx * p.ny * p.nz);
-  const size_t smem = (size_t)nv * sizeof(double);
-  if (ctx->fp64)
-    k_specdiag<double2><<<nblk, 256, smem, ctx->stream>>>((const double2 *)uh, (long long)ctx->nh, p.nx, p.ny,
-                                                          p.nz, p.alpha_x, p.alpha_y, p.alpha_z, ctx->nspec,
-                                                          p.Deltak, single, s * s, ctx->red);
-  else
-    k_specdiag<float2><<<nblk, 256, smem, ctx->stream>>>((const float2 *)uh, (long long)ctx->nh, p.nx, p.ny,
-                                                         p.nz, p.alpha_x, p.alpha_y, p.alpha_z, ctx->nspec,
-                                                         p.Deltak, single, s * s, ctx->red);
-  CK(cudaGetLastError());
-  k_sum_partials<<<(nv + 255) / 256, 256, 0, ctx->stream>>>(ctx->red, nblk, nv, ctx->red + (size_t)nblk * nv);
-  CK(cudaGetLastError());
+  int copies = 8;   // one histogram per warp where they fit
+  while (copies > 1 && (size_t)copies * ctx->nspec * sizeof(double) > 40 * 1024) copies >>= 1;
+  const size_t smem = HIST ? (size_t)copies * ctx->nspec * sizeof(double) : 0;
+  CK(launch_pdl(k_specdiag<C, HIST>, nblk, 256, smem, ctx->stream, (const C *)uh, (long long)ctx->nh, p.nx, p.ny, p.nz,
+                p.alpha_x, p.alpha_y, p.alpha_z, ctx->nspec, p.Deltak, single, s * s, copies, ctx->red));
+  double *sums = ctx->red + (size_t)nblk * nv;
+  CK(launch_pdl(k_sum_partials, (nv + 7) / 8, 256, 0, ctx->stream, ctx->red, nblk, nv, sums));
   out.resize(nv);
-  CK(cudaMemcpyAsync(out.data(), ctx->red + (size_t)nblk * nv, nv * sizeof(double), cudaMemcpyDeviceToHost,
-                     ctx->stream));
+  // small results by the pinned staging buffer, so that the copy is asynchronous
+  double *dst = nv <= 32 ? ctx->hstage : out.data();
+  CK(cudaMemcpyAsync(dst, sums, nv * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   RET(tc_check(ctx));
+  if (dst != out.data()) memcpy(out.data(), dst, nv * sizeof(double));
+  return DNSBOX_OK;
+}
+static int specdiag(dnsbox_ctx *ctx, const void *uh, int single, std::vector<double> &out) {
+  return ctx->fp64 ? specdiag_t<double2, true>(ctx, uh, single, out) : specdiag_t<float2, true>(ctx, uh, single, out);
+}
+// the energy and dissipation sums alone
+static int energy_sums(dnsbox_ctx *ctx, const void *uh, double *e, double *d) {
+  std::vector<double> v;
+  RET(ctx->fp64 ? (specdiag_t<double2, false>(ctx, uh, 0, v)) : (specdiag_t<float2, false>(ctx, uh, 0, v)));
+  *e = v[3];
+  *d = v[4];
   return DNSBOX_OK;
 }
 
@@ -1513,11 +1533,11 @@ extern "C" int dnsbox_kinetic(dnsbox_ctx *ctx, const void *uh, double *ekin) {
   BEGIN(ctx);
   SINGLE(ctx);
   if (!uh || !ekin) return set_err(DNSBOX_ERR_ARG, "null pointer");
-  std::vector<double> v;
-  RET(specdiag(ctx, uh, 0, v));
+  double e, d;
+  RET(energy_sums(ctx, uh, &e, &d));
   const dnsbox_params &p = ctx->p;
   const double s = 1.0 / ((double)p.nx * p.ny * p.nz);
-  *ekin = v[ctx->nspec + 3] * s * s;
+  *ekin = e * s * s;
   return DNSBOX_OK;
 }
 
@@ -1525,11 +1545,11 @@ extern "C" int dnsbox_dissipation(dnsbox_ctx *ctx, const void *uh, double *disp)
   BEGIN(ctx);
   SINGLE(ctx);
   if (!uh || !disp) return set_err(DNSBOX_ERR_ARG, "null pointer");
-  std::vector<double> v;
-  RET(specdiag(ctx, uh, 0, v));
+  double e, d;
+  RET(energy_sums(ctx, uh, &e, &d));
   const dnsbox_params &p = ctx->p;
   const double s = 1.0 / ((double)p.nx * p.ny * p.nz);
-  *disp = p.nu * v[ctx->nspec + 4] * s * s;
+  *disp = p.nu * d * s * s;
   return DNSBOX_OK;
 }
 
@@ -1567,19 +1587,24 @@ template <typename T> static int state_to_phys(dnsbox_ctx *ctx, const void *uh, 
   return c2r_fields<T>(ctx, 3, in, out, scale);
 }
 
-static int reduce_max(dnsbox_ctx *ctx, const void *f, bool fp64, long long n, int absval, double *host) {
-  const int nblk = 148 * 4;
-  RET(ensure_red(ctx, nblk + 1));
-  if (fp64)
-    k_max<double><<<nblk, 256, 0, ctx->stream>>>((const double *)f, n, absval, ctx->red);
-  else
-    k_max<float><<<nblk, 256, 0, ctx->stream>>>((const float *)f, n, absval, ctx->red);
-  CK(cudaGetLastError());
-  k_max_partials<<<1, 1024, 0, ctx->stream>>>(ctx->red, nblk, ctx->red + nblk);
-  CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(ctx->hstage, ctx->red + nblk, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+// Maxima (signed, or of |.|) over the grid of the C2R of nf spectral fields,
+// taken as the x pass forms the lines: nothing is stored.
+template <typename T>
+static int c2r_maxima(dnsbox_ctx *ctx, int nf, const void *const *in, double scale, int absval, double *host) {
+  RET(ensure_red(ctx, 8));
+  unsigned long long *keys = reinterpret_cast<unsigned long long *>(ctx->red);
+  CK(cudaMemsetAsync(keys, 0, nf * sizeof(*keys), ctx->stream));
+  SpecJob jobs[6];
+  for (int f = 0; f < nf; ++f) jobs[f] = SpecJob{{{in[f], 1.0, 0.0, 0}, {nullptr, 0, 0, 0}}, 1};
+  RET(c2r_jobs<T>(ctx, nf, jobs, nullptr, scale, keys, absval));
+  CK(cudaMemcpyAsync(ctx->hstage, keys, nf * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   RET(tc_check(ctx));
-  *host = ctx->hstage[0];
+  for (int f = 0; f < nf; ++f) {
+    unsigned long long k;
+    memcpy(&k, ctx->hstage + f, sizeof(k));
+    k = k >> 63 ? k & 0x7fffffffffffffffull : ~k;
+    memcpy(host + f, &k, sizeof(k));
+  }
   return DNSBOX_OK;
 }
 
@@ -1589,10 +1614,10 @@ extern "C" int dnsbox_courant(dnsbox_ctx *ctx, const void *uh, double dt, double
   if (!uh || !courant) return set_err(DNSBOX_ERR_ARG, "null pointer");
   const dnsbox_params &p = ctx->p;
   const double s = 1.0 / ((double)p.nx * p.ny * p.nz);
-  void *phys[3];
-  RET(ctx->fp64 ? state_to_phys<double>(ctx, uh, s, phys) : state_to_phys<float>(ctx, uh, s, phys));
+  const void *in[3];
+  for (int f = 0; f < 3; ++f) in[f] = cfield(reinterpret_cast<const char *>(uh), ctx, f);
   double m[3];
-  for (int c = 0; c < 3; ++c) RET(reduce_max(ctx, phys[c], ctx->fp64, (long long)ctx->np, 1, &m[c]));
+  RET(ctx->fp64 ? c2r_maxima<double>(ctx, 3, in, s, 1, m) : c2r_maxima<float>(ctx, 3, in, s, 1, m));
   // io.f90:669-671
   *courant = m[0] * dt / ((2 * M_PI / p.alpha_x) / p.nx) + m[1] * dt / ((2 * M_PI / p.alpha_y) / p.ny) +
              m[2] * dt / ((2 * M_PI / p.alpha_z) / p.nz);
@@ -1607,20 +1632,17 @@ extern "C" int dnsbox_divergence(dnsbox_ctx *ctx, const void *uh, double *divmax
   if (!uh || !divmax) return set_err(DNSBOX_ERR_ARG, "null pointer");
   const dnsbox_params &p = ctx->p;
   const double s = 1.0 / ((double)p.nx * p.ny * p.nz);
-  // (i k . u) s into W2 slot 5, C2R into W1 slot 4
-  void *dh = field(ctx->W2, ctx, 5);
-  const int g = grid_for((long long)ctx->nh);
+  // (i k . u) s into W2 slot 5
+  void *dh = wfield(ctx->W2, ctx, 5);
+  const int g = (p.ny * p.nz + 7) / 8;
   if (ctx->fp64)
-    k_divhat<double2><<<g, 256, 0, ctx->stream>>>((const double2 *)uh, (double2 *)dh, (long long)ctx->nh, p.nx,
-                                                  p.ny, p.nz, p.alpha_x, p.alpha_y, p.alpha_z, s);
+    CK(launch_pdl(k_divhat<double2>, g, 256, 0, ctx->stream, (const double2 *)uh, (double2 *)dh, (long long)ctx->nh, p.nx,
+                  p.ny, p.nz, p.alpha_x, p.alpha_y, p.alpha_z, s));
   else
-    k_divhat<float2><<<g, 256, 0, ctx->stream>>>((const float2 *)uh, (float2 *)dh, (long long)ctx->nh, p.nx,
-                                                 p.ny, p.nz, p.alpha_x, p.alpha_y, p.alpha_z, s);
-  CK(cudaGetLastError());
+    CK(launch_pdl(k_divhat<float2>, g, 256, 0, ctx->stream, (const float2 *)uh, (float2 *)dh, (long long)ctx->nh, p.nx,
+                  p.ny, p.nz, p.alpha_x, p.alpha_y, p.alpha_z, s));
   const void *in[1] = {dh};
-  void *out[1] = {field(ctx->W1, ctx, 4)};
-  RET(ctx->fp64 ? c2r_fields<double>(ctx, 1, in, out, 1.0) : c2r_fields<float>(ctx, 1, in, out, 1.0));
-  return reduce_max(ctx, out[0], ctx->fp64, (long long)ctx->np, 0, divmax);
+  return ctx->fp64 ? c2r_maxima<double>(ctx, 1, in, 1.0, 0, divmax) : c2r_maxima<float>(ctx, 1, in, 1.0, 0, divmax);
 }
 
 extern "C" int dnsbox_c2r(dnsbox_ctx *ctx, const void *spec, void *phys) {

@@ -420,10 +420,12 @@ struct SpecJob {
   int nt;
 };
 
-// 3D C2R of nf outputs described by jobs, through W1/W2 in chunks of 6.
+// 3D C2R of nf outputs described by jobs, through W1/W2 in chunks of 6; with
+// vmax, the outputs' maxima as keys (zeroed by the caller) and no outputs.
 // Inputs must not live in W1 or W2 slots [0, 6).
 template <typename T>
-static int c2r_jobs(dnsbox_ctx *c, int nf, const SpecJob *jobs, void *const *out, double scale) {
+static int c2r_jobs(dnsbox_ctx *c, int nf, const SpecJob *jobs, void *const *out, double scale,
+                    unsigned long long *vmax = nullptr, int absval = 0) {
   for (int f0 = 0; f0 < nf; f0 += 6) {
     const int m = nf - f0 < 6 ? nf - f0 : 6;
     StridedArgs<T> a = strided_base<T>(c, 2);
@@ -445,8 +447,10 @@ static int c2r_jobs(dnsbox_ctx *c, int nf, const SpecJob *jobs, void *const *out
     memset(&x, 0, sizeof(x));
     for (int j = 0; j < m; ++j) {
       x.in[j] = wfield(c->W2, c, j);
-      x.out[j] = out[f0 + j];
+      x.out[j] = vmax ? nullptr : out[f0 + j];
     }
+    x.vmax = vmax ? vmax + f0 : nullptr;
+    x.absval = absval;
     x.pitch = c->wp;
     x.tw = reinterpret_cast<const typename CT<T>::type *>(c->tw[0]);
     x.nlines = c->p.ny * c->p.nz;

@@ -884,6 +884,28 @@ __device__ __forceinline__ double2 ld_on(const double2 *p, bool on) {
                : "l"(p), "r"((unsigned)on));
   return x;
 }
+// The Hermitian sequence of two real lines: put(q, re, im) with the value of
+// row p + P q of X1 + i X2, q < E, from the own rows n = p + P i <= N/2 (i <=
+// E/2; i = E/2 is lane 0's Nyquist row) of the half lines x1, x2, whose
+// imaginary parts at rows 0 and N/2 are zero.  Lane p forms its rows' values
+// and their mirrors', which belong to lane P - p.
+template <int E, typename C, typename PUT> __device__ __forceinline__ void pack_lines(const C *x1, const C *x2, int p,
+                                                                                      int mirror, PUT put) {
+  using T = decltype(C{}.x);
+#pragma unroll
+  for (int i = 0; i < E / 2; ++i) put(i, x1[i].x - x2[i].y, x1[i].y + x2[i].x);
+#pragma unroll
+  for (int i = 0; i < E / 2; ++i) {
+    // lane p sends the mirror of its row i, lane 0 (its own partner) that of row i + 1
+    const int j = i + 1;
+    T re = x1[i].x + x2[i].y, im = x2[i].x - x1[i].y;
+    const T re0 = x1[j].x + x2[j].y, im0 = x2[j].x - x1[j].y;
+    re = p == 0 ? re0 : re;
+    im = p == 0 ? im0 : im;
+    put(E - 1 - i, __shfl_sync(0xffffffffu, re, mirror), __shfl_sync(0xffffffffu, im, mirror));
+  }
+}
+
 // Exchange tile of one line: rows skewed by row / R0, or for the 4 x 4 x ..
 // plans of 96 and 192 exchanged by an exclusive or within 16, so that the
 // strided writes of a stage and the consecutive reads of the next fall in
@@ -968,22 +990,7 @@ __global__ void __launch_bounds__(XReg<T, N>::NT, XReg<T, N>::minb)
     if (p == 0) x[0].y = x[H].y = 0;   // a C2R drops these imaginary parts
   };
   auto shfl = [&](T v) { return __shfl_sync(0xffffffffu, v, mirror); };
-  // X1 + i X2 at the own rows and the mirror rows from the half lines x1, x2:
-  // put(q, re, im) with the value of row p + P q
-  auto pack = [&](const C *x1, const C *x2, auto put) {
-#pragma unroll
-    for (int i = 0; i < H; ++i) put(i, x1[i].x - x2[i].y, x1[i].y + x2[i].x);
-#pragma unroll
-    for (int i = 0; i < H; ++i) {
-      // lane p sends the mirror of its row i, lane 0 (its own partner) that of row i + 1
-      const int j = i + 1;
-      T re = x1[i].x + x2[i].y, im = x2[i].x - x1[i].y;
-      const T re0 = x1[j].x + x2[j].y, im0 = x2[j].x - x1[j].y;   // row N/2: imaginary parts are 0
-      re = p == 0 ? re0 : re;
-      im = p == 0 ? im0 : im;
-      put(E - 1 - i, shfl(re), shfl(im));
-    }
-  };
+  auto pack = [&](const C *x1, const C *x2, auto put) { pack_lines<E>(x1, x2, p, mirror, put); };
   T up = 1, down = 1;
   V1 w[E];   // (w, 2^e oz) at row p + P q in w[out_i(q)]
   T u_[E], v_[E], ox_[E], oy_[E];
@@ -1148,6 +1155,7 @@ __global__ void __launch_bounds__(XReg<T, N>::NT, XReg<T, N>::minb)
   }
 }
 
+// ------------------------------------------------------- plain x-line transforms
 template <typename T> struct XlineArgs {
   using C = typename CT<T>::type;
   const void *in[6];
@@ -1155,100 +1163,145 @@ template <typename T> struct XlineArgs {
   const C *tw;
   int nlines, nxh;
   int pitch;               // row pitch (complex elements) of the half lines; 0: nxh
+  int absval;              // with vmax: maxima of |x| (1) or of x (0)
   double scale;            // multiplies the output
+  unsigned long long *vmax;   // C2R: take the maximum of each field into vmax[field] (max_key) and store nothing
 };
 
-template <typename T, int N> struct XlinePlainB {
-  static constexpr int v = (sizeof(T) == 8 ? 16 : 32) / ((N >= 512) ? 4 : 1);
+// Doubles in increasing order as unsigned integers, for an atomic maximum
+// (0 is below every value); the host inverts it (max_of_key).
+__host__ __device__ __forceinline__ unsigned long long max_key_bits(unsigned long long b) {
+  return b >> 63 ? ~b : b | 0x8000000000000000ull;
+}
+
+// P lanes own a pair of lines (la, lb) as one complex sequence X1 + i X2, in
+// registers but for the exchanges (the plans and tiles of k_xline_nl_g; 16
+// values a thread in both precisions, 32 at 1024).
+template <int N> struct LPlan : VPlan<N> {};
+#define DNSBOX_LPLAN(NN, EE, ...)                                                                                    \
+  template <> struct LPlan<NN> {                                                                                     \
+    static constexpr int N = NN, E = EE, P = NN / EE;                                                                \
+    static constexpr int R[] = {__VA_ARGS__};                                                                        \
+    static constexpr int NST = sizeof(R) / sizeof(int);                                                              \
+    __host__ __device__ static constexpr int ns(int s) { int q = 1; for (int i = 0; i < s; ++i) q *= R[i]; return q; } \
+  };
+DNSBOX_LPLAN(512, 16, 16, 8, 4)
+DNSBOX_LPLAN(1024, 32, 16, 16, 4)
+#undef DNSBOX_LPLAN
+template <typename T, int N> struct XPlain {
+  using PL = LPlan<N>;
+  static constexpr int NT = 128;
+  static constexpr size_t tw = ((size_t)vtw_size<PL>() * 2 * sizeof(T) + 15) / 16 * 16;
+  static constexpr size_t line = (size_t)XTile<PL>::pitch * 2 * sizeof(T);
+  static constexpr size_t smem(int threads) { return tw + threads / PL::P * line; }
+  static constexpr int minb = sizeof(T) == 8 ? (PL::E > 16 ? 2 : 3) : (PL::E > 16 ? 3 : 5);
 };
 
-// C2R along x: half lines (nxh complex) -> real lines (N), two lines per FFT.
+// C2R along x: half lines (nxh complex) -> real lines (N).  blockIdx.y = field.
+// Against the row-tile kernels before it the 256^3 FP32 pair of transforms goes
+// from 240 to 170 us.
 template <typename T, int N>
-__global__ void __launch_bounds__(round32((XlinePlainB<T, N>::v / 2) * (N / FftPlan<N>::E)))
+__global__ void __launch_bounds__(XPlain<T, N>::NT, XPlain<T, N>::minb)
     k_xline_c2r(const __grid_constant__ XlineArgs<T> a) {
   using C = typename CT<T>::type;
-  using EN = FftEnds<N>;
-  constexpr int B = XlinePlainB<T, N>::v;
-  constexpr int NC = B / 2;
-  constexpr int LD = NC + 1;
-  constexpr int E = EN::E;
-  constexpr int P = N / E;
-  constexpr int NF = NC * P;
+  using SH = XPlain<T, N>;
+  using PL = typename SH::PL;
+  using EN = VEnds<PL>;
+  using V = VC<T>;
+  constexpr int E = PL::E, P = PL::P, H = E / 2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C *s = reinterpret_cast<C *>(smem_raw);
-  const C *in = reinterpret_cast<const C *>(a.in[blockIdx.y]);
-  T *out = reinterpret_cast<T *>(a.out[blockIdx.y]);
-  const int pitch = a.pitch ? a.pitch : a.nxh;
-  const bool act = threadIdx.x < NF;
-  const int p = threadIdx.x % P, j = threadIdx.x / P;
-  const int la = blockIdx.x * B + 2 * j, lb = la + 1;
-  const bool va = act && la < a.nlines, vb = act && lb < a.nlines;
-  C v[E];
+  V *twt = reinterpret_cast<V *>(smem_raw);
+  pdl_launch();
+  vtw_fill<PL, V>(twt, a.tw, threadIdx.x, blockDim.x);
+  __syncthreads();
+  pdl_wait();
+  const int g = threadIdx.x / P, p = threadIdx.x % P, lane = threadIdx.x & 31;
+  V *s = reinterpret_cast<V *>(smem_raw + SH::tw + (size_t)g * SH::line);
+  const long long la = 2 * ((long long)blockIdx.x * (blockDim.x / P) + g);
+  const bool va = la < a.nlines, vb = la + 1 < a.nlines;
+  const long long pitch = a.pitch ? a.pitch : a.nxh;
+  const C *in = reinterpret_cast<const C *>(a.in[blockIdx.y]) + la * pitch;
+  C x1[H + 1], x2[H + 1];
 #pragma unroll
-  for (int i = 0; i < E; ++i) {
-    const int n = EN::in_row(p, i);
-    const int kk = n <= N / 2 ? n : N - n;
-    const C X1 = va ? in[(long long)la * pitch + kk] : mkc<C>(0, 0);
-    const C X2 = vb ? in[(long long)lb * pitch + kk] : mkc<C>(0, 0);
-    v[i] = pack_pair<C, N>(n, X1, X2);
+  for (int i = 0; i <= H; ++i) {
+    x1[i] = ld_on(in + p + P * i, va && (i < H || p == 0));
+    x2[i] = ld_on(in + pitch + p + P * i, vb && (i < H || p == 0));
   }
-  fft_regs<C, N, true>(v, s, LD, j, p, act, a.tw);
+  if (p == 0) x1[0].y = x1[H].y = x2[0].y = x2[H].y = 0;   // a C2R drops these imaginary parts
+  V z[E], x[E];
+  pack_lines<E>(x1, x2, p, (lane & ~(P - 1)) | ((P - p) & (P - 1)), [&](int q, T r, T i) { z[EN::in_i(q)] = V{r, i}; });
+  vfft<PL, true, XTile<PL>>(z, x, s, 0, p, twt, []() { __syncwarp(); });
   const T sc = T(a.scale);
+  if (a.vmax) {
+    T m = -INFINITY;
 #pragma unroll
-  for (int i = 0; i < E; ++i) {
-    const int n = EN::out_row(p, i);
-    if (va) out[(long long)la * N + n] = v[i].x * sc;
-    if (vb) out[(long long)lb * N + n] = v[i].y * sc;
+    for (int i = 0; i < E; ++i) {
+      const T r = x[i].re * sc, q = x[i].im * sc;
+      if (va) m = fmax(m, a.absval ? fabs(r) : r);
+      if (vb) m = fmax(m, a.absval ? fabs(q) : q);
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0) {   // only a larger value needs the atomic
+      const unsigned long long key = max_key_bits((unsigned long long)__double_as_longlong((double)m));
+      if (key > __ldcg(a.vmax + blockIdx.y)) atomicMax(a.vmax + blockIdx.y, key);
+    }
+    return;
+  }
+  T *out = reinterpret_cast<T *>(a.out[blockIdx.y]) + la * N + p;
+#pragma unroll
+  for (int q = 0; q < E; ++q) {
+    const V v = x[EN::out_i(q)];
+    if (va) out[P * q] = v.re * sc;
+    if (vb) out[N + P * q] = v.im * sc;
   }
 }
 
-// R2C along x: real lines -> half lines, two lines per FFT.
+// R2C along x: real lines -> half lines, two lines per transform.
 template <typename T, int N>
-__global__ void __launch_bounds__(round32((XlinePlainB<T, N>::v / 2) * (N / FftPlan<N>::E)))
+__global__ void __launch_bounds__(XPlain<T, N>::NT, XPlain<T, N>::minb)
     k_xline_r2c(const __grid_constant__ XlineArgs<T> a) {
   using C = typename CT<T>::type;
-  using EN = FftEnds<N>;
-  constexpr int B = XlinePlainB<T, N>::v;
-  constexpr int NC = B / 2;
-  constexpr int LD = NC + 1;
-  constexpr int H = N / 2 + 1;
-  constexpr int E = EN::E;
-  constexpr int P = N / E;
-  constexpr int NF = NC * P;
+  using SH = XPlain<T, N>;
+  using PL = typename SH::PL;
+  using EN = VEnds<PL>;
+  using V = VC<T>;
+  constexpr int E = PL::E, P = PL::P, H = E / 2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C *s = reinterpret_cast<C *>(smem_raw);
-  const T *in = reinterpret_cast<const T *>(a.in[blockIdx.y]);
-  C *out = reinterpret_cast<C *>(a.out[blockIdx.y]);
-  const int pitch = a.pitch ? a.pitch : a.nxh;
-  const int NT = blockDim.x;
-  const bool act = threadIdx.x < NF;
-  const int p = threadIdx.x % P, j = threadIdx.x / P;
-  const int line0 = blockIdx.x * B;
-  {
-    const int la = line0 + 2 * j, lb = la + 1;
-    const bool va = act && la < a.nlines, vb = act && lb < a.nlines;
-    C v[E];
-#pragma unroll
-    for (int i = 0; i < E; ++i) {
-      const int n = EN::in_row(p, i);
-      v[i] = mkc<C>(va ? in[(long long)la * N + n] : T(0), vb ? in[(long long)lb * N + n] : T(0));
-    }
-    fft_regs<C, N, false>(v, s, LD, j, p, act, a.tw);
-    if (act) {
-#pragma unroll
-      for (int i = 0; i < E; ++i) s[EN::out_row(p, i) * LD + j] = v[i];
-    }
-  }
+  V *twt = reinterpret_cast<V *>(smem_raw);
+  pdl_launch();
+  vtw_fill<PL, V>(twt, a.tw, threadIdx.x, blockDim.x);
   __syncthreads();
-  const T sc = T(a.scale);
-  for (int it = threadIdx.x; it < NC * H; it += NT) {
-    const int k = it % H, jj = it / H;
-    const int la = line0 + 2 * jj, lb = la + 1;
-    const C zk = s[k * LD + jj], zn = s[((N - k) % N) * LD + jj];
-    const C X1 = mkc<C>(T(0.5) * (zk.x + zn.x) * sc, T(0.5) * (zk.y - zn.y) * sc);
-    const C X2 = mkc<C>(T(0.5) * (zk.y + zn.y) * sc, T(-0.5) * (zk.x - zn.x) * sc);
-    if (la < a.nlines) out[(long long)la * pitch + k] = X1;
-    if (lb < a.nlines) out[(long long)lb * pitch + k] = X2;
+  pdl_wait();
+  const int g = threadIdx.x / P, p = threadIdx.x % P, lane = threadIdx.x & 31;
+  V *s = reinterpret_cast<V *>(smem_raw + SH::tw + (size_t)g * SH::line);
+  const long long la = 2 * ((long long)blockIdx.x * (blockDim.x / P) + g);
+  const bool va = la < a.nlines, vb = la + 1 < a.nlines;
+  const T *in = reinterpret_cast<const T *>(a.in[blockIdx.y]) + la * N + p;
+  V z[E], x[E];
+#pragma unroll
+  for (int q = 0; q < E; ++q) {
+    const T r = va ? in[P * q] : T(0), i = vb ? in[N + P * q] : T(0);
+    z[EN::in_i(q)] = V{r, i};
+  }
+  vfft<PL, false, XTile<PL>>(z, x, s, 0, p, twt, []() { __syncwarp(); });
+  const T sc = T(a.scale), hs = T(0.5);
+  const long long pitch = a.pitch ? a.pitch : a.nxh;
+  C *out = reinterpret_cast<C *>(a.out[blockIdx.y]) + la * pitch;
+  const int mirror = (lane & ~(P - 1)) | ((P - p) & (P - 1));
+#pragma unroll
+  for (int i = 0; i <= H; ++i) {
+    const V zk = x[EN::out_i(i)];
+    T nr = zk.re, ni = zk.im;   // i = H: row N/2, its own mirror
+    if (i < H) {
+      const V b = x[EN::out_i(E - 1 - i)], b0 = x[EN::out_i((E - i) % E)];
+      nr = __shfl_sync(0xffffffffu, p == 0 ? b0.re : b.re, mirror);
+      ni = __shfl_sync(0xffffffffu, p == 0 ? b0.im : b.im, mirror);
+    }
+    if (i < H || p == 0) {
+      if (va) out[p + P * i] = mkc<C>(hs * (zk.re + nr) * sc, hs * (zk.im - ni) * sc);
+      if (vb) out[pitch + p + P * i] = mkc<C>(hs * (zk.im + ni) * sc, hs * (nr - zk.re) * sc);
+    }
   }
 }
 

@@ -195,30 +195,29 @@ cudaError_t Launcher<T, N>::xline_nl(const XlineNLArgs<T> &a, int variant, cudaS
   return cudaGetLastError();
 }
 
+// Threads of a plain x-line block: smaller blocks where the lines are few.
+template <typename T, int N> static int xplain_threads(const XlineArgs<T> &a, int nf) {
+  int nt = XPlain<T, N>::NT;
+  while (nt > 32 && (long long)nf * a.nlines * XPlain<T, N>::PL::P < 2 * 148LL * 4 * nt) nt >>= 1;
+  return nt;
+}
+
 template <typename T, int N>
 cudaError_t Launcher<T, N>::xline_c2r(const XlineArgs<T> &a, int nf, cudaStream_t st) {
-  using C = typename CT<T>::type;
-  constexpr int B = XlinePlainB<T, N>::v;
-  const size_t smem = (size_t)N * (B / 2 + 1) * sizeof(C);
-  const int nt = round32((B / 2) * (N / FftPlan<N>::E));
-  cudaError_t e;
-  if ((e = set_smem(k_xline_c2r<T, N>, smem)) != cudaSuccess) return e;
-  dim3 grid((unsigned)((a.nlines + B - 1) / B), (unsigned)nf);
-  k_xline_c2r<T, N><<<grid, nt, smem, st>>>(a);
-  return cudaGetLastError();
+  using SH = XPlain<T, N>;
+  const int nt = xplain_threads<T, N>(a, nf), lpb = 2 * (nt / SH::PL::P);
+  const cudaError_t e = set_smem(k_xline_c2r<T, N>, SH::smem(nt));
+  if (e != cudaSuccess) return e;
+  return launch_pdl(k_xline_c2r<T, N>, dim3((unsigned)((a.nlines + lpb - 1) / lpb), (unsigned)nf), nt, SH::smem(nt), st, a);
 }
 
 template <typename T, int N>
 cudaError_t Launcher<T, N>::xline_r2c(const XlineArgs<T> &a, int nf, cudaStream_t st) {
-  using C = typename CT<T>::type;
-  constexpr int B = XlinePlainB<T, N>::v;
-  const size_t smem = (size_t)N * (B / 2 + 1) * sizeof(C);
-  const int nt = round32((B / 2) * (N / FftPlan<N>::E));
-  cudaError_t e;
-  if ((e = set_smem(k_xline_r2c<T, N>, smem)) != cudaSuccess) return e;
-  dim3 grid((unsigned)((a.nlines + B - 1) / B), (unsigned)nf);
-  k_xline_r2c<T, N><<<grid, nt, smem, st>>>(a);
-  return cudaGetLastError();
+  using SH = XPlain<T, N>;
+  const int nt = xplain_threads<T, N>(a, nf), lpb = 2 * (nt / SH::PL::P);
+  const cudaError_t e = set_smem(k_xline_r2c<T, N>, SH::smem(nt));
+  if (e != cudaSuccess) return e;
+  return launch_pdl(k_xline_r2c<T, N>, dim3((unsigned)((a.nlines + lpb - 1) / lpb), (unsigned)nf), nt, SH::smem(nt), st, a);
 }
 
 #endif
