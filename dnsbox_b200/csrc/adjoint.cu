@@ -66,25 +66,45 @@ __device__ __forceinline__ bool adj_masked(const Grid3 &g, double kx, double ky,
   for (long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x; m < (n);           \
        m += (long long)gridDim.x * blockDim.x)
 
-// h / W = -P(D g) / W
+// One warp per (kz, ky) row of the half spectrum: kx = lane, lane + 32, ...
+#define ROW_LOOP(gr)                                                                      \
+  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);                    \
+  if (row >= (gr).ny * (gr).nz) return;                                                   \
+  const double kz = k_full(row / (gr).ny, (gr).nz, (gr).az), ky = k_full(row % (gr).ny, (gr).ny, (gr).ay); \
+  pdl_wait();                                                                             \
+  for (int ix = threadIdx.x & 31; ix < (gr).nxh; ix += 32)
+static inline int row_blocks(const Grid3 &g) { return (g.ny * g.nz + 7) / 8; }
+
+// -P(D v) / W of one mode
 template <typename C>
-__global__ void k_vjp_pre(const C *g, C *hw, long long nh, Grid3 gr) {
+__device__ __forceinline__ void vjp_pre_mode(const Grid3 &gr, double kx, double ky, double kz, const double (*v)[2],
+                                             C *hw, long long nh, long long m) {
   using T = decltype(C{}.x);
-  GRID_LOOP(m, nh) {
-    double kx, ky, kz;
-    mode_k(gr, m, kx, ky, kz);
-    if (rhs_masked(gr, kx, ky, kz)) {
-      for (int c = 0; c < 3; ++c) hw[c * nh + m] = mkc<C>(0, 0);
-      continue;
+  if (rhs_masked(gr, kx, ky, kz)) {
+    for (int c = 0; c < 3; ++c) hw[c * nh + m] = mkc<C>(0, 0);
+    return;
+  }
+  const double k2 = kx * kx + ky * ky + kz * kz;
+  const double kr[3] = {kx, ky, kz};
+  const double dre = (kx * v[0][0] + ky * v[1][0] + kz * v[2][0]) / k2;
+  const double dim = (kx * v[0][1] + ky * v[1][1] + kz * v[2][1]) / k2;
+  const double w = (kx == 0.0) ? 1.0 : 0.5;   // 1 / W
+  for (int c = 0; c < 3; ++c)
+    hw[c * nh + m] = mkc<C>(T(-(v[c][0] - kr[c] * dre) * w), T(-(v[c][1] - kr[c] * dim) * w));
+}
+
+// h / W = -P(D scale g) / W
+template <typename C>
+__global__ void k_vjp_pre(const C *g, C *hw, long long nh, Grid3 gr, double scale) {
+  pdl_launch();
+  ROW_LOOP(gr) {
+    const long long m = (long long)row * gr.nxh + ix;
+    double v[3][2];
+    for (int c = 0; c < 3; ++c) {
+      const C q = g[c * nh + m];
+      v[c][0] = scale * q.x, v[c][1] = scale * q.y;
     }
-    const double k2 = kx * kx + ky * ky + kz * kz;
-    const double kr[3] = {kx, ky, kz};
-    const C v[3] = {g[m], g[nh + m], g[2 * nh + m]};
-    const double dre = (kx * v[0].x + ky * v[1].x + kz * v[2].x) / k2;
-    const double dim = (kx * v[0].y + ky * v[1].y + kz * v[2].y) / k2;
-    const double w = (kx == 0.0) ? 1.0 : 0.5;   // 1 / W
-    for (int c = 0; c < 3; ++c)
-      hw[c * nh + m] = mkc<C>(T(-(v[c].x - kr[c] * dre) * w), T(-(v[c].y - kr[c] * dim) * w));
+    vjp_pre_mode<C>(gr, k_half(ix, gr.nx, gr.ax), ky, kz, v, hw, nh, m);
   }
 }
 
@@ -104,23 +124,63 @@ __global__ void k_vjp_cross(T *f, long long np) {
   }
 }
 
-// out = s W (ik x A + B)
-template <typename C>
-__global__ void k_vjp_combine(const C *A, const C *Bv, C *out, long long nh, Grid3 gr, double s) {
+// What is done with the transposed term a = s W (ik x A + B) of a mode.
+enum CombineMode : int {
+  CB_OUT = 0,      // out = a
+  CB_ADD = 1,      // out += a
+  CB_LINEAR = 2,   // out = a + L g  (the residual's gradient)
+  CB_STEP = 3,     // out = IF (g + a) and h / W of IF (dt/2 g + dt a) (the step transpose's first half)
+};
+template <typename C> struct CombineArgs {
+  const C *ws;               // A (3 fields) and B (3), rows of `pitch`, fields wst apart
+  long long wst;
+  int pitch;
+  C *out;
+  const C *g;
+  C *hw;
+  long long nh;
+  Grid3 gr;
+  double s, nu, Q, dt;
+};
+template <typename C, int MODE> __global__ void k_vjp_combine(CombineArgs<C> a) {
   using T = decltype(C{}.x);
-  GRID_LOOP(m, nh) {
-    double kx, ky, kz;
-    mode_k(gr, m, kx, ky, kz);
-    const double sw = s * ((kx == 0.0) ? 1.0 : 2.0);
-    const C a0 = A[m], a1 = A[nh + m], a2 = A[2 * nh + m];
+  pdl_launch();
+  const Grid3 &gr = a.gr;
+  ROW_LOOP(gr) {
+    const double kx = k_half(ix, gr.nx, gr.ax);
+    const double sw = a.s * ((kx == 0.0) ? 1.0 : 2.0);
+    const C *w = a.ws + (long long)row * a.pitch + ix;
+    const long long m = (long long)row * gr.nxh + ix, nh = a.nh;
+    const C a0 = w[0], a1 = w[a.wst], a2 = w[2 * a.wst], b0 = w[3 * a.wst], b1 = w[4 * a.wst], b2 = w[5 * a.wst];
     // i (k x a): component = i (k_j a_k - k_k a_j)
-    const double cx_re = -(ky * a2.y - kz * a1.y), cx_im = ky * a2.x - kz * a1.x;
-    const double cy_re = -(kz * a0.y - kx * a2.y), cy_im = kz * a0.x - kx * a2.x;
-    const double cz_re = -(kx * a1.y - ky * a0.y), cz_im = kx * a1.x - ky * a0.x;
-    const C b0 = Bv[m], b1 = Bv[nh + m], b2 = Bv[2 * nh + m];
-    out[m] = mkc<C>(T(sw * (cx_re + b0.x)), T(sw * (cx_im + b0.y)));
-    out[nh + m] = mkc<C>(T(sw * (cy_re + b1.x)), T(sw * (cy_im + b1.y)));
-    out[2 * nh + m] = mkc<C>(T(sw * (cz_re + b2.x)), T(sw * (cz_im + b2.y)));
+    const double r[3][2] = {{sw * (-(ky * a2.y - kz * a1.y) + b0.x), sw * (ky * a2.x - kz * a1.x + b0.y)},
+                            {sw * (-(kz * a0.y - kx * a2.y) + b1.x), sw * (kz * a0.x - kx * a2.x + b1.y)},
+                            {sw * (-(kx * a1.y - ky * a0.y) + b2.x), sw * (kx * a1.x - ky * a0.x + b2.y)}};
+    const double L = a.Q - a.nu * (kx * kx + ky * ky + kz * kz);
+    if (MODE == CB_STEP) {
+      const double IF = exp(L * a.dt);
+      double arg[3][2];
+      for (int c = 0; c < 3; ++c) {
+        const C g = a.g[c * nh + m];
+        a.out[c * nh + m] = mkc<C>(T(IF * (g.x + r[c][0])), T(IF * (g.y + r[c][1])));
+        arg[c][0] = IF * (0.5 * a.dt * g.x + a.dt * r[c][0]);
+        arg[c][1] = IF * (0.5 * a.dt * g.y + a.dt * r[c][1]);
+      }
+      vjp_pre_mode<C>(gr, kx, ky, kz, arg, a.hw, nh, m);
+    } else {
+      for (int c = 0; c < 3; ++c) {
+        double re = r[c][0], im = r[c][1];
+        if (MODE == CB_ADD) {
+          const C o = a.out[c * nh + m];
+          re += o.x, im += o.y;
+        }
+        if (MODE == CB_LINEAR) {
+          const C g = a.g[c * nh + m];
+          re += L * g.x, im += L * g.y;
+        }
+        a.out[c * nh + m] = mkc<C>(T(re), T(im));
+      }
+    }
   }
 }
 
@@ -267,21 +327,6 @@ __global__ void k_residual(const C *u, const C *N, C *gE, long long nh, Grid3 gr
   if (threadIdx.x == 0) partials[blockIdx.x] = v[0];
 }
 
-// grad += L gE
-template <typename C>
-__global__ void k_add_linear(C *grad, const C *gE, long long nh, Grid3 gr, double nu, double Q) {
-  using T = decltype(C{}.x);
-  GRID_LOOP(m, nh) {
-    double kx, ky, kz;
-    mode_k(gr, m, kx, ky, kz);
-    const double L = Q - nu * (kx * kx + ky * ky + kz * kz);
-    for (int c = 0; c < 3; ++c) {
-      const C a = grad[c * nh + m], b = gE[c * nh + m];
-      grad[c * nh + m] = mkc<C>(T(a.x + L * b.x), T(a.y + L * b.y));
-    }
-  }
-}
-
 // d = -P D (grad / (s^2 W)): the steepest-descent direction in the
 // mean-square metric <|u|^2> = s^2 sum_half W |uhat|^2 of J's own norm,
 // projected and dealiased so the state stays admissible; per-block partials
@@ -313,22 +358,6 @@ __global__ void k_descent_dir(const C *grad, C *d, long long nh, Grid3 gr, doubl
   double v[1] = {acc};
   block_sum<1>(v, red);
   if (threadIdx.x == 0) partials[blockIdx.x] = v[0];
-}
-
-// out = IF (u + dt n), IF = exp((Q - nu |k|^2) dt): the FIN_PRED arithmetic of k_finish_rows
-template <typename C>
-__global__ void k_if_pred(const C *u, const C *n, C *out, long long nh, Grid3 gr, double nu, double Q, double dt) {
-  using T = decltype(C{}.x);
-  GRID_LOOP(m, nh) {
-    double kx, ky, kz;
-    mode_k(gr, m, kx, ky, kz);
-    const T IF = T(exp((Q - nu * (kx * kx + ky * ky + kz * kz)) * dt));
-    const T tdt = T(dt);
-    for (int c = 0; c < 3; ++c) {
-      const C a = u[c * nh + m], b = n[c * nh + m];
-      out[c * nh + m] = mkc<C>((a.x + tdt * b.x) * IF, (a.y + tdt * b.y) * IF);
-    }
-  }
 }
 
 // y = s x over n complex values
@@ -435,56 +464,159 @@ int sum_to_host(dnsbox_ctx *c, int nblk, double *out) {
   return DNSBOX_OK;
 }
 
+// The transposed term from hw = h / W (spectral): C2R of u, omega and phi, the
+// cross products and their R2C, and the combination in `mode`.  The fields run
+// through the padded workspace (W1, W2 and the six slots of wphi); lines that
+// the fused x kernel does not take go through physical fields.
 template <typename T>
-int vjp_impl(dnsbox_ctx *c, const void *uh, const void *g, void *out) {
+int vjp_core(dnsbox_ctx *c, const void *uh, const char *hw, int mode, CombineArgs<typename CT<T>::type> cb) {
   using C = typename CT<T>::type;
   const dnsbox_params &p = c->p;
   const double s = 1.0 / ((double)p.nx * p.ny * p.nz);
   const size_t pb = c->np * sizeof(T), sb = c->nh * sizeof(C);
-  char *P = nullptr, *S = nullptr;
-  RET(ensure_adj(c, 9, 6, &P, &S));
-  const Grid3 gr = grid3(c);
-  const int gb = grid_for((long long)c->nh);
-  const long long nh = (long long)c->nh, np = (long long)c->np;
+  const long long np = (long long)c->np;
   const char *u = reinterpret_cast<const char *>(uh);
-  k_vjp_pre<C><<<gb, 256, 0, c->stream>>>(reinterpret_cast<const C *>(g), reinterpret_cast<C *>(S), nh, gr);
-  CK(cudaGetLastError());
-  // u (scaled), omega = ik x u (scaled), phi = C2R(h / W)
-  const void *u0 = u, *u1 = u + sb, *u2 = u + 2 * sb;
-  SpecJob jobs[9] = {
-      {{{u0, s, 0, 0}, {nullptr, 0, 0, 0}}, 1},
-      {{{u1, s, 0, 0}, {nullptr, 0, 0, 0}}, 1},
-      {{{u2, s, 0, 0}, {nullptr, 0, 0, 0}}, 1},
-      {{{u2, 0, s, 2}, {u1, 0, -s, 1}}, 2},   // i (ky w - kz v)
-      {{{u0, 0, s, 1}, {u2, 0, -s, 0}}, 2},   // i (kz u - kx w)
-      {{{u1, 0, s, 0}, {u0, 0, -s, 2}}, 2},   // i (kx v - ky u)
-      {{{S, 1, 0, 0}, {nullptr, 0, 0, 0}}, 1},
-      {{{S + sb, 1, 0, 0}, {nullptr, 0, 0, 0}}, 1},
-      {{{S + 2 * sb, 1, 0, 0}, {nullptr, 0, 0, 0}}, 1},
-  };
-  void *outs[9];
-  for (int i = 0; i < 9; ++i) outs[i] = P + i * pb;
-  RET(c2r_jobs<T>(c, 9, jobs, outs, 1.0));
-  k_vjp_cross<T><<<grid_for(np), 256, 0, c->stream>>>(reinterpret_cast<T *>(P), np);
-  CK(cudaGetLastError());
-  const void *ins[6];
-  void *specs[6];
-  for (int i = 0; i < 6; ++i) {
-    ins[i] = P + i * pb;
-    specs[i] = S + i * sb;
-  }
-  RET(r2c_fields<T>(c, 6, ins, specs));
-  k_vjp_combine<C><<<gb, 256, 0, c->stream>>>(reinterpret_cast<const C *>(S), reinterpret_cast<const C *>(S + 3 * sb),
-                                              reinterpret_cast<C *>(out), nh, gr, s);
-  CK(cudaGetLastError());
-  if (p.bandlim && c->nband) {
-    k_eband<C><<<1, 256, 0, c->stream>>>(band_args(c, uh), p.nx, 0);
-    k_vjp_band<C><<<1, 256, 0, c->stream>>>(reinterpret_cast<const C *>(uh), reinterpret_cast<const C *>(g),
-                                            reinterpret_cast<C *>(out), nh, c->band, c->nband, gr, c->st, p.Pin,
-                                            s * s);
+  auto wf = [&](char *base, int slot) { return wfield(base, c, slot); };
+  if (Ops<T>::has_xline_vjp(p.nx)) {
+    if (!c->wphi) CK(cudaMalloc(&c->wphi, 6 * c->wstride * c->cbytes));
+    // inverse z: u (scaled), -dz v, dz u, phi
+    StridedArgs<T> a = strided_base<T>(c, 2);
+    strided_ws<T>(c, a, 2, false, true);
+    a.njobs = 8;
+    for (int f = 0; f < 3; ++f) {
+      set_job<T>(a, f, u + f * sb, wf(c->W1, f), s);
+      set_job<T>(a, 5 + f, hw + f * sb, wf(c->wphi, f));
+    }
+    set_job<T>(a, 3, u + sb, wf(c->W1, 3), 0.0, -s, 1);
+    set_job<T>(a, 4, u, wf(c->W1, 4), 0.0, s, 1);
+    RET(run_strided<T>(c, 2, true, a, DNSBOX_PASS_OTHER, false));
+    // inverse y: u, omega (the derivatives along y and x of the scaled u), phi
+    StridedArgs<T> b = strided_base<T>(c, 1);
+    strided_ws<T>(c, b, 1, true, true);
+    b.njobs = 9;
+    for (int f = 0; f < 3; ++f) {
+      set_job<T>(b, f, wf(c->W1, f), wf(c->W2, f));
+      set_job<T>(b, 6 + f, wf(c->wphi, f), wf(c->wphi, 3 + f));
+    }
+    set_job<T>(b, 3, wf(c->W1, 2), wf(c->W2, 3), 0.0, 1.0, 1, wf(c->W1, 3));
+    set_job<T>(b, 4, wf(c->W1, 4), wf(c->W2, 4), 1.0, 0.0, 0, wf(c->W1, 2), 0.0, -1.0, 0);
+    set_job<T>(b, 5, wf(c->W1, 0), wf(c->W2, 5), 0.0, -1.0, 1, wf(c->W1, 1), 0.0, 1.0, 0);
+    RET(run_strided<T>(c, 1, true, b, DNSBOX_PASS_OTHER, false));
+    XlineVjpArgs<T> x;
+    memset(&x, 0, sizeof(x));
+    const C **in[9] = {&x.U, &x.V, &x.W, &x.OX, &x.OY, &x.OZ, &x.FX, &x.FY, &x.FZ};
+    for (int f = 0; f < 9; ++f) *in[f] = reinterpret_cast<const C *>(f < 6 ? wf(c->W2, f) : wf(c->wphi, f - 3));
+    for (int f = 0; f < 3; ++f) {
+      x.A[f] = reinterpret_cast<C *>(wf(c->W1, f));
+      x.B[f] = reinterpret_cast<C *>(wf(c->W1, 3 + f));
+    }
+    x.tw = reinterpret_cast<const C *>(c->tw[0]);
+    x.nlines = p.ny * p.nz;
+    x.pitch = c->wp;
+    {
+      Prof pr(c, DNSBOX_PASS_OTHER);
+      CK(Ops<T>::xline_vjp(p.nx, x, c->stream));
+    }
+  } else {
+    char *P = nullptr, *S = nullptr;
+    RET(ensure_adj(c, 9, 6, &P, &S));
+    const char *u0 = u, *u1 = u + sb, *u2 = u + 2 * sb;
+    SpecJob jobs[9] = {
+        {{{u0, s, 0, 0}, {nullptr, 0, 0, 0}}, 1},
+        {{{u1, s, 0, 0}, {nullptr, 0, 0, 0}}, 1},
+        {{{u2, s, 0, 0}, {nullptr, 0, 0, 0}}, 1},
+        {{{u2, 0, s, 2}, {u1, 0, -s, 1}}, 2},   // i (ky w - kz v)
+        {{{u0, 0, s, 1}, {u2, 0, -s, 0}}, 2},   // i (kz u - kx w)
+        {{{u1, 0, s, 0}, {u0, 0, -s, 2}}, 2},   // i (kx v - ky u)
+        {{{hw, 1, 0, 0}, {nullptr, 0, 0, 0}}, 1},
+        {{{hw + sb, 1, 0, 0}, {nullptr, 0, 0, 0}}, 1},
+        {{{hw + 2 * sb, 1, 0, 0}, {nullptr, 0, 0, 0}}, 1},
+    };
+    void *outs[9];
+    for (int i = 0; i < 9; ++i) outs[i] = P + i * pb;
+    RET(c2r_jobs<T>(c, 9, jobs, outs, 1.0));
+    k_vjp_cross<T><<<grid_for(np), 256, 0, c->stream>>>(reinterpret_cast<T *>(P), np);
     CK(cudaGetLastError());
+    XlineArgs<T> x;
+    memset(&x, 0, sizeof(x));
+    for (int f = 0; f < 6; ++f) {
+      x.in[f] = P + f * pb;
+      x.out[f] = wf(c->W1, f);
+    }
+    x.tw = reinterpret_cast<const C *>(c->tw[0]);
+    x.nlines = p.ny * p.nz;
+    x.nxh = c->nxh;
+    x.pitch = c->wp;
+    x.scale = 1.0;
+    Prof pr(c, DNSBOX_PASS_OTHER);
+    CK(Ops<T>::xline_r2c(p.nx, x, 6, c->stream));
+  }
+  // forward y, forward z in place
+  StridedArgs<T> d = strided_base<T>(c, 1);
+  strided_ws<T>(c, d, 1, true, true);
+  d.njobs = 6;
+  for (int f = 0; f < 6; ++f) set_job<T>(d, f, wf(c->W1, f), wf(c->W2, f));
+  RET(run_strided<T>(c, 1, false, d, DNSBOX_PASS_OTHER, false));
+  StridedArgs<T> z = strided_base<T>(c, 2);
+  strided_ws<T>(c, z, 2, true, true);
+  z.njobs = 6;
+  for (int f = 0; f < 6; ++f) set_job<T>(z, f, wf(c->W2, f), wf(c->W2, f));
+  RET(run_strided<T>(c, 2, false, z, DNSBOX_PASS_OTHER, false));
+  cb.ws = reinterpret_cast<const C *>(c->W2);
+  cb.wst = (long long)c->wstride;
+  cb.pitch = c->wp;
+  cb.nh = (long long)c->nh;
+  cb.gr = grid3(c);
+  cb.s = s;
+  cb.nu = p.nu;
+  cb.Q = p.Q;
+  const int nb = row_blocks(cb.gr);
+  switch (mode) {
+    case CB_OUT: CK(launch_pdl(k_vjp_combine<C, CB_OUT>, nb, 256, 0, c->stream, cb)); break;
+    case CB_ADD: CK(launch_pdl(k_vjp_combine<C, CB_ADD>, nb, 256, 0, c->stream, cb)); break;
+    case CB_LINEAR: CK(launch_pdl(k_vjp_combine<C, CB_LINEAR>, nb, 256, 0, c->stream, cb)); break;
+    default: CK(launch_pdl(k_vjp_combine<C, CB_STEP>, nb, 256, 0, c->stream, cb)); break;
   }
   return DNSBOX_OK;
+}
+
+// h / W = -P(D scale g) / W into the arena's first spectral slots.
+template <typename T> int vjp_pre(dnsbox_ctx *c, const void *g, double scale, char **hw) {
+  using C = typename CT<T>::type;
+  char *P = nullptr;
+  RET(ensure_adj(c, 9, 6, &P, hw));
+  const Grid3 gr = grid3(c);
+  CK(launch_pdl(k_vjp_pre<C>, row_blocks(gr), 256, 0, c->stream, reinterpret_cast<const C *>(g),
+                reinterpret_cast<C *>(*hw), (long long)c->nh, gr, scale));
+  return DNSBOX_OK;
+}
+
+// The band forcing's part of the transposed term, added to out.
+template <typename T> int vjp_band(dnsbox_ctx *c, const void *uh, const void *g, void *out) {
+  using C = typename CT<T>::type;
+  const dnsbox_params &p = c->p;
+  if (!p.bandlim || !c->nband) return DNSBOX_OK;
+  const double s = 1.0 / ((double)p.nx * p.ny * p.nz);
+  k_eband<C><<<1, 256, 0, c->stream>>>(band_args(c, uh), p.nx, 0);
+  k_vjp_band<C><<<1, 256, 0, c->stream>>>(reinterpret_cast<const C *>(uh), reinterpret_cast<const C *>(g),
+                                          reinterpret_cast<C *>(out), (long long)c->nh, c->band, c->nband, grid3(c),
+                                          c->st, p.Pin, s * s);
+  CK(cudaGetLastError());
+  return DNSBOX_OK;
+}
+
+// out = N'(u)^T g; with linear, out = (L + N'(u))^T g.
+template <typename T>
+int vjp_impl(dnsbox_ctx *c, const void *uh, const void *g, void *out, bool linear = false) {
+  using C = typename CT<T>::type;
+  char *hw = nullptr;
+  RET(vjp_pre<T>(c, g, 1.0, &hw));
+  CombineArgs<C> cb;
+  memset(&cb, 0, sizeof(cb));
+  cb.out = reinterpret_cast<C *>(out);
+  cb.g = reinterpret_cast<const C *>(g);
+  RET(vjp_core<T>(c, uh, hw, linear ? CB_LINEAR : CB_OUT, cb));
+  return vjp_band<T>(c, uh, g, out);
 }
 
 template <typename T>
@@ -561,17 +693,10 @@ int residual_fwd(dnsbox_ctx *c, const void *uh, bool weighted, double *partials)
 template <typename T>
 int residual_bwd(dnsbox_ctx *c, const void *uh, void *grad) {
   using C = typename CT<T>::type;
-  const dnsbox_params &p = c->p;
   const size_t sb = c->nh * sizeof(C);
   char *P = nullptr, *S = nullptr;
   RET(ensure_adj(c, 9, 12, &P, &S));
-  char *gE = S + 9 * sb;
-  const Grid3 gr = grid3(c);
-  RET(vjp_impl<T>(c, uh, gE, grad));
-  k_add_linear<C><<<grid_for((long long)c->nh), 256, 0, c->stream>>>(
-      reinterpret_cast<C *>(grad), reinterpret_cast<const C *>(gE), (long long)c->nh, gr, p.nu, p.Q);
-  CK(cudaGetLastError());
-  return DNSBOX_OK;
+  return vjp_impl<T>(c, uh, S + 9 * sb, grad, true);
 }
 
 // J (and, when grad != null, its Euclidean gradient) at uh.  Uses arena
@@ -580,8 +705,19 @@ template <typename T>
 int residual_impl(dnsbox_ctx *c, const void *uh, void *grad, double *J) {
   RET(ensure_red(c, 2 * kRedBlocks + 2));
   RET(residual_fwd<T>(c, uh, grad != nullptr, c->red));
-  RET(sum_to_host(c, kRedBlocks, J));
-  if (grad) RET(residual_bwd<T>(c, uh, grad));
+  if (!grad || c->tc) {
+    RET(sum_to_host(c, kRedBlocks, J));
+    return grad ? residual_bwd<T>(c, uh, grad) : DNSBOX_OK;
+  }
+  // J is on its way to the host while the gradient half is queued and runs
+  k_sum_scalar<256><<<1, 256, 0, c->stream>>>(c->red, kRedBlocks, c->red + kRedBlocks);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(c->hstage, c->red + kRedBlocks, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  if (!c->read_ev) CK(cudaEventCreateWithFlags(&c->read_ev, cudaEventDisableTiming));
+  CK(cudaEventRecord(c->read_ev, c->stream));
+  RET(residual_bwd<T>(c, uh, grad));
+  CK(cudaEventSynchronize(c->read_ev));
+  *J = c->hstage[0];
   return DNSBOX_OK;
 }
 
@@ -786,34 +922,44 @@ int step_vjp_ok(dnsbox_ctx *c) {
   return DNSBOX_OK;
 }
 
-// One step transpose: out = S'(u)^T g.  Arena spectral slots 21-32 (0-5 belong
-// to the rhs VJP).  out may not alias u or g.
+// One step transpose: out = S'(u)^T g.  Arena spectral slots 24-32 (0-5 belong
+// to the rhs VJP).  out may not alias u or g.  pruned: u (and the arena's u*,
+// whose cut set the caller zeroed) vanishes on the 2/3-rule cut set.
 template <typename T>
-int step_vjp_impl(dnsbox_ctx *c, const void *uh, const void *g, void *out, double dt) {
+int step_vjp_impl(dnsbox_ctx *c, const void *uh, const void *g, void *out, double dt, bool pruned = false) {
   using C = typename CT<T>::type;
   const dnsbox_params &p = c->p;
   const size_t sb = c->nh * sizeof(C);
-  char *P = nullptr, *S = nullptr;
+  char *P = nullptr, *S = nullptr, *hw = nullptr;
   RET(ensure_adj(c, 9, 33, &P, &S));
-  char *n0 = S + 21 * sb, *ust = S + 24 * sb, *A = S + 27 * sb, *tmp = S + 30 * sb;
-  const Grid3 gr = grid3(c);
-  const long long nh = (long long)c->nh, n3 = 3 * nh;
-  {
-    const int rc = dnsbox_rhs_nonlinear(c, uh, n0, nullptr);
-    if (rc != DNSBOX_OK) return rc;
+  char *ust = S + 24 * sb, *A = S + 27 * sb, *tmp = S + 30 * sb;
+  const long long nh = (long long)c->nh;
+  RET(rhs_predictor_impl(c, uh, ust, pruned));            // u* = IF (u + dt N(u))
+  CombineArgs<C> cb;
+  memset(&cb, 0, sizeof(cb));
+  cb.g = reinterpret_cast<const C *>(g);
+  cb.dt = dt;
+  if (!(p.bandlim && c->nband)) {
+    RET(vjp_pre<T>(c, g, 0.5 * dt, &hw));
+    cb.out = reinterpret_cast<C *>(out);
+    cb.hw = reinterpret_cast<C *>(hw);
+    RET(vjp_core<T>(c, ust, hw, CB_STEP, cb));            // a = N'(u*)^T (dt/2 g); out = IF (g + a); h of IF (dt/2 g + dt a)
+    RET(vjp_core<T>(c, uh, hw, CB_ADD, cb));              // out += N'(u)^T (IF (dt/2 g + dt a))
+    return DNSBOX_OK;
   }
-  k_if_pred<C><<<grid_for(nh), 256, 0, c->stream>>>(reinterpret_cast<const C *>(uh), reinterpret_cast<const C *>(n0),
-                                                     reinterpret_cast<C *>(ust), nh, gr, p.nu, p.Q, dt);
+  // with band forcing its part comes between
+  const Grid3 gr = grid3(c);
+  const long long n3 = 3 * nh;
   k_scale<C><<<grid_for(n3), 256, 0, c->stream>>>(reinterpret_cast<const C *>(g), reinterpret_cast<C *>(tmp), n3,
                                                    0.5 * dt);
   CK(cudaGetLastError());
-  RET(vjp_impl<T>(c, ust, tmp, A));                       // a = N'(u*)^T (dt/2 g)
+  RET(vjp_impl<T>(c, ust, tmp, A));
   k_step_mix<C><<<grid_for(nh), 256, 0, c->stream>>>(reinterpret_cast<const C *>(g), reinterpret_cast<const C *>(A),
                                                       reinterpret_cast<C *>(out), reinterpret_cast<C *>(tmp), nh, gr,
                                                       p.nu, p.Q, dt);
   CK(cudaGetLastError());
-  RET(vjp_impl<T>(c, uh, tmp, n0));                       // N'(u)^T (IF (dt/2 g + dt a))
-  k_accum<C><<<grid_for(n3), 256, 0, c->stream>>>(reinterpret_cast<C *>(out), reinterpret_cast<const C *>(n0), n3,
+  RET(vjp_impl<T>(c, uh, tmp, A));
+  k_accum<C><<<grid_for(n3), 256, 0, c->stream>>>(reinterpret_cast<C *>(out), reinterpret_cast<const C *>(A), n3,
                                                    1.0);
   CK(cudaGetLastError());
   return DNSBOX_OK;
@@ -847,6 +993,12 @@ int steps_vjp_impl(dnsbox_ctx *c, const void *u0, int nsteps, int every, const v
     if (n % every == 0) CK(cudaMemcpyAsync(cp + (size_t)(n / every) * sb3, seg, sb3, cudaMemcpyDeviceToDevice, c->stream));
     RET(step_advance_decided(c, seg, 1, n == 0));   // pruning decided once for the trajectory
   }
+  const bool pruned = c->prune_now;   // of every state of this trajectory
+  if (pruned) {   // the pruned predictor leaves the cut set of u* as it is
+    char *P = nullptr, *S = nullptr;
+    RET(ensure_adj(c, 9, 33, &P, &S));
+    CK(cudaMemsetAsync(S + 24 * c->nh * sizeof(C), 0, sb3, c->stream));
+  }
   if (uT_out) CK(cudaMemcpyAsync(uT_out, seg, sb3, cudaMemcpyDeviceToDevice, c->stream));
   // backward sweep, one segment at a time
   CK(cudaMemcpyAsync(ga, gT, sb3, cudaMemcpyDeviceToDevice, c->stream));
@@ -859,7 +1011,7 @@ int steps_vjp_impl(dnsbox_ctx *c, const void *u0, int nsteps, int every, const v
       RET(step_advance_decided(c, seg + (size_t)j * sb3, 1, false));
     }
     for (int j = len - 1; j >= 0; --j) {
-      RET(step_vjp_impl<T>(c, seg + (size_t)j * sb3, ga, gb, dt));
+      RET(step_vjp_impl<T>(c, seg + (size_t)j * sb3, ga, gb, dt, pruned));
       char *t = ga;
       ga = gb;
       gb = t;

@@ -1144,6 +1144,8 @@ static void free_ctx(dnsbox_ctx *c) {
   if (!c) return;
   cudaFree(c->adft);
   cudaFree(c->tc_status);
+  cudaFree(c->wphi);
+  if (c->read_ev) cudaEventDestroy(c->read_ev);
   cudaFree(c->cut_flag);
   for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
   cudaFree(c->W1);
@@ -1408,6 +1410,12 @@ extern "C" int dnsbox_reset_history(dnsbox_ctx *ctx) {
 int rhs_nonlinear_impl(dnsbox_ctx *ctx, const void *uh, void *out) {
   return ctx->fp64 ? run_rhs<double>(ctx, uh, FIN_RHS, out, nullptr, nullptr, false, 0, nullptr)
                    : run_rhs<float>(ctx, uh, FIN_RHS, out, nullptr, nullptr, false, 0, nullptr);
+}
+
+// Internal: the predictor IF (u + dt N(u)) into out, with the context's dt.
+int rhs_predictor_impl(dnsbox_ctx *ctx, const void *uh, void *out, bool pruned) {
+  return ctx->fp64 ? run_rhs<double>(ctx, uh, FIN_PRED, out, nullptr, nullptr, false, 0, nullptr, pruned)
+                   : run_rhs<float>(ctx, uh, FIN_PRED, out, nullptr, nullptr, false, 0, nullptr, pruned);
 }
 
 extern "C" int dnsbox_rhs_nonlinear(dnsbox_ctx *ctx, const void *uh, void *out, double *eband) {

@@ -42,6 +42,9 @@ int step_advance_decided(dnsbox_ctx *c, void *uh, int nsteps, bool decide);
 // N(u) into out on the context's stream, without device selection or host
 // synchronisation (api.cu).
 int rhs_nonlinear_impl(dnsbox_ctx *ctx, const void *uh, void *out);
+// IF (u + dt N(u)) into out on the context's stream; pruned passes (which leave
+// out's cut set as it is) where the caller knows that u vanishes there (api.cu).
+int rhs_predictor_impl(dnsbox_ctx *ctx, const void *uh, void *out, bool pruned);
 // Releases the adjoint descent's captured graphs and stream (adjoint.cu).
 void descent_graphs_free(dnsbox_ctx *c);
 // Synchronises the context's stream and returns DNSBOX_ERR_TIMEOUT (clearing
@@ -109,6 +112,8 @@ struct dnsbox_ctx {
   int sched_x = 0;
   char *adj = nullptr;                   // adjoint arena
   size_t adj_bytes = 0;
+  char *wphi = nullptr;                  // transposed term: 6 workspace slots beside W1 and W2 (on first use)
+  cudaEvent_t read_ev = nullptr;         // a read-back that later work does not delay (on first use)
   char *orbit = nullptr;                 // checkpoints and segment states of the step-transpose chain
   size_t orbit_bytes = 0;
   DescentGraphs *descent = nullptr;      // adjoint descent: captured launch sequences (adjoint.cu)
@@ -214,6 +219,18 @@ template <typename T> struct Ops {
   static bool has_xline_warp(int n) {
     switch (n) { DNSBOX_SIZES(DNSBOX_CASE_HASXW) }
     return false;
+  }
+#define DNSBOX_CASE_HASXV(NN) \
+  case NN: return Launcher<T, NN>::has_xline_vjp();
+  static bool has_xline_vjp(int n) {
+    switch (n) { DNSBOX_SIZES(DNSBOX_CASE_HASXV) }
+    return false;
+  }
+#define DNSBOX_CASE_XV(NN) \
+  case NN: return Launcher<T, NN>::xline_vjp(a, st);
+  static cudaError_t xline_vjp(int n, const XlineVjpArgs<T> &a, cudaStream_t st) {
+    switch (n) { DNSBOX_SIZES(DNSBOX_CASE_XV) }
+    return cudaErrorInvalidValue;
   }
 #define DNSBOX_CASE_C2R(NN) \
   case NN: return Launcher<T, NN>::xline_c2r(a, nf, st);

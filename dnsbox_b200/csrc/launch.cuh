@@ -43,6 +43,8 @@ template <typename T, int N> struct Launcher {
   // 1 is the block kernel and anything else the warp kernel; at 1024 the block kernel
   static cudaError_t xline_nl(const XlineNLArgs<T> &a, int variant, cudaStream_t st);
   static bool has_xline_warp();
+  static bool has_xline_vjp();
+  static cudaError_t xline_vjp(const XlineVjpArgs<T> &a, cudaStream_t st);
   static cudaError_t xline_c2r(const XlineArgs<T> &a, int nf, cudaStream_t st);
   static cudaError_t xline_r2c(const XlineArgs<T> &a, int nf, cudaStream_t st);
 };
@@ -193,6 +195,23 @@ cudaError_t Launcher<T, N>::xline_nl(const XlineNLArgs<T> &a, int variant, cudaS
     k_xline_nl<T, N><<<(unsigned)((a.nlines + B - 1) / B), nt, smem, st>>>(a);
   }
   return cudaGetLastError();
+}
+
+template <typename T, int N> bool Launcher<T, N>::has_xline_vjp() { return XReg<T, N>::on; }
+template <typename T, int N>
+cudaError_t Launcher<T, N>::xline_vjp(const XlineVjpArgs<T> &a, cudaStream_t st) {
+  if constexpr (XReg<T, N>::on) {
+    using SH = XReg<T, N>;
+    int nt = SH::NT;
+    while (nt > 32 && (long long)a.nlines * SH::PL::P < 148LL * 4 * nt) nt >>= 1;
+    const int lpb = nt / SH::PL::P;
+    const cudaError_t e = set_smem(k_xline_vjp<T, N>, SH::smem(nt));
+    if (e != cudaSuccess) return e;
+    return launch_pdl(k_xline_vjp<T, N>, (unsigned)((a.nlines + lpb - 1) / lpb), nt, SH::smem(nt), st, a);
+  } else {
+    (void)a, (void)st;
+    return cudaErrorInvalidValue;
+  }
 }
 
 // Threads of a plain x-line block: smaller blocks where the lines are few.

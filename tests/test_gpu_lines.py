@@ -60,3 +60,18 @@ def test_maxima_of_boxes_sharing_a_warp(nx):
         assert torch.equal(v, u[:, i])
         one.close()
     batch.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("nx", SIZES[:-1])
+def test_transposed_term_line_length(nx, prec):
+    """The transposed right-hand side at every x length (fused kernel and, at 512 in FP64, the physical fields)."""
+    from dnsbox_b200.ops import Box
+    ny, nz = 12, 8
+    g = O.Grid(O.Params(nx=nx, ny=ny, nz=nz, bandlim=False))
+    uh, gr = rough(g, nx, ny, nz, seed=nx), rough(g, nx, ny, nz, seed=nx + 1) * 1e-3
+    b = Box(nx=nx, ny=ny, nz=nz, precision=prec, bandlim=False)
+    got = b.rhs_nonlinear_vjp(b.from_numpy(uh), b.from_numpy(gr))
+    # a chain of transforms for u and one for g: twice the bar of a right-hand side
+    assert rel(got.cpu().numpy(), O.rhs_nonlinear_vjp(g, uh, gr)) < 2 * TOL[prec]
+    b.close()
