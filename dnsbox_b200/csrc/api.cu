@@ -537,25 +537,28 @@ __global__ void k_convert(const A *src, B *dst, long long n) {
     dst[i] = (B)src[i];
 }
 
-// Sets *flag when any component of a state (3 fields nh apart) is nonzero
-// (or not a number) at a mode outside the kept set of the pruning rule.
+// Sets *flag when any component of a state is nonzero (or not a number) at a
+// mode outside the kept set of the pruning rule.  One warp per (kz, ky) row and
+// box (blockIdx.y): whole rows outside the kept kz and ky, elsewhere the cut kx
+// only (256^3 FP32: 69 -> 30 us against one mode per thread over all modes).
 template <typename C>
-__global__ void k_cut_check(const C *u, long long nh, long long fstride, int nxh, int ny, AxisKeep kx, AxisKeep ky,
+__global__ void k_cut_check(const C *u, long long nh, long long fstride, int nxh, int ny, int nz, AxisKeep kx, AxisKeep ky,
                             AxisKeep kz, int *flag) {
-  // m runs over the modes of every box (fstride = nbatch * nh per component)
-  for (long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x; m < fstride;
-       m += (long long)gridDim.x * blockDim.x) {
-    const long long mb = m % nh;
-    const int ix = (int)(mb % nxh), iy = (int)((mb / nxh) % ny), iz = (int)(mb / ((long long)nxh * ny));
-    if (kx.keep(ix) && ky.keep(iy) && kz.keep(iz)) continue;
-    for (int c = 0; c < 3; ++c) {
-      const C v = u[c * fstride + m];
-      if (!(v.x == 0 && v.y == 0)) {
-        *flag = 1;
-        return;
-      }
+  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= ny * nz) return;
+  const int iz = row / ny, iy = row - iz * ny;
+  const bool kept = ky.keep(iy) && kz.keep(iz);
+  const C *r = u + (long long)blockIdx.y * nh + (long long)row * nxh;
+  const int nyq = kx.n >> 1;
+  bool bad = false;
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll 2
+    for (int ix = (kept ? kx.a : 0) + lane; ix < (kept ? nyq : nxh); ix += 32) {
+      const C v = r[c * fstride + ix];
+      bad = bad || !(v.x == 0 && v.y == 0);
     }
-  }
+  if (__any_sync(0xffffffffu, bad) && lane == 0) *flag = 1;
 }
 
 template <typename T> static FinishArgs<T> finish_base(const dnsbox_ctx *c) {
@@ -1037,8 +1040,8 @@ template <typename T> static int step_once(dnsbox_ctx *c, void *uh) {
 template <typename T> static int cut_check_async(dnsbox_ctx *c, const void *uh) {
   using C = typename CT<T>::type;
   CK(cudaMemsetAsync(c->cut_flag, 0, sizeof(int), c->stream));
-  k_cut_check<C><<<grid_for((long long)c->fstride), 256, 0, c->stream>>>(
-      reinterpret_cast<const C *>(uh), (long long)c->nh, (long long)c->fstride, c->nxh, c->p.ny, c->keep[0],
+  k_cut_check<C><<<dim3((unsigned)((c->p.ny * c->p.nz + 7) / 8), (unsigned)c->nbatch), 256, 0, c->stream>>>(
+      reinterpret_cast<const C *>(uh), (long long)c->nh, (long long)c->fstride, c->nxh, c->p.ny, c->p.nz, c->keep[0],
       c->keep[1], c->keep[2], c->cut_flag);
   CK(cudaGetLastError());
   return DNSBOX_OK;

@@ -301,7 +301,7 @@ DNSBOX_VPLAN(96, 12, 4, 4, 6)
 DNSBOX_VPLAN(128, 16, 16, 8)
 DNSBOX_VPLAN(192, 12, 4, 4, 12)
 DNSBOX_VPLAN(256, 16, 16, 16)
-DNSBOX_VPLAN(512, 8, 8, 8, 8)
+DNSBOX_VPLAN(512, 16, 16, 8, 4)
 DNSBOX_VPLAN(1024, 16, 16, 16, 4)
 #undef DNSBOX_VPLAN
 
@@ -316,7 +316,6 @@ template <typename T, int N> struct XPlan : VPlan<N> {};
     static constexpr int NST = sizeof(R) / sizeof(int);                                                              \
     __host__ __device__ static constexpr int ns(int s) { int q = 1; for (int i = 0; i < s; ++i) q *= R[i]; return q; } \
   };
-DNSBOX_XPLAN(float, 512, 16, 16, 8, 4)
 DNSBOX_XPLAN(double, 128, 8, 8, 4, 4)
 DNSBOX_XPLAN(double, 256, 8, 8, 8, 4)
 #undef DNSBOX_XPLAN

@@ -105,6 +105,7 @@ __device__ __forceinline__ void eband_block(const BandArgs &b, int nx, int box, 
   const C *u = reinterpret_cast<const C *>(b.u) + (long long)box * b.bstride;
   StepState *st = b.st + box;
   double acc = 0.0;
+#pragma unroll 4
   for (int i = threadIdx.x; i < b.n; i += blockDim.x) {
     const long long off = (long long)(unsigned)b.modes[3 * i] | ((long long)b.modes[3 * i + 1] << 32);
     const int kx = b.modes[3 * i + 2];
@@ -230,11 +231,13 @@ template <typename T, int N> struct StridedShape {
     return n < 256 ? 256 : n;   // 32 doubles for the band block
   }
   // Resident CTAs asked of the register allocator: 16 warps per SM where a
-  // thread holds 16 values (128 registers), 20 at 12 (96), 24 at 8 (80), 32 in
-  // the 512-thread blocks of N = 512 (64).  The 256-row pass with 8 values,
-  // three stages and 32 warps measured the same (57.7 against 56.7 us for pass
-  // D): the loads in flight per SM are equal.
-  static constexpr int warps = PL::E >= 16 ? 16 : PL::E == 12 ? 20 : N >= 512 ? 32 : 24;
+  // thread holds 16 values (128 registers), 20 at 12 (96), 24 at 8 (80).  The
+  // 256-row pass with 8 values, three stages and 32 warps measured the same
+  // (57.7 against 56.7 us for pass D: the loads in flight per SM are equal);
+  // at 512, whose 8-value plan spills at the 64 registers of 32 warps, 16
+  // values take passes A / D / E1 from 553 / 355 / 261 to 516 / 326 / 236 us
+  // (512^3 FP32); at 96, 24 values in two stages take pass B from 224 to 252.
+  static constexpr int warps = PL::E >= 16 ? 16 : PL::E == 12 ? 20 : 24;
   static constexpr int wcta = round32(NT) / 32;
   static constexpr int minb = warps / wcta < 1 ? 1 : warps / wcta;
 };
@@ -423,8 +426,7 @@ __global__ void __launch_bounds__(StridedShape<T, N>::NT, StridedShape<T, N>::mi
   }
   // second inputs: a part of the rows at a time, so that their loads in flight
   // fit beside the first input's values; the first part right away
-  // (at 512, held to 64 registers, a quarter: all eight rows spill 290 bytes)
-  constexpr int QN = N == 512 ? 2 : E <= 8 ? E : E / 2;
+  constexpr int QN = E <= 8 ? E : E / 2;
   const C *const in2p = INV ? jb.in2 : nullptr;
   Raw w[INV ? QN : 1];
   if (INV && in2p) load(in2p, w, 0, QN);
@@ -906,10 +908,11 @@ template <int E, typename C, typename PUT> __device__ __forceinline__ void pack_
   }
 }
 
-// The power of two that brings the half line x2 of a line to the magnitude of
-// x1 (the exponent difference of their largest components, over the line's P
-// lanes): the parts of one complex sequence are rounded relative to each other.
-template <int P, int H, typename C> __device__ __forceinline__ decltype(C{}.x) balance(const C *x1, const C *x2) {
+// The exponent e with which 2^e brings the half line x2 of a line to the
+// magnitude of x1 (the exponent difference of their largest components, over
+// the line's P lanes): the parts of one complex sequence are rounded relative
+// to each other.
+template <int P, int H, typename C> __device__ __forceinline__ int balance(const C *x1, const C *x2) {
   using T = decltype(C{}.x);
   T m1 = 0, m2 = 0;
 #pragma unroll
@@ -925,7 +928,7 @@ template <int P, int H, typename C> __device__ __forceinline__ decltype(C{}.x) b
   int e1 = 0, e2 = 0;
   frexp(m1, &e1);
   frexp(m2, &e2);
-  return ldexp(T(1), m1 > 0 && m2 > 0 ? max(-96, min(96, e1 - e2)) : 0);
+  return m1 > 0 && m2 > 0 ? max(-96, min(96, e1 - e2)) : 0;
 }
 
 // Exchange tile of one line: rows skewed by row / R0, or for the 4 x 4 x ..
@@ -1051,8 +1054,9 @@ __global__ void __launch_bounds__(XReg<T, N>::NT, XReg<T, N>::minb)
     }
   }
   {
-    up = balance<P, H>(xw, xo);
-    down = T(1) / up;   // a power of two
+    const int d = balance<P, H>(xw, xo);
+    up = ldexp(T(1), d);
+    down = ldexp(T(1), -d);
 #pragma unroll
     for (int i = 0; i <= H; ++i) xo[i] = mkc<C>(xo[i].x * up, xo[i].y * up);
     V1 z[E];
@@ -1310,11 +1314,12 @@ __global__ void __launch_bounds__(XReg<T, N>::NT, XVjp<T, N>::minb)
     load(a.W, x5);   // on their way during the first transforms
     load(a.FZ, x6);
     inv2(x1, x2, x3, x4, u, v, fx, fy);
-    const T up = balance<P, H>(x5, x6);
+    const int d = balance<P, H>(x5, x6);
+    const T up = ldexp(T(1), d);
 #pragma unroll
     for (int i = 0; i <= H; ++i) x6[i] = mkc<C>(x6[i].x * up, x6[i].y * up);
     inv1(x5, x6, w, fz);
-    const T down = T(1) / up;   // a power of two
+    const T down = ldexp(T(1), -d);
 #pragma unroll
     for (int i = 0; i < E; ++i) fz[i] *= down;
   }
@@ -1370,7 +1375,6 @@ template <int N> struct LPlan : VPlan<N> {};
     static constexpr int NST = sizeof(R) / sizeof(int);                                                              \
     __host__ __device__ static constexpr int ns(int s) { int q = 1; for (int i = 0; i < s; ++i) q *= R[i]; return q; } \
   };
-DNSBOX_LPLAN(512, 16, 16, 8, 4)
 DNSBOX_LPLAN(1024, 32, 16, 16, 4)
 #undef DNSBOX_LPLAN
 template <typename T, int N> struct XPlain {
@@ -1544,8 +1548,10 @@ inline double kcut2_of(double kcut) {
 // right-hand side's pass E): per mode the 2/3 mask, the pressure projection,
 // band or fixed forcing and the integrating-factor update, one warp per
 // (kz, ky) row of kx modes.  n3 holds the z-transformed nonlinear term.  Rows
-// run over the kept kz and ky indices (every row when not pruning) and cut kx
-// modes are skipped; the row's E and D sums (fixed lane order) go to
+// run over the kept kz and ky indices (every row when not pruning), by ky, last
+// ky first (the order in which pass E1 wrote them: the newest still in L2),
+// over the kept kx only (two rows per warp, the second in place of the next 32
+// columns, measured 64 against 57 us at 256^3 FP32); the row's E and D sums (fixed lane order) go to
 // partials[kz ny + ky] of the box, and the finalize reads the rows a pruned
 // launch does not visit as zero.  Each lane batches the global operands of
 // two modes before any store.  MODE (a FinishMode) is a template parameter so
