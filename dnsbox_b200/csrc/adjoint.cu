@@ -975,6 +975,15 @@ int ensure_orbit(dnsbox_ctx *c, size_t bytes) {
   return DNSBOX_OK;
 }
 
+// Advances the clock by n steps that were not taken.
+__global__ void k_skip_clock(StepState *st, int n) {
+  for (int i = 0; i < n; ++i) {
+    st->t_prev = st->t;
+    st->t += st->dt;
+    st->step += 1.0;
+  }
+}
+
 // g0 = (Phi^nsteps)'(u0)^T gT, checkpoints every `every` steps.  Also leaves
 // u(T) in *uT_out when non-null.  States advance with dnsbox_step, the
 // library's fused step.
@@ -987,11 +996,26 @@ int steps_vjp_impl(dnsbox_ctx *c, const void *u0, int nsteps, int every, const v
   char *cp = c->orbit, *seg = cp + (size_t)ncp * sb3, *ga = seg + (size_t)every * sb3, *gb = ga + sb3;
   double dt = 0.0;
   RET(dnsbox_get_dt(c, &dt));
-  // forward sweep: checkpoints
+  // forward sweep: checkpoints, and the last segment's states kept as they pass
+  // (the backward sweep starts with them); u(T) itself only where it is asked for
+  const int last0 = (ncp - 1) * every;
+  int skipped = 0;
   CK(cudaMemcpyAsync(seg, u0, sb3, cudaMemcpyDeviceToDevice, c->stream));
+  RET(step_advance_decided(c, seg, 0, true));   // pruning decided once for the trajectory
+  char *cur = seg;
   for (int n = 0; n < nsteps; ++n) {
-    if (n % every == 0) CK(cudaMemcpyAsync(cp + (size_t)(n / every) * sb3, seg, sb3, cudaMemcpyDeviceToDevice, c->stream));
-    RET(step_advance_decided(c, seg, 1, n == 0));   // pruning decided once for the trajectory
+    if (n % every == 0 && n != last0)
+      CK(cudaMemcpyAsync(cp + (size_t)(n / every) * sb3, cur, sb3, cudaMemcpyDeviceToDevice, c->stream));
+    if (n >= last0) {
+      char *next = n + 1 < nsteps ? seg + (size_t)(n + 1 - last0) * sb3 : reinterpret_cast<char *>(uT_out);
+      if (!next) {
+        ++skipped;
+        break;
+      }
+      CK(cudaMemcpyAsync(next, cur, sb3, cudaMemcpyDeviceToDevice, c->stream));
+      cur = next;
+    }
+    RET(step_advance_decided(c, cur, 1, false));
   }
   const bool pruned = c->prune_now;   // of every state of this trajectory
   if (pruned) {   // the pruned predictor leaves the cut set of u* as it is
@@ -999,13 +1023,13 @@ int steps_vjp_impl(dnsbox_ctx *c, const void *u0, int nsteps, int every, const v
     RET(ensure_adj(c, 9, 33, &P, &S));
     CK(cudaMemsetAsync(S + 24 * c->nh * sizeof(C), 0, sb3, c->stream));
   }
-  if (uT_out) CK(cudaMemcpyAsync(uT_out, seg, sb3, cudaMemcpyDeviceToDevice, c->stream));
   // backward sweep, one segment at a time
   CK(cudaMemcpyAsync(ga, gT, sb3, cudaMemcpyDeviceToDevice, c->stream));
   for (int k = ncp - 1; k >= 0; --k) {
     const int n0 = k * every, len = (nsteps - n0 < every) ? nsteps - n0 : every;
-    CK(cudaMemcpyAsync(seg, cp + (size_t)k * sb3, sb3, cudaMemcpyDeviceToDevice, c->stream));
-    for (int j = 1; j < len; ++j) {
+    if (k == ncp - 1) skipped += len - 1;
+    else CK(cudaMemcpyAsync(seg, cp + (size_t)k * sb3, sb3, cudaMemcpyDeviceToDevice, c->stream));
+    for (int j = 1; j < len && k != ncp - 1; ++j) {
       CK(cudaMemcpyAsync(seg + (size_t)j * sb3, seg + (size_t)(j - 1) * sb3, sb3, cudaMemcpyDeviceToDevice,
                          c->stream));
       RET(step_advance_decided(c, seg + (size_t)j * sb3, 1, false));
@@ -1018,6 +1042,10 @@ int steps_vjp_impl(dnsbox_ctx *c, const void *u0, int nsteps, int every, const v
     }
   }
   CK(cudaMemcpyAsync(g0, ga, sb3, cudaMemcpyDeviceToDevice, c->stream));
+  // the context's clock counts every step of the plain scheme, which recomputes the last segment too
+  k_skip_clock<<<1, 1, 0, c->stream>>>(c->st, skipped);
+  CK(cudaGetLastError());
+  c->host_step += skipped;
   RET(tc_check(c));
   return DNSBOX_OK;
 }
