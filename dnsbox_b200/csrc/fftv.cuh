@@ -305,6 +305,23 @@ DNSBOX_VPLAN(512, 16, 16, 8, 4)
 DNSBOX_VPLAN(1024, 16, 16, 16, 4)
 #undef DNSBOX_VPLAN
 
+// Two-stage plans N = R0 R1 with one butterfly a thread in each stage: R1
+// threads of R0 values, rows p + R1 q, then R0 threads of R1 values, rows p +
+// R0 q.  The x lines of 96 and 192 points, whose plans of equal shares need two
+// exchanges, run their inverse transforms this way and their forward ones the
+// other way round.
+template <int N> struct SplitPlan {
+  static constexpr bool on = false;
+};
+template <> struct SplitPlan<96> {
+  static constexpr bool on = true;
+  static constexpr int R0 = 12, R1 = 8, pitch = 108;
+};
+template <> struct SplitPlan<192> {
+  static constexpr bool on = true;
+  static constexpr int R0 = 12, R1 = 16, pitch = 220;
+};
+
 // Plans of the x lines, at most 32 threads per line (a warp synchronises
 // itself): 16 values in single precision, 8 in double precision (three
 // sequences of a line are held at once) where the length allows it.

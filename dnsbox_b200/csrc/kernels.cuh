@@ -966,12 +966,11 @@ template <typename T, int N> struct XReg {
 // Forward, px + i py and pz + i 0 (its transform is the half line itself).
 // A lane loads its rows up to N/2 and forms both that row's value and its
 // Hermitian mirror's, which goes to the lane that holds row N - n by shuffle.
-// Against the block kernel (fields in shared memory, 45% bank conflicts at 96)
-// and the warp kernels it replaces, us: 32 boxes of 96^3 FP32 625 -> 287, of
-// 64^3 152 -> 82, of 32^3 29 -> 19, 128^3 55 -> 27, 192^3 191 -> 78, 256^3 162 ->
-// 138 (FP64 397 -> 352), 512^3 1698 -> 1335.  At 256 in FP32 it is balanced:
-// issue 57%, FMA pipe 50%, L1 60%, 12 warps by registers; FP64 (78%) and 96
-// (87%) are bound by L1, the exchanges.  All loads of a line up front (the
+// Against the block kernel (fields in shared memory, bank conflicts) and the
+// warp kernels it replaces, us: 32 boxes of 64^3 FP32 152 -> 72, of 32^3 29 -> 18,
+// 128^3 55 -> 25, 256^3 162 -> 131 (FP64 397 -> 333), 512^3 1698 -> 1295.  At 256 in
+// FP32 it is balanced: issue 57%, FMA pipe 50%, L1 60%, 12 warps by registers;
+// FP64 is bound by L1 (78%), the exchanges.  All loads of a line up front (the
 // third sequence's during the pair's transform) brought 179 -> 140 at 256.
 template <typename T, int N>
 __global__ void __launch_bounds__(XReg<T, N>::NT, XReg<T, N>::minb)
@@ -1166,6 +1165,202 @@ __global__ void __launch_bounds__(XReg<T, N>::NT, XReg<T, N>::minb)
   }
 }
 
+// The fused x pass of 96- and 192-point lines: k_xline_nl_g with split plans
+// (SplitPlan), so that each transform exchanges once, not twice, through the
+// shared memory that bounds it.  A block of 8 lines: R1 lanes a line load,
+// form the sequences and run the inverse transforms' first stage; after one
+// barrier R0 lanes a line run the second stage, form the products and run the
+// forward transforms' first stage; R1 lanes a line finish and store.  The tile
+// rows are skewed by row / R of the stage that writes them (16-byte accesses
+// of every stage free of bank conflicts at the pitches of SplitPlan).  Against
+// k_xline_nl_g, us: 32 boxes of 96^3 FP32 285 -> 258 (L1 87% -> 65%, now bound by
+// load latency and the block's barriers), 192^3 FP32 78 -> 65, FP64 156 -> 148.
+template <typename T, int N> struct XSplit {
+  using SP = SplitPlan<N>;
+  static constexpr int L = 8, PO = SP::R1, PI = SP::R0, NT = L * (PO > PI ? PO : PI);
+  static constexpr int ntw = (SP::R1 - 1) * SP::R0 + (SP::R0 - 1) * SP::R1;
+  static constexpr size_t tw = ((size_t)ntw * 2 * sizeof(T) + 15) / 16 * 16;
+  static constexpr size_t buf = (size_t)L * SP::pitch * 16;   // a pair of sequences (FP32) or one (FP64)
+  static constexpr size_t smem = tw + (sizeof(T) == 4 ? buf + buf / 2 : 3 * buf);
+  // 96 FP32: 18 warps by 96 registers (some spills) 258 us, 15 by 128 270, 21 by
+  // 80 275 (32 boxes of 96^3); 192 FP32: 16 warps 65 us, 12 71 (192^3)
+  static constexpr int minb = sizeof(T) == 8 ? (N == 96 ? 3 : 2) : (N == 96 ? 6 : 4);
+};
+template <typename T, int N>
+__global__ void __launch_bounds__(XSplit<T, N>::NT, XSplit<T, N>::minb)
+    k_xline_nl_s(const __grid_constant__ XlineNLArgs<T> a) {
+  using C = typename CT<T>::type;
+  using SH = XSplit<T, N>;
+  using SP = SplitPlan<N>;
+  using V1 = VC<T>;
+  using VP = VC<typename VecOf<T>::R>;   // the pair (FP32); FP64 transforms its two sequences one by one
+  constexpr int R0 = SP::R0, R1 = SP::R1, H = R0 / 2, L = SH::L, PO = SH::PO, PI = SH::PI, NP = sizeof(T) == 4 ? 1 : 2;
+  constexpr bool PAIR = NP == 1;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int ex[L];
+  V1 *twi = reinterpret_cast<V1 *>(smem_raw), *twf = twi + (R1 - 1) * R0;
+  pdl_launch();
+  for (int i = threadIdx.x; i < (R1 - 1) * R0; i += SH::NT) twi[i] = VtwOf<V1>::of(__ldg(a.tw + (1 + i / R0) * (i % R0)));
+  for (int i = threadIdx.x; i < (R0 - 1) * R1; i += SH::NT) twf[i] = VtwOf<V1>::of(__ldg(a.tw + (1 + i / R1) * (i % R1)));
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const unsigned blk = gridDim.x - 1 - blockIdx.x;   // last lines first, as pass B left them in L2
+  const long long line0 = (long long)blk * L;
+  const bool outer = threadIdx.x < L * PO, inner = threadIdx.x < L * PI;   // whole warps
+  const int lo = threadIdx.x / PO, po = threadIdx.x % PO, li = threadIdx.x / PI, pi = threadIdx.x % PI;
+  const bool on = outer && line0 + lo < a.nlines;
+  const long long pin = a.pin ? a.pin : a.nxh, pout = a.pout ? a.pout : a.nxh;
+  const int mirror = (lane & ~(PO - 1)) | ((PO - po) & (PO - 1));
+  const int nyq = a.nyq ? a.nyq : N / 2;
+  auto bufp = [&](int k, int line) { return reinterpret_cast<VP *>(smem_raw + SH::tw + k * SH::buf) + line * SP::pitch; };
+  auto bufs = [&](int line) { return reinterpret_cast<V1 *>(smem_raw + SH::tw + NP * SH::buf) + line * SP::pitch; };
+  auto inv_at = [](int row) { return row + row / R0; };   // written p R0 + r
+  auto fwd_at = [](int row) { return row + row / R1; };   // written p R1 + r
+  unsigned own = 0;   // bit i: row po + PO i is read and written
+#pragma unroll
+  for (int i = 0; i <= H; ++i)
+    if (on && (i < H || po == 0) && xkeep(a.kxa, po + PO * i, N)) own |= 1u << i;
+  if (outer) {
+    auto load = [&](const C *f, C *x) {
+      const C *r = f + (line0 + lo) * pin;
+#pragma unroll
+      for (int i = 0; i <= H; ++i) x[i] = ld_on(r + (i == H ? nyq : po + PO * i), own >> i & 1);
+      if (po == 0) x[0].y = x[H].y = 0;   // a C2R drops these imaginary parts
+    };
+    C x1[H + 1], x2[H + 1], x3[H + 1], x4[H + 1], x5[H + 1], x6[H + 1];
+    load(a.U, x1);
+    load(a.V, x2);
+    load(a.OX, x3);
+    load(a.OY, x4);
+    load(a.W, x5);
+    load(a.OZ, x6);
+    if constexpr (PAIR) {
+      VP z[R0], y[R0];
+      T re[R0], im[R0];
+      pack_lines<R0>(x1, x2, po, mirror, [&](int q, T r, T i) { re[q] = r, im[q] = i; });
+      pack_lines<R0>(x3, x4, po, mirror, [&](int q, T r, T i) { z[q] = VP{mkf2(re[q], r), mkf2(im[q], i)}; });
+      vdft<R0, true>(z, y);
+#pragma unroll
+      for (int r = 0; r < R0; ++r) bufp(0, lo)[inv_at(po * R0 + r)] = y[r];
+    } else {
+      V1 z[R0], y[R0];
+      pack_lines<R0>(x1, x2, po, mirror, [&](int q, T r, T i) { z[q] = V1{r, i}; });
+      vdft<R0, true>(z, y);
+#pragma unroll
+      for (int r = 0; r < R0; ++r) reinterpret_cast<V1 *>(bufp(0, lo))[inv_at(po * R0 + r)] = y[r];
+      pack_lines<R0>(x3, x4, po, mirror, [&](int q, T r, T i) { z[q] = V1{r, i}; });
+      vdft<R0, true>(z, y);
+#pragma unroll
+      for (int r = 0; r < R0; ++r) reinterpret_cast<V1 *>(bufp(1, lo))[inv_at(po * R0 + r)] = y[r];
+    }
+    const int d = balance<PO, H>(x5, x6);
+    if (po == 0) ex[lo] = d;
+    const T up = ldexp(T(1), d);
+#pragma unroll
+    for (int i = 0; i <= H; ++i) x6[i] = mkc<C>(x6[i].x * up, x6[i].y * up);
+    V1 z[R0], y[R0];
+    pack_lines<R0>(x5, x6, po, mirror, [&](int q, T r, T i) { z[q] = V1{r, i}; });
+    vdft<R0, true>(z, y);
+#pragma unroll
+    for (int r = 0; r < R0; ++r) bufs(lo)[inv_at(po * R0 + r)] = y[r];
+  }
+  __syncthreads();
+  VP fy[NP][R1];   // first stage of the forward transforms
+  T m0 = 0, m1 = 0, m2 = 0;
+  if (inner) {
+    auto second = [&](auto *b, auto *x) {
+      using V = std::remove_pointer_t<decltype(b)>;
+      V v[R1];
+#pragma unroll
+      for (int r = 0; r < R1; ++r) v[r] = b[inv_at(pi + r * R0)];
+#pragma unroll
+      for (int r = 1; r < R1; ++r) v[r] = vtwmul<true>(v[r], twi[(r - 1) * R0 + pi]);
+      vdft<R1, true>(v, x);
+    };
+    VP x[NP][R1];
+    V1 w[R1];
+#pragma unroll
+    for (int k = 0; k < NP; ++k) second(bufp(k, li), x[k]);
+    second(bufs(li), w);
+    const T down = ldexp(T(1), -ex[li]), sc = T(a.s);
+    VP f[NP][R1];
+#pragma unroll
+    for (int q = 0; q < R1; ++q) {
+      T u, v, ox, oy;
+      if constexpr (PAIR) u = f2_lo(x[0][q].re), v = f2_lo(x[0][q].im), ox = f2_hi(x[0][q].re), oy = f2_hi(x[0][q].im);
+      else u = x[0][q].re, v = x[0][q].im, ox = x[1][q].re, oy = x[1][q].im;
+      const T ww = w[q].re, oz = w[q].im * down;
+      const T px = (oy * ww - oz * v) * sc, py = (oz * u - ox * ww) * sc, pz = (ox * v - oy * u) * sc;
+      m0 = fmax(m0, fabs(u));
+      m1 = fmax(m1, fabs(v));
+      m2 = fmax(m2, fabs(ww));
+      if constexpr (PAIR) f[0][q] = VP{mkf2(px, pz), mkf2(py, T(0))};
+      else f[0][q] = VP{px, py}, f[1][q] = VP{pz, T(0)};
+    }
+#pragma unroll
+    for (int k = 0; k < NP; ++k) vdft<R1, false>(f[k], fy[k]);
+  }
+  __syncthreads();   // the inverse transforms' tiles are free
+  if (inner) {
+#pragma unroll
+    for (int k = 0; k < NP; ++k)
+#pragma unroll
+      for (int r = 0; r < R1; ++r) bufp(k, li)[fwd_at(pi * R1 + r)] = fy[k][r];
+  }
+  __syncthreads();
+  if (outer) {
+    VP x[NP][R0];
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+      VP v[R0];
+#pragma unroll
+      for (int r = 0; r < R0; ++r) v[r] = bufp(k, lo)[fwd_at(po + r * R1)];
+#pragma unroll
+      for (int r = 1; r < R0; ++r) v[r] = vtwmul<false>(v[r], twf[(r - 1) * R1 + po]);
+      vdft<R0, false>(v, x[k]);
+    }
+    // rows k = po + PO i <= N/2 of the half lines (as k_xline_nl_g)
+    C *const dx = a.NX + (line0 + lo) * pout, *const dy = a.NY + (line0 + lo) * pout, *const dz = a.NZ + (line0 + lo) * pout;
+    auto re = [&](int k, int i) {
+      if constexpr (PAIR) return k == 0 ? f2_lo(x[0][i].re) : f2_hi(x[0][i].re);
+      else return x[k][i].re;
+    };
+    auto im = [&](int k, int i) {
+      if constexpr (PAIR) return k == 0 ? f2_lo(x[0][i].im) : f2_hi(x[0][i].im);
+      else return x[k][i].im;
+    };
+#pragma unroll
+    for (int i = 0; i <= H; ++i) {
+      const T zr = re(0, i), zi = im(0, i);
+      T nr = zr, ni = zi;   // i = H: row N/2, its own mirror
+      if (i < H) {
+        nr = __shfl_sync(0xffffffffu, po == 0 ? re(0, (R0 - i) % R0) : re(0, R0 - 1 - i), mirror);
+        ni = __shfl_sync(0xffffffffu, po == 0 ? im(0, (R0 - i) % R0) : im(0, R0 - 1 - i), mirror);
+      }
+      if (own >> i & 1) {
+        const int sl = i == H ? nyq : po + PO * i;
+        dx[sl] = mkc<C>(T(0.5) * (zr + nr), T(0.5) * (zi - ni));
+        dy[sl] = mkc<C>(T(0.5) * (zi + ni), T(0.5) * (nr - zr));
+        dz[sl] = mkc<C>(re(1, i), im(1, i));
+      }
+    }
+    if (on)
+      for (int j = po; j < a.npad; j += PO) dx[nyq + 1 + j] = dy[nyq + 1 + j] = dz[nyq + 1 + j] = mkc<C>(0, 0);
+  }
+  if (!a.st || !inner) return;
+  // CFL maxima (a box has a multiple of 16 lines, so the block's lines share one)
+  m0 = warp_max(m0);
+  m1 = warp_max(m1);
+  m2 = warp_max(m2);
+  if (lane == 0) {
+    double *um = a.st[line0 / a.lines_per_box].umax;
+    const double m[3] = {(double)m0 * a.s, (double)m1 * a.s, (double)m2 * a.s};
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      if (!(m[c] <= __ldcg(um + c))) atomic_max_nonneg(um + c, m[c]);
+  }
+}
+
 // ----------------------------------------------- fused x pass of the transposed term
 template <typename T> struct XlineVjpArgs {
   using C = typename CT<T>::type;
@@ -1185,7 +1380,7 @@ template <typename T, int N> struct XVjp {
 // holds two vectors at a time: U + iV and FX + i FY (a pair in FP32), W +
 // i 2^e FZ, then u x phi forward, then OX + i OY with OZ (+ i 0), phi x omega
 // forward.  It replaces nine C2R and six R2C lines of global memory traffic and
-// a pointwise kernel: the transposed term at 96^3 FP32 goes from 45 to 24 us in x.
+// a pointwise kernel: at 96^3 FP32 one kernel of 24 us where four took 58.
 template <typename T, int N>
 __global__ void __launch_bounds__(XReg<T, N>::NT, XVjp<T, N>::minb)
     k_xline_vjp(const __grid_constant__ XlineVjpArgs<T> a) {

@@ -168,7 +168,18 @@ template <typename T, int N>
 cudaError_t Launcher<T, N>::xline_nl(const XlineNLArgs<T> &a, int variant, cudaStream_t st) {
   using C = typename CT<T>::type;
   cudaError_t e;
-  if constexpr (XReg<T, N>::on) {   // the only kernel for these lines, whatever the choice
+  if constexpr (SplitPlan<N>::on) {
+    // from two waves of blocks on: 32 boxes of 96^3 285 -> 258 us, 192^3 78 -> 65;
+    // with fewer lines its barriers cost more than they save (a 192 x 48 x 96
+    // step, 4608 lines, 92 -> 94 us, the 96^3 horizon gradient 5.66 -> 5.73 ms)
+    using SH = XSplit<T, N>;
+    const int blocks = (a.nlines + SH::L - 1) / SH::L;
+    if (blocks >= 2 * 148 * SH::minb) {
+      if ((e = set_smem(k_xline_nl_s<T, N>, SH::smem)) != cudaSuccess) return e;
+      return launch_pdl(k_xline_nl_s<T, N>, (unsigned)blocks, SH::NT, SH::smem, st, a);
+    }
+  }
+  if constexpr (XReg<T, N>::on) {   // whatever the choice
     using SH = XReg<T, N>;
     // few lines: smaller blocks, so that every SM gets some
     int nt = SH::NT;

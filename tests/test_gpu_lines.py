@@ -75,3 +75,28 @@ def test_transposed_term_line_length(nx, prec):
     # a chain of transforms for u and one for g: twice the bar of a right-hand side
     assert rel(got.cpu().numpy(), O.rhs_nonlinear_vjp(g, uh, gr)) < 2 * TOL[prec]
     b.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("nx,nbatch", [(96, 40), (192, 20)])
+def test_x_kernel_of_many_lines(nx, nbatch, prec):
+    """Boxes enough for the split x kernel (two waves of its blocks) against the same boxes one by one (the other one)."""
+    from dnsbox_b200.ops import Box
+    ny, nz = 12, 48
+    kw = dict(nx=nx, ny=ny, nz=nz, precision=prec, nu=2e-3, bandlim=False, tstep_fix=True, dt=1e-3)
+    g = O.Grid(O.Params(nx=nx, ny=ny, nz=nz, bandlim=False))
+    fields = [rough(g, nx, ny, nz, seed=s) * (s + 1) for s in range(3)]
+    batch = Box(nbatch=nbatch, **kw)
+    u = batch.zeros()
+    for i in range(nbatch):
+        u[:, i] = torch.from_numpy(fields[i % 3]).to(u.device, u.dtype)
+    recs = batch.step(u, 1)[0]
+    for i in range(3):
+        one = Box(**kw)
+        v = one.from_numpy(fields[i])
+        r = one.step(v, 1)[0]
+        for j in range(i, nbatch, 3):
+            assert rel(u[:, j].cpu().numpy(), v.cpu().numpy()) < 2 * TOL[prec]   # two right-hand sides
+            assert np.allclose(recs[j]["umax"], r["umax"], rtol=TOL[prec], atol=0)
+        one.close()
+    batch.close()
