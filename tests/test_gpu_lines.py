@@ -100,3 +100,42 @@ def test_x_kernel_of_many_lines(nx, nbatch, prec):
             assert np.allclose(recs[j]["umax"], r["umax"], rtol=TOL[prec], atol=0)
         one.close()
     batch.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("nx", SIZES[:-1])
+def test_vanishing_component(nx, prec):
+    """A mean flow with w(x, y): the z vorticity is exactly zero where w is not, and (transposed) a cotangent without z
+    part; each shares a complex sequence of the x kernels with a nonzero field and must stay zero."""
+    from dnsbox_b200.ops import Box
+    ny, nz = 12, 8
+    g = O.Grid(O.Params(nx=nx, ny=ny, nz=nz, bandlim=False))
+    rng = np.random.default_rng(nx)
+    w = np.broadcast_to(rng.standard_normal((1, ny, nx)), (nz, ny, nx))
+    u = O.state_dealias(g, O.state_u2uhat(g, np.stack([np.zeros_like(w), np.zeros_like(w), w])))
+    u[:2, 0, 0, 0] = nx * ny * nz * np.array([0.7, -1.3])   # the mean flow, kept by every mask but dealias's
+    b = Box(nx=nx, ny=ny, nz=nz, precision=prec, bandlim=False)
+    ub = b.from_numpy(u)
+    got, _ = b.rhs_nonlinear(ub)
+    assert rel(got.cpu().numpy(), O.rhs_nonlinear(g, u)) < TOL[prec]
+    z = b.zeros()
+    assert not b.rhs_nonlinear_vjp(ub, z).abs().max().item()   # a zero cotangent: exactly zero
+    c = u.copy()
+    c[2] = 0
+    c[0] = O.state_dealias(g, O.state_u2uhat(g, np.stack([np.roll(w, 3, 1)] * 3)))[0]
+    assert rel(b.rhs_nonlinear_vjp(ub, b.from_numpy(c)).cpu().numpy(), O.rhs_nonlinear_vjp(g, u, c)) < 2 * TOL[prec]
+    b.close()
+
+
+@pytest.mark.parametrize("n", [8, 12, 24, 32])
+def test_band_energy_in_pass_a(n):
+    """The band energy of a box whose pass-A block has fewer threads than a warp (n = 8, 12, 24)."""
+    from dnsbox_b200.ops import Box
+    kw = dict(nu=2e-3, kCutOff=2.5, Pin=0.1, bandlim=True)
+    g = O.Grid(O.Params(nx=24, ny=16, nz=n, **kw))
+    uh = rough(g, 24, 16, n, seed=n)
+    b = Box(nx=24, ny=16, nz=n, tstep_fix=True, dt=1e-3, **kw)
+    u = b.from_numpy(uh)
+    assert abs(b.rhs_nonlinear(u)[1] / O.rhs_eband(g, uh) - 1) < 1e-13
+    assert abs(b.step(u, 1)[0]["eband"] / O.rhs_eband(g, uh) - 1) < 1e-13
+    b.close()
