@@ -662,7 +662,6 @@ static int run_rhs(dnsbox_ctx *c, const void *uin, int mode, void *out, void *st
     x.nyq = c->keep[0].a;
     x.npad = a.nslot - x.nyq - 1;
   }
-  x.status = c->tc_status;
   x.tw = reinterpret_cast<const C *>(c->tw[0]);
   x.st = cfl ? c->st : nullptr;   // the CFL maxima, where they are used
   x.lines_per_box = p.ny * p.nz;
@@ -904,7 +903,7 @@ int tc_check(dnsbox_ctx *c) {
   }
   int *flag = reinterpret_cast<int *>(c->hstage + 63);
   *flag = 0;
-  if (c->tc_status) CK(cudaMemcpyAsync(flag, c->tc_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(flag, c->tc_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   if (*flag) {
     CK(cudaMemsetAsync(c->tc_status, 0, sizeof(int), c->stream));
@@ -1229,9 +1228,6 @@ extern "C" int dnsbox_create(const dnsbox_params *p, dnsbox_ctx **out) {
   if (p->precision == DNSBOX_TC_SPLIT) {
     c->tc = 1;
     if ((rc = alloc_dft64(c))) return fail(rc);
-  } else {   // the status flag of bounded device waits (the staged x pass)
-    if ((e = cudaMalloc(&c->tc_status, sizeof(int))) != cudaSuccess || (e = cudaMemset(c->tc_status, 0, sizeof(int))) != cudaSuccess)
-      return fail(set_err(DNSBOX_ERR_OOM, "device allocation failed: %s", cudaGetErrorString(e)));
   }
   // pruning rule per axis, derived from the dealiasing mask and checked against it
   {

@@ -27,17 +27,6 @@ template <int N> struct FftPlan;
     static constexpr int NST = sizeof(R) / sizeof(int);                        \
     __host__ __device__ static constexpr int ns(int s) { int p = 1; for (int i = 0; i < s; ++i) p *= R[i]; return p; } \
   };
-DNSBOX_PLAN(8, 8, 8)
-DNSBOX_PLAN(12, 12, 4, 3)
-DNSBOX_PLAN(16, 16, 16)
-DNSBOX_PLAN(24, 24, 8, 3)
-DNSBOX_PLAN(32, 8, 8, 4)
-DNSBOX_PLAN(48, 12, 4, 4, 3)
-DNSBOX_PLAN(64, 8, 8, 8)
-DNSBOX_PLAN(96, 12, 4, 4, 2, 3)
-DNSBOX_PLAN(128, 16, 16, 8)
-DNSBOX_PLAN(192, 24, 8, 8, 3)
-DNSBOX_PLAN(256, 16, 16, 16)
 DNSBOX_PLAN(512, 8, 8, 8, 8)
 DNSBOX_PLAN(1024, 16, 16, 16, 4)
 #undef DNSBOX_PLAN
@@ -86,17 +75,6 @@ template <typename C, bool INV> __device__ __forceinline__ void dft4(C &a0, C &a
   a2 = csub(t0, t2);
   a1 = cadd(t1, t3);
   a3 = csub(t1, t3);
-}
-
-template <typename C, bool INV> __device__ __forceinline__ void dft3(C &a0, C &a1, C &a2) {
-  using R = decltype(C{}.x);
-  const R h = R(0.86602540378443864676372317075294);  // sqrt(3)/2
-  C t = cadd(a1, a2), d = csub(a1, a2);
-  C m = mkc<C>(a0.x - R(0.5) * t.x, a0.y - R(0.5) * t.y);
-  a0 = cadd(a0, t);
-  C q = mul_i<INV>(cscale(d, h));  // forward: -i h d
-  a1 = cadd(m, q);
-  a2 = csub(m, q);
 }
 
 // multiply by exp(-+ 2 pi i k / 8)
@@ -170,26 +148,15 @@ template <typename C, bool INV> __device__ __forceinline__ void dft16(C *v) {
 
 template <int R, typename C, bool INV> __device__ __forceinline__ void dft(C *v) {
   if constexpr (R == 2) dft2<C, INV>(v[0], v[1]);
-  else if constexpr (R == 3) dft3<C, INV>(v[0], v[1], v[2]);
   else if constexpr (R == 4) dft4<C, INV>(v[0], v[1], v[2], v[3]);
   else if constexpr (R == 8) dft8<C, INV>(v);
   else if constexpr (R == 16) dft16<C, INV>(v);
   else static_assert(R == 2, "unsupported radix");
 }
 
-// ----------------------------------------------------------- twiddle sources
-// W_N^(r j TS) of stage S of plan PL (r in [1, R), j in [0, NS)).  TwGlobal
-// reads the N-point table exp(-2 pi i k / N) through the read-only cache;
-// TwShared reads per-stage [r - 1][j] tables in shared memory, so that the
-// lanes of a warp with consecutive j read consecutive words (one shared
-// wavefront instead of a scatter of L1 sectors), filled by tw_fill.
-template <class PL, int S> __host__ __device__ constexpr int tw_off() {
-  int o = 0;
-  for (int t = 1; t < S; ++t) o += (PL::R[t] - 1) * PL::ns(t);
-  return o;
-}
-template <class PL> __host__ __device__ constexpr int tw_size() { return tw_off<PL, PL::NST>(); }
-
+// ----------------------------------------------------------- twiddles
+// W_N^(r j TS) of stage S of plan PL (r in [1, R), j in [0, NS)), from the
+// N-point table exp(-2 pi i k / N) through the read-only cache.
 template <typename C> struct TwGlobal {
   const C *__restrict__ tw;
   template <class PL, int S> __device__ __forceinline__ C get(int r, int j) const {
@@ -197,25 +164,6 @@ template <typename C> struct TwGlobal {
     return __ldg(&tw[r * j * TS]);
   }
 };
-template <typename C> struct TwShared {
-  const C *t;
-  template <class PL, int S> __device__ __forceinline__ C get(int r, int j) const {
-    return t[tw_off<PL, S>() + (r - 1) * PL::ns(S) + j];
-  }
-};
-// Fills the shared tables of plan PL from the global N-point table (all
-// threads of the block take part; the caller synchronises afterwards).
-template <typename C, class PL, int S = 1>
-__device__ __forceinline__ void tw_fill(C *t, const C *__restrict__ tw, int tid, int nthreads) {
-  if constexpr (S < PL::NST) {
-    constexpr int NS = PL::ns(S), R = PL::R[S], TS = PL::N / (NS * R);
-    for (int i = tid; i < (R - 1) * NS; i += nthreads) {
-      const int r = 1 + i / NS, j = i % NS;
-      t[tw_off<PL, S>() + i] = tw[r * j * TS];
-    }
-    tw_fill<C, PL, S + 1>(t, tw, tid, nthreads);
-  }
-}
 
 // ----------------------------------------------------------------- stages
 // One Stockham stage on column `col` of the tile; p in [0, N/E).  All threads
@@ -258,20 +206,6 @@ __device__ __forceinline__ void fft_stage_p(C *s, int LD, int col, int p, bool a
     }
   }
   fft_sync<WARP>();
-}
-
-template <typename C, int N, int S, bool INV>
-__device__ __forceinline__ void fft_stage(C *s, int LD, int col, int p, bool active, const C *__restrict__ tw) {
-  fft_stage_p<C, FftPlan<N>, S, INV, false>(s, LD, col, p, active, TwGlobal<C>{tw});
-}
-
-template <typename C, int N, bool INV, int S = 0>
-__device__ __forceinline__ void fft_columns(C *s, int LD, int col, int p, bool active,
-                                            const C *__restrict__ tw) {
-  if constexpr (S < FftPlan<N>::NST) {
-    fft_stage<C, N, S, INV>(s, LD, col, p, active, tw);
-    fft_columns<C, N, INV, S + 1>(s, LD, col, p, active, tw);
-  }
 }
 
 // ------------------------------------------------- register-resident ends

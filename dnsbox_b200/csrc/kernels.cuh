@@ -9,7 +9,7 @@
 //             curl into the inverse transforms;
 //   x       : k_xline_*  -- whole lines along x, two real lines per complex FFT.
 // The nonlinear term fuses the last inverse x pass, the u x omega product, the
-// max|u_i| (CFL) reduction and the first forward x pass (k_xline_nl); after
+// max|u_i| (CFL) reduction and the first forward x pass (k_xline_nl_g, ..); after
 // the last forward z pass (k_strided, in place) one streaming kernel applies
 // dealiasing, pressure projection, band forcing, the integrating-factor
 // stepper and the energy/dissipation row sums (k_finish_rows).
@@ -511,7 +511,6 @@ template <typename T> struct XlineNLArgs {
   int pin, pout;                       // row pitch (complex elements) of the inputs / outputs; 0: nxh
   int npad;                            // compact rows: slots after nyq that complete its 32-byte sector (written as 0)
   int nyq;                             // slot of the Nyquist column in a row (kxa in compact workspace rows); 0: N/2
-  int *status;                         // set to 1 when a bounded wait of a staged kernel gives up (or null)
   double alpha_x;
   double s;                            // scalemodes
 };
