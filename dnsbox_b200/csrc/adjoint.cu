@@ -466,8 +466,10 @@ int sum_to_host(dnsbox_ctx *c, int nblk, double *out) {
 
 // The transposed term from hw = h / W (spectral): C2R of u, omega and phi, the
 // cross products and their R2C, and the combination in `mode`.  The fields run
-// through the padded workspace (W1, W2 and the six slots of wphi); lines that
-// the fused x kernel does not take go through physical fields.
+// through the padded workspace: W1, W2 and six slots more, which lie in the
+// arena's nine physical fields where those are large enough (a new context's
+// first gradient at 64^3 takes one allocation of some 250 us less); lines that the
+// fused x kernel does not take go through physical fields.
 template <typename T>
 int vjp_core(dnsbox_ctx *c, const void *uh, const char *hw, int mode, CombineArgs<typename CT<T>::type> cb) {
   using C = typename CT<T>::type;
@@ -478,14 +480,18 @@ int vjp_core(dnsbox_ctx *c, const void *uh, const char *hw, int mode, CombineArg
   const char *u = reinterpret_cast<const char *>(uh);
   auto wf = [&](char *base, int slot) { return wfield(base, c, slot); };
   if (Ops<T>::has_xline_vjp(p.nx)) {
-    if (!c->wphi) CK(cudaMalloc(&c->wphi, 6 * c->wstride * c->cbytes));
+    char *wphi = c->adj;   // hw lies behind the nine fields
+    if (6 * c->wstride * c->cbytes > 9 * pb) {
+      if (!c->wphi) CK(cudaMalloc(&c->wphi, 6 * c->wstride * c->cbytes));
+      wphi = c->wphi;
+    }
     // inverse z: u (scaled), -dz v, dz u, phi
     StridedArgs<T> a = strided_base<T>(c, 2);
     strided_ws<T>(c, a, 2, false, true);
     a.njobs = 8;
     for (int f = 0; f < 3; ++f) {
       set_job<T>(a, f, u + f * sb, wf(c->W1, f), s);
-      set_job<T>(a, 5 + f, hw + f * sb, wf(c->wphi, f));
+      set_job<T>(a, 5 + f, hw + f * sb, wf(wphi, f));
     }
     set_job<T>(a, 3, u + sb, wf(c->W1, 3), 0.0, -s, 1);
     set_job<T>(a, 4, u, wf(c->W1, 4), 0.0, s, 1);
@@ -496,7 +502,7 @@ int vjp_core(dnsbox_ctx *c, const void *uh, const char *hw, int mode, CombineArg
     b.njobs = 9;
     for (int f = 0; f < 3; ++f) {
       set_job<T>(b, f, wf(c->W1, f), wf(c->W2, f));
-      set_job<T>(b, 6 + f, wf(c->wphi, f), wf(c->wphi, 3 + f));
+      set_job<T>(b, 6 + f, wf(wphi, f), wf(wphi, 3 + f));
     }
     set_job<T>(b, 3, wf(c->W1, 2), wf(c->W2, 3), 0.0, 1.0, 1, wf(c->W1, 3));
     set_job<T>(b, 4, wf(c->W1, 4), wf(c->W2, 4), 1.0, 0.0, 0, wf(c->W1, 2), 0.0, -1.0, 0);
@@ -505,7 +511,7 @@ int vjp_core(dnsbox_ctx *c, const void *uh, const char *hw, int mode, CombineArg
     XlineVjpArgs<T> x;
     memset(&x, 0, sizeof(x));
     const C **in[9] = {&x.U, &x.V, &x.W, &x.OX, &x.OY, &x.OZ, &x.FX, &x.FY, &x.FZ};
-    for (int f = 0; f < 9; ++f) *in[f] = reinterpret_cast<const C *>(f < 6 ? wf(c->W2, f) : wf(c->wphi, f - 3));
+    for (int f = 0; f < 9; ++f) *in[f] = reinterpret_cast<const C *>(f < 6 ? wf(c->W2, f) : wf(wphi, f - 3));
     for (int f = 0; f < 3; ++f) {
       x.A[f] = reinterpret_cast<C *>(wf(c->W1, f));
       x.B[f] = reinterpret_cast<C *>(wf(c->W1, 3 + f));

@@ -112,7 +112,7 @@ struct dnsbox_ctx {
   int sched_x = 0;
   char *adj = nullptr;                   // adjoint arena
   size_t adj_bytes = 0;
-  char *wphi = nullptr;                  // transposed term: 6 workspace slots beside W1 and W2 (on first use)
+  char *wphi = nullptr;                  // transposed term: its 6 workspace slots where the arena's fields are too small (on first use)
   cudaEvent_t read_ev = nullptr;         // a read-back that later work does not delay (on first use)
   char *orbit = nullptr;                 // checkpoints and segment states of the step-transpose chain
   size_t orbit_bytes = 0;
