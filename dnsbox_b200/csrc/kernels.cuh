@@ -981,10 +981,10 @@ template <typename T, int N> struct XReg {
 // A lane loads its rows up to N/2 and forms both that row's value and its
 // Hermitian mirror's, which goes to the lane that holds row N - n by shuffle.
 // Against the block kernel (fields in shared memory, bank conflicts) and the
-// warp kernels it replaces, us: 32 boxes of 64^3 FP32 152 -> 72, of 32^3 29 -> 18,
-// 128^3 55 -> 25, 256^3 162 -> 131 (FP64 397 -> 333), 512^3 1698 -> 1295.  At 256 in
-// FP32 it is balanced: issue 57%, FMA pipe 50%, L1 60%, 12 warps by registers;
-// FP64 is bound by L1 (78%), the exchanges.  All loads of a line up front (the
+// warp kernels it replaces, us: 32 boxes of 64^3 FP32 150 -> 73, of 32^3 29 -> 17,
+// 128^3 56 -> 25, 256^3 162 -> 130 (FP64 397 -> 325), 512^3 1698 -> 1285.  At 256 in
+// FP32 it is balanced: issue 57-60%, FMA pipe 50%, L1 61-65%, 12 warps by registers;
+// FP64 is bound by L1 (82-87%), the exchanges.  All loads of a line up front (the
 // third sequence's during the pair's transform) brought 179 -> 140 at 256.
 template <typename T, int N>
 __global__ void __launch_bounds__(XReg<T, N>::NT, XReg<T, N>::minb)
@@ -1187,8 +1187,8 @@ __global__ void __launch_bounds__(XReg<T, N>::NT, XReg<T, N>::minb)
 // forward transforms' first stage; R1 lanes a line finish and store.  The tile
 // rows are skewed by row / R of the stage that writes them (16-byte accesses
 // of every stage free of bank conflicts at the pitches of SplitPlan).  Against
-// k_xline_nl_g, us: 32 boxes of 96^3 FP32 285 -> 258 (L1 87% -> 65%, now bound by
-// load latency and the block's barriers), 192^3 FP32 78 -> 65, FP64 156 -> 148.
+// k_xline_nl_g, us: 32 boxes of 96^3 FP32 285 -> 250 (L1 87% -> 67-75%, now bound by
+// load latency and the block's barriers), 192^3 FP32 78 -> 64, FP64 156 -> 144.
 template <typename T, int N> struct XSplit {
   using SP = SplitPlan<N>;
   static constexpr int L = 8, PO = SP::R1, PI = SP::R0, NT = L * (PO > PI ? PO : PI);

@@ -169,7 +169,7 @@ cudaError_t Launcher<T, N>::xline_nl(const XlineNLArgs<T> &a, int variant, cudaS
   using C = typename CT<T>::type;
   cudaError_t e;
   if constexpr (SplitPlan<N>::on) {
-    // from two waves of blocks on: 32 boxes of 96^3 285 -> 258 us, 192^3 78 -> 65;
+    // from two waves of blocks on: 32 boxes of 96^3 285 -> 250 us, 192^3 78 -> 64;
     // with fewer lines its barriers cost more than they save (a 192 x 48 x 96
     // step, 4608 lines, 92 -> 94 us, the 96^3 horizon gradient 5.66 -> 5.73 ms)
     using SH = XSplit<T, N>;

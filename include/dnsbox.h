@@ -377,7 +377,7 @@ int dnsbox_ensemble_destroy(dnsbox_ensemble *ens);
  * p3dfft / FFTW (variables.f90:154).  The schedule picks, per tensor-core
  * strided pass of the right-hand side of the tensor-core form, the TMA-staged
  * or the cp.async-fed tensor-core kernel or the FP32 SIMT kernel, and for the
- * fused x pass the block or the warp kernel. */
+ * fused x pass of FP64 lines of 512 points the block or the warp kernel. */
 typedef struct dnsbox_schedule {
   int32_t tc_kernel[4];   /* passes A (inverse z), B (inverse y), D (forward y): 0 TMA-staged tensor-core
                              kernel, 1 cp.async-fed one (the default), 2 FP32 SIMT kernel; [3] pass E1
