@@ -139,3 +139,26 @@ def test_band_energy_in_pass_a(n):
     assert abs(b.rhs_nonlinear(u)[1] / O.rhs_eband(g, uh) - 1) < 1e-13
     assert abs(b.step(u, 1)[0]["eband"] / O.rhs_eband(g, uh) - 1) < 1e-13
     b.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("nx", [12, 96, 256, 512])
+def test_cut_check_single_mode(nx, prec):
+    """One mode at the edges of the kept set decides whether a step prunes: rows of several rounds of the check and
+    of a part of one, every component, a value that is not a number."""
+    from dnsbox_b200.ops import Box
+    ny, nz = 12, 16
+    ax, ay, az, nyq = -(-nx // 3), -(-ny // 3), -(-nz // 3), nx // 2   # kept: i < a, n/2, i > n - a
+    b = Box(nx=nx, ny=ny, nz=nz, precision=prec, bandlim=False, tstep_fix=True, dt=1e-3)
+    kept = [(2, 0, 0, ax - 1), (0, 0, 0, nyq), (1, nz - az + 1, ny // 2, nyq), (2, az - 1, ay - 1, 0)]
+    cut = [(0, 0, 0, ax), (2, 0, 0, nyq - 1), (1, az, 0, 0), (2, nz - az, ny // 2, nyq), (0, 0, ny - ay, 0)]
+    for at in kept + cut:
+        u = b.zeros()
+        u[at] = 1e-30 if at in cut else 1.0
+        b.step(u, 1, diag=False)
+        assert b.step_pruned() == (at in kept), at
+    u = b.zeros()
+    u[2, 0, 0, nyq - 1] = float("nan")
+    b.step(u, 1, diag=False)
+    assert not b.step_pruned()
+    b.close()
