@@ -981,12 +981,29 @@ int ensure_orbit(dnsbox_ctx *c, size_t bytes) {
   return DNSBOX_OK;
 }
 
-// Advances the clock by n steps that were not taken.
-__global__ void k_skip_clock(StepState *st, int n) {
-  for (int i = 0; i < n; ++i) {
-    st->t_prev = st->t;
-    st->t += st->dt;
-    st->step += 1.0;
+// Advances the clock by n steps (n < 1024) that were not taken because they
+// repeat steps taken `back` steps earlier, and writes their records: those
+// steps' with the clock's own t and step.  One block, a thread per record; the
+// ring holds all `back` records, and every one is read before any is written.
+__global__ void k_repeat_records(StepState *st, dnsbox_diag *ring, int cap, int back, int n) {
+  const int j = threadIdx.x;
+  const long long step = (long long)st->step + j;
+  double t = st->t;
+  const double dt = st->dt;
+  dnsbox_diag r;
+  if (j < n) {
+    r = ring[(step - back) % cap];
+    for (int i = 0; i < j; ++i) t += dt;
+    r.t = t + dt;
+    r.step = (int)step + 1;
+  }
+  __syncthreads();
+  if (j >= n) return;
+  ring[step % cap] = r;
+  if (j == n - 1) {
+    st->t_prev = t;
+    st->t = r.t;
+    st->step = (double)(step + 1);
   }
 }
 
@@ -1002,26 +1019,31 @@ int steps_vjp_impl(dnsbox_ctx *c, const void *u0, int nsteps, int every, const v
   char *cp = c->orbit, *seg = cp + (size_t)ncp * sb3, *ga = seg + (size_t)every * sb3, *gb = ga + sb3;
   double dt = 0.0;
   RET(dnsbox_get_dt(c, &dt));
-  // forward sweep: checkpoints, and the last segment's states kept as they pass
-  // (the backward sweep starts with them); u(T) itself only where it is asked for
-  const int last0 = (ncp - 1) * every;
-  int skipped = 0;
+  // The plain scheme steps to u(T) and recomputes every segment's states from its
+  // checkpoint, the last segment first.  That segment's states are the ones the
+  // forward sweep has just passed: they are kept, and of its recomputation only
+  // the records and the clock are carried out (where the ring still holds the
+  // records of the whole segment).
+  const int last0 = (ncp - 1) * every, last_len = nsteps - last0;
+  const bool keep = last_len <= c->ring_cap;
   CK(cudaMemcpyAsync(seg, u0, sb3, cudaMemcpyDeviceToDevice, c->stream));
   RET(step_advance_decided(c, seg, 0, true));   // pruning decided once for the trajectory
   char *cur = seg;
   for (int n = 0; n < nsteps; ++n) {
-    if (n % every == 0 && n != last0)
+    if (n % every == 0 && !(keep && n == last0))
       CK(cudaMemcpyAsync(cp + (size_t)(n / every) * sb3, cur, sb3, cudaMemcpyDeviceToDevice, c->stream));
-    if (n >= last0) {
-      char *next = n + 1 < nsteps ? seg + (size_t)(n + 1 - last0) * sb3 : reinterpret_cast<char *>(uT_out);
-      if (!next) {
-        ++skipped;
-        break;
-      }
+    if (keep && n >= last0) {
+      char *next = n + 1 < nsteps ? seg + (size_t)(n + 1 - last0) * sb3 : gb;
       CK(cudaMemcpyAsync(next, cur, sb3, cudaMemcpyDeviceToDevice, c->stream));
       cur = next;
     }
     RET(step_advance_decided(c, cur, 1, false));
+  }
+  if (uT_out) CK(cudaMemcpyAsync(uT_out, cur, sb3, cudaMemcpyDeviceToDevice, c->stream));
+  if (keep && last_len > 1) {
+    k_repeat_records<<<1, last_len - 1, 0, c->stream>>>(c->st, c->ddiag, c->ring_cap, last_len, last_len - 1);
+    CK(cudaGetLastError());
+    c->host_step += last_len - 1;
   }
   const bool pruned = c->prune_now;   // of every state of this trajectory
   if (pruned) {   // the pruned predictor leaves the cut set of u* as it is
@@ -1033,9 +1055,9 @@ int steps_vjp_impl(dnsbox_ctx *c, const void *u0, int nsteps, int every, const v
   CK(cudaMemcpyAsync(ga, gT, sb3, cudaMemcpyDeviceToDevice, c->stream));
   for (int k = ncp - 1; k >= 0; --k) {
     const int n0 = k * every, len = (nsteps - n0 < every) ? nsteps - n0 : every;
-    if (k == ncp - 1) skipped += len - 1;
-    else CK(cudaMemcpyAsync(seg, cp + (size_t)k * sb3, sb3, cudaMemcpyDeviceToDevice, c->stream));
-    for (int j = 1; j < len && k != ncp - 1; ++j) {
+    const bool kept = keep && k == ncp - 1;
+    if (!kept) CK(cudaMemcpyAsync(seg, cp + (size_t)k * sb3, sb3, cudaMemcpyDeviceToDevice, c->stream));
+    for (int j = 1; j < len && !kept; ++j) {
       CK(cudaMemcpyAsync(seg + (size_t)j * sb3, seg + (size_t)(j - 1) * sb3, sb3, cudaMemcpyDeviceToDevice,
                          c->stream));
       RET(step_advance_decided(c, seg + (size_t)j * sb3, 1, false));
@@ -1048,10 +1070,6 @@ int steps_vjp_impl(dnsbox_ctx *c, const void *u0, int nsteps, int every, const v
     }
   }
   CK(cudaMemcpyAsync(g0, ga, sb3, cudaMemcpyDeviceToDevice, c->stream));
-  // the context's clock counts every step of the plain scheme, which recomputes the last segment too
-  k_skip_clock<<<1, 1, 0, c->stream>>>(c->st, skipped);
-  CK(cudaGetLastError());
-  c->host_step += skipped;
   RET(tc_check(c));
   return DNSBOX_OK;
 }

@@ -149,3 +149,34 @@ def test_periodic_orbit_96():
         alpha *= 0.5
     print(f"periodic orbit 96^3 T=5: J {J:.6e} -> {Jt:.6e} (alpha {alpha:.3e})")
     assert Jt < J
+
+
+@pytest.mark.parametrize("want_uT", [False, True])
+@pytest.mark.parametrize("ns,every", [(16, 32), (16, 5), (9, 9), (1, 1), (7, 2), (1026, 1026)])
+def test_horizon_gradient_clock_and_records(ns, every, want_uT):
+    """The clock and the record ring after a horizon gradient are those of its plain scheme, whatever it keeps: the
+    steps forward, then every segment's recomputed from its checkpoint, the last segment first (1026: a segment longer
+    than the ring)."""
+    from dnsbox_b200.ops import Box
+    n = 8 if ns > 100 else 16
+    kw = dict(nu=0.025, bandlim=True, kCutOff=2.5, Pin=0.1, tstep_fix=True, dt=1e-3)
+    u = ic.random_field(n, seed=2, k0=3.0)
+    a, b = Box(n, **kw), Box(n, **kw)
+    u0 = a.from_numpy(u)
+    gT = a.from_numpy(solenoidal(n, 4))
+    got = a.heun_steps_vjp(u0, ns, gT, every=every, want_uT=want_uT)
+    states, recs = [b.from_numpy(u)], []
+    for _ in range(ns):
+        states.append(states[-1].clone())
+        recs += b.step(states[-1], 1)
+    for first in reversed(range(0, ns, every)):
+        v = states[first].clone()
+        for _ in range(min(every, ns - first) - 1):
+            recs += b.step(v, 1)
+    if want_uT:
+        assert torch.equal(got[1], states[ns])
+    assert a.get_time() == b.get_time()
+    keep = min(len(recs), 1024)
+    assert a.diag_read(keep) == recs[-keep:]
+    with pytest.raises(Exception):
+        a.diag_read(len(recs) + 1)
