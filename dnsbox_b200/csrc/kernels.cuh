@@ -1391,10 +1391,18 @@ template <typename T, int N> struct XVjp {
 // The x pass of rhs_nonlinear's transpose: C2R of u, omega and phi, the cross
 // products u x phi and phi x omega, and their R2C, in the manner of
 // k_xline_nl_g.  The products are taken one after the other, so that a lane
-// holds two vectors at a time: U + iV and FX + i FY (a pair in FP32), W +
-// i 2^e FZ, then u x phi forward, then OX + i OY with OZ (+ i 0), phi x omega
-// forward.  It replaces nine C2R and six R2C lines of global memory traffic and
-// a pointwise kernel: at 96^3 FP32 one kernel of 24 us where four took 58.
+// holds two vectors at a time.
+// A transform rounds the parts of its sequence relative to the larger one, and
+// neither the cotangent's scale is the flow's nor one component's another's: a
+// sequence holds two neighbouring lines (a, b) of one field.  The P-lane groups
+// of a and b (neighbours in a warp) each transform one of two fields,
+// U_a + i U_b and V_a + i V_b, and swap a real line, after which either holds
+// both fields of its own line; the other way round forward.  (FX, FY) are the
+// second of a pair in FP32; then (W, FZ); (OX, OY) with OZ, alone on its line.
+// It replaces nine C2R and six R2C lines of global memory traffic and a
+// pointwise kernel, four kernels of 58 us at 96^3 FP32.  With both parts of a
+// sequence from one line, and small ones lost in large ones, it took 28.5 us at
+// 96^3 FP32 and 12.1 at 64^3 FP64 (from a cold L2); the swaps make it 29.9, 12.8.
 template <typename T, int N>
 __global__ void __launch_bounds__(XReg<T, N>::NT, XVjp<T, N>::minb)
     k_xline_vjp(const __grid_constant__ XlineVjpArgs<T> a) {
@@ -1414,19 +1422,52 @@ __global__ void __launch_bounds__(XReg<T, N>::NT, XVjp<T, N>::minb)
   __syncthreads();
   pdl_wait();
   const int g = threadIdx.x / P, p = threadIdx.x % P, lane = threadIdx.x & 31;
+  const bool odd = g & 1;
   unsigned char *tile = smem_raw + SH::tw + (size_t)g * SH::line;
   V1 *s1 = reinterpret_cast<V1 *>(tile);
   V2 *s2 = reinterpret_cast<V2 *>(tile);
   const unsigned blk = gridDim.x - 1 - blockIdx.x;   // last lines first, as pass B left them in L2
-  const long long line = (long long)blk * (blockDim.x / P) + g;
-  const bool on = line < a.nlines;
+  const long long line = (long long)blk * (blockDim.x / P) + g, la = line - odd;
+  const bool on = line < a.nlines;   // of both lines: their number is even
   const int mirror = (lane & ~(P - 1)) | ((P - p) & (P - 1));
   auto sync = []() { __syncwarp(); };
-  auto load = [&](const C *f, C *x) {
-    const C *r = f + line * a.pitch + p;
+  auto load = [&](const C *f, long long l, C *x) {
+    const C *r = f + l * a.pitch + p;
 #pragma unroll
     for (int i = 0; i <= H; ++i) x[i] = ld_on(r + P * i, on && (i < H || p == 0));
     if (p == 0) x[0].y = x[H].y = 0;   // a C2R drops these imaginary parts
+  };
+  // v[i] of the other line's group in exchange for this one's
+  auto swap = [&](T *v) {
+    if constexpr (P < 32) {
+#pragma unroll
+      for (int i = 0; i < E; ++i) v[i] = __shfl_xor_sync(0xffffffffu, v[i], P);
+    } else {   // the two warps of a pair, through their tiles
+      auto both = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + (g >> 1)) : "memory"); };
+      T *mine = reinterpret_cast<T *>(tile) + lane;
+      const T *other = reinterpret_cast<const T *>(smem_raw + SH::tw + (size_t)(g ^ 1) * SH::line) + lane;
+      static_assert(E * 32 * sizeof(T) <= SH::line, "a line's values fit its tile");
+      sync();   // the transform's reads of the tile are through
+#pragma unroll
+      for (int i = 0; i < E; ++i) mine[32 * i] = v[i];
+      both();
+#pragma unroll
+      for (int i = 0; i < E; ++i) v[i] = other[32 * i];
+      both();
+    }
+  };
+  // the real lines of both fields on the own line, from lines a (re) and b (im) of the own field
+  auto own = [&](T *re, T *im, T *f0, T *f1) {
+    T x[E];
+#pragma unroll
+    for (int i = 0; i < E; ++i) x[i] = odd ? re[i] : im[i];
+    swap(x);
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      const T r = re[i], m = im[i];
+      f0[i] = odd ? x[i] : r;
+      f1[i] = odd ? m : x[i];
+    }
   };
   // inverse transform of X1 + i X2 into (re, im) at row p + P q in [out_i(q)]
   auto inv1 = [&](const C *x1, const C *x2, T *re, T *im) {
@@ -1453,16 +1494,28 @@ __global__ void __launch_bounds__(XReg<T, N>::NT, XVjp<T, N>::minb)
       inv1(x3, x4, r2, i2);
     }
   };
-  // forward transforms of c0 + i c1 and c2 + i 0, stored as the half lines of d[0..2]
-  auto fwd = [&](const T *c0, const T *c1, const T *c2, C *const *d) {
+  // forward transforms of the own line's c0, c1, c2, stored as half lines of d[0..2]:
+  // one of c0 and c1 for both lines, c2 + i 0
+  auto fwd = [&](T *c0, T *c1, const T *c2, C *const *d) {
+    T x1[E];
+#pragma unroll
+    for (int i = 0; i < E; ++i) x1[i] = odd ? c0[i] : c1[i];
+    swap(x1);
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      const T r = odd ? x1[i] : c0[i];
+      c1[i] = odd ? c1[i] : x1[i];   // line b
+      c0[i] = r;                     // line a
+    }
+    C *const d0 = odd ? d[1] : d[0], *const d2 = d[2];
     auto store = [&](int i, T zr, T zi, T nr, T ni) {
       if (!(on && (i < H || p == 0))) return;
-      const long long o = line * a.pitch + p + P * i;
-      d[0][o] = mkc<C>(T(0.5) * (zr + nr), T(0.5) * (zi - ni));
-      d[1][o] = mkc<C>(T(0.5) * (zi + ni), T(0.5) * (nr - zr));
+      C *const o = d0 + la * a.pitch + p + P * i;
+      o[0] = mkc<C>(T(0.5) * (zr + nr), T(0.5) * (zi - ni));
+      o[a.pitch] = mkc<C>(T(0.5) * (zi + ni), T(0.5) * (nr - zr));
     };
     auto store3 = [&](int i, T zr, T zi) {
-      if (on && (i < H || p == 0)) d[2][line * a.pitch + p + P * i] = mkc<C>(zr, zi);
+      if (on && (i < H || p == 0)) d2[line * a.pitch + p + P * i] = mkc<C>(zr, zi);
     };
     if constexpr (PAIR) {
       V2 z[E], x[E];
@@ -1516,26 +1569,24 @@ __global__ void __launch_bounds__(XReg<T, N>::NT, XVjp<T, N>::minb)
   T u[E], v[E], w[E], fx[E], fy[E], fz[E];
   {
     C x1[H + 1], x2[H + 1], x3[H + 1], x4[H + 1], x5[H + 1], x6[H + 1];
-    load(a.U, x1);
-    load(a.V, x2);
-    load(a.FX, x3);
-    load(a.FY, x4);
-    load(a.W, x5);   // on their way during the first transforms
-    load(a.FZ, x6);
+    const C *const q1 = odd ? a.V : a.U, *const q2 = odd ? a.FY : a.FX, *const q3 = odd ? a.FZ : a.W;
+    load(q1, la, x1);
+    load(q1, la + 1, x2);
+    load(q2, la, x3);
+    load(q2, la + 1, x4);
+    load(q3, la, x5);   // on their way during the first transforms
+    load(q3, la + 1, x6);
     inv2(x1, x2, x3, x4, u, v, fx, fy);
-    const int d = balance<P, H>(x5, x6);
-    const T up = pow2<T>(d);
-#pragma unroll
-    for (int i = 0; i <= H; ++i) x6[i] = mkc<C>(x6[i].x * up, x6[i].y * up);
+    own(u, v, u, v);
+    own(fx, fy, fx, fy);
     inv1(x5, x6, w, fz);
-    const T down = pow2<T>(-d);
-#pragma unroll
-    for (int i = 0; i < E; ++i) fz[i] *= down;
+    own(w, fz, w, fz);
   }
   C x1[H + 1], x2[H + 1], x3[H + 1], x0[H + 1];
-  load(a.OX, x1);
-  load(a.OY, x2);
-  load(a.OZ, x3);
+  const C *const q1 = odd ? a.OY : a.OX;
+  load(q1, la, x1);
+  load(q1, la + 1, x2);
+  load(a.OZ, line, x3);
 #pragma unroll
   for (int i = 0; i <= H; ++i) x0[i] = mkc<C>(0, 0);
 #pragma unroll
@@ -1546,6 +1597,7 @@ __global__ void __launch_bounds__(XReg<T, N>::NT, XVjp<T, N>::minb)
   fwd(u, v, w, a.A);
   T zero[E];
   inv2(x1, x2, x3, x0, u, v, w, zero);   // omega
+  own(u, v, u, v);
 #pragma unroll
   for (int i = 0; i < E; ++i) {   // phi x omega
     const T c0 = fy[i] * w[i] - fz[i] * v[i], c1 = fz[i] * u[i] - fx[i] * w[i], c2 = fx[i] * v[i] - fy[i] * u[i];

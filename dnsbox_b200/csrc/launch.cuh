@@ -213,8 +213,8 @@ template <typename T, int N>
 cudaError_t Launcher<T, N>::xline_vjp(const XlineVjpArgs<T> &a, cudaStream_t st) {
   if constexpr (XReg<T, N>::on) {
     using SH = XReg<T, N>;
-    int nt = SH::NT;
-    while (nt > 32 && (long long)a.nlines * SH::PL::P < 148LL * 4 * nt) nt >>= 1;
+    int nt = SH::NT;   // pairs of lines: at least two in a block
+    while (nt > 32 && nt > 2 * SH::PL::P && (long long)a.nlines * SH::PL::P < 148LL * 4 * nt) nt >>= 1;
     const int lpb = nt / SH::PL::P;
     const cudaError_t e = set_smem(k_xline_vjp<T, N>, SH::smem(nt));
     if (e != cudaSuccess) return e;

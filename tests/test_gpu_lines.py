@@ -162,3 +162,60 @@ def test_cut_check_single_mode(nx, prec):
     b.step(u, 1, diag=False)
     assert not b.step_pruned()
     b.close()
+
+
+def single_parts(nx, ny, nz, delta):
+    """(name, u, g, component): fields whose transposed term's `component` comes from the part of size delta alone,
+    which shares a complex sequence of the x kernel with a part of size 1 (u and v, phi_x and phi_y, omega_x and omega_y;
+    the products of each likewise)."""
+    z, y, x = np.meshgrid(*(2 * np.pi * np.arange(n) / n for n in (nz, ny, nx)), indexing="ij")
+    full = lambda *f: np.stack([a + 0 * x for a in f])
+    s = np.cos(y) + np.sin(2 * y)
+    return [("u", full(np.cos(y), delta * np.cos(x), 0), full(0, 0, s), 2),
+            ("phi", full(0, 0, s), full(np.cos(y), delta * np.cos(x) * np.cos(y) * np.cos(z),
+                                        delta * np.cos(x) * np.sin(y) * np.sin(z)), 2),
+            ("omega", full(0, 0, np.cos(y) + delta * np.cos(x)), full(0, 0, s), 0)]
+
+
+@pytest.mark.parametrize("prec,delta", [("fp64", 1e-8), ("fp32", 1e-5)])
+@pytest.mark.parametrize("nx", SIZES[:-1])
+def test_transposed_term_small_parts(nx, prec, delta):
+    """Every part of the transposed term to its own precision: the bar of test_transposed_term_line_length for the small
+    component alone (a transform rounds the parts of a sequence relative to the larger one: 1e-8 and 1e-3 and more here)."""
+    from dnsbox_b200.ops import Box
+    ny, nz = 12, 8
+    g = O.Grid(O.Params(nx=nx, ny=ny, nz=nz, bandlim=False))
+    b = Box(nx=nx, ny=ny, nz=nz, precision=prec, bandlim=False)
+    for name, u, c, part in single_parts(nx, ny, nz, delta):
+        uh, ch = O.state_u2uhat(g, u), O.state_u2uhat(g, c)
+        got = b.rhs_nonlinear_vjp(b.from_numpy(uh), b.from_numpy(ch)).cpu().numpy()
+        want = O.rhs_nonlinear_vjp(g, uh, ch)
+        assert rel(got[part], want[part]) < 2 * TOL[prec], name
+        assert rel(got, want) < 2 * TOL[prec], name
+    b.close()
+
+
+def plane_flow(g, nx, ny, nz, seed):
+    """u(x, y), v(x, y), w = 0."""
+    rng = np.random.default_rng(seed)
+    f = np.broadcast_to(rng.standard_normal((3, 1, ny, nx)), (3, nz, ny, nx)).copy()
+    f[2] = 0
+    return O.state_dealias(g, O.state_project(g, O.state_u2uhat(g, f)))
+
+
+@pytest.mark.parametrize("prec,powers", [("fp64", (-300, 300)), ("fp32", (-50, 100))])
+@pytest.mark.parametrize("nx", SIZES[:-1])
+def test_transposed_term_scales_with_the_cotangent(nx, prec, powers):
+    """The transposed term is linear in the cotangent, and a power of two is exact, however far the cotangent is from the
+    velocity whose complex sequences it shares; with w = 0 and with a rough field."""
+    from dnsbox_b200.ops import Box
+    ny, nz = 12, 8
+    g = O.Grid(O.Params(nx=nx, ny=ny, nz=nz, bandlim=False))
+    b = Box(nx=nx, ny=ny, nz=nz, precision=prec, bandlim=False)
+    c = b.from_numpy(rough(g, nx, ny, nz, seed=nx + 1) * 1e-3)
+    for uh in (plane_flow(g, nx, ny, nz, seed=nx), rough(g, nx, ny, nz, seed=nx)):
+        u = b.from_numpy(uh)
+        one = b.rhs_nonlinear_vjp(u, c)
+        for k in powers:
+            assert torch.equal(b.rhs_nonlinear_vjp(u, c * 2.0 ** k), one * 2.0 ** k), k
+    b.close()
