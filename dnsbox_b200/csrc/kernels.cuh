@@ -927,10 +927,11 @@ template <typename T> __device__ __forceinline__ T pow2(int e) {
 // (largest component of each, over the line's P lanes): they share one complex
 // sequence, whose parts are rounded relative to each other; pow2(-e) undoes it.
 // Where one of them vanishes, its part of the result is the other's rounding,
-// which may be far above the field it belongs to: x2 is brought down to 2^-40,
-// or for a vanishing x2, e is the type's bias, whose pow2(-e) is 0.
-template <int P, int H, typename C> __device__ __forceinline__ int balance(const C *x1, const C *x2) {
+// which may be far above the field it belongs to: for a vanishing x2, e is the
+// type's bias, whose pow2(-e) is 0; for a vanishing x1, flat is set.
+template <int P, int H, typename C> __device__ __forceinline__ int balance(const C *x1, const C *x2, bool &flat) {
   using T = decltype(C{}.x);
+  constexpr int bias = sizeof(T) == 4 ? 127 : 1023;
   T m1 = 0, m2 = 0;
 #pragma unroll
   for (int i = 0; i <= H; ++i) {
@@ -942,7 +943,8 @@ template <int P, int H, typename C> __device__ __forceinline__ int balance(const
     m1 = fmax(m1, __shfl_xor_sync(0xffffffffu, m1, o));
     m2 = fmax(m2, __shfl_xor_sync(0xffffffffu, m2, o));
   }
-  return m2 > 0 ? m1 > 0 ? max(-96, min(96, expo(m1) - expo(m2))) : -40 : sizeof(T) == 4 ? 127 : 1023;
+  flat = m1 == 0;
+  return m2 > 0 ? m1 > 0 ? max(1 - bias, min(bias - 1, expo(m1) - expo(m2))) : 0 : bias;
 }
 
 // Exchange tile of one line: rows skewed by row / R0, or for the 4 x 4 x ..
@@ -1029,7 +1031,7 @@ __global__ void __launch_bounds__(XReg<T, N>::NT, XReg<T, N>::minb)
   };
   auto shfl = [&](T v) { return __shfl_sync(0xffffffffu, v, mirror); };
   auto pack = [&](const C *x1, const C *x2, auto put) { pack_lines<E>(x1, x2, p, mirror, put); };
-  T up = 1, down = 1;
+  T down, keep;   // factors of oz and w (0 where they vanish: a value that is no number stays one)
   V1 w[E];   // (w, 2^e oz) at row p + P q in w[out_i(q)]
   T u_[E], v_[E], ox_[E], oy_[E];
   C xw[H + 1], xo[H + 1];
@@ -1067,9 +1069,9 @@ __global__ void __launch_bounds__(XReg<T, N>::NT, XReg<T, N>::minb)
     }
   }
   {
-    const int d = balance<P, H>(xw, xo);
-    up = pow2<T>(d);
-    down = pow2<T>(-d);
+    bool flat;
+    const int d = balance<P, H>(xw, xo, flat);
+    const T up = pow2<T>(d);
 #pragma unroll
     for (int i = 0; i <= H; ++i) xo[i] = mkc<C>(xo[i].x * up, xo[i].y * up);
     V1 z[E];
@@ -1077,6 +1079,8 @@ __global__ void __launch_bounds__(XReg<T, N>::NT, XReg<T, N>::minb)
     sync();
     vfft<PL, true, AD>(z, w, s1, 0, p, twt, sync);
     sync();
+    down = pow2<T>(-d);
+    keep = flat ? T(0) : T(1);
   }
   // (omega x u) s at the lane's rows, and the CFL maxima
   const T sc = T(a.s);
@@ -1084,7 +1088,7 @@ __global__ void __launch_bounds__(XReg<T, N>::NT, XReg<T, N>::minb)
   T px[E], py[E], pz[E];
 #pragma unroll
   for (int i = 0; i < E; ++i) {
-    const T u = u_[i], v = v_[i], ww = w[i].re, oz = w[i].im * down, ox = ox_[i], oy = oy_[i];
+    const T u = u_[i], v = v_[i], ww = w[i].re * keep, oz = w[i].im * down, ox = ox_[i], oy = oy_[i];
     px[i] = (oy * ww - oz * v) * sc;
     py[i] = (oz * u - ox * ww) * sc;
     pz[i] = (ox * v - oy * u) * sc;
@@ -1212,6 +1216,7 @@ __global__ void __launch_bounds__(XSplit<T, N>::NT, XSplit<T, N>::minb)
   constexpr bool PAIR = NP == 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int ex[L];
+  __shared__ bool noW[L];
   V1 *twi = reinterpret_cast<V1 *>(smem_raw), *twf = twi + (R1 - 1) * R0;
   pdl_launch();
   for (int i = threadIdx.x; i < (R1 - 1) * R0; i += SH::NT) twi[i] = VtwOf<V1>::of(__ldg(a.tw + (1 + i / R0) * (i % R0)));
@@ -1267,8 +1272,9 @@ __global__ void __launch_bounds__(XSplit<T, N>::NT, XSplit<T, N>::minb)
 #pragma unroll
       for (int r = 0; r < R0; ++r) reinterpret_cast<V1 *>(bufp(1, lo))[inv_at(po * R0 + r)] = y[r];
     }
-    const int d = balance<PO, H>(x5, x6);
-    if (po == 0) ex[lo] = d;
+    bool flat;
+    const int d = balance<PO, H>(x5, x6, flat);
+    if (po == 0) ex[lo] = d, noW[lo] = flat;
     const T up = ldexp(T(1), d);   // ldexp: 251 us where pow2 takes 262 (32 boxes of 96^3)
 #pragma unroll
     for (int i = 0; i <= H; ++i) x6[i] = mkc<C>(x6[i].x * up, x6[i].y * up);
@@ -1296,14 +1302,16 @@ __global__ void __launch_bounds__(XSplit<T, N>::NT, XSplit<T, N>::minb)
 #pragma unroll
     for (int k = 0; k < NP; ++k) second(bufp(k, li), x[k]);
     second(bufs(li), w);
-    const T down = ex[li] > 96 ? T(0) : ldexp(T(1), -ex[li]), sc = T(a.s);
+    constexpr int bias = sizeof(T) == 4 ? 127 : 1023;
+    const T keep = noW[li] ? T(0) : T(1);
+    const T down = ex[li] == bias ? T(0) : ldexp(T(1), -ex[li]), sc = T(a.s);
     VP f[NP][R1];
 #pragma unroll
     for (int q = 0; q < R1; ++q) {
       T u, v, ox, oy;
       if constexpr (PAIR) u = f2_lo(x[0][q].re), v = f2_lo(x[0][q].im), ox = f2_hi(x[0][q].re), oy = f2_hi(x[0][q].im);
       else u = x[0][q].re, v = x[0][q].im, ox = x[1][q].re, oy = x[1][q].im;
-      const T ww = w[q].re, oz = w[q].im * down;
+      const T ww = w[q].re * keep, oz = w[q].im * down;
       const T px = (oy * ww - oz * v) * sc, py = (oz * u - ox * ww) * sc, pz = (ox * v - oy * u) * sc;
       m0 = fmax(m0, fabs(u));
       m1 = fmax(m1, fabs(v));

@@ -219,3 +219,18 @@ def test_transposed_term_scales_with_the_cotangent(nx, prec, powers):
         for k in powers:
             assert torch.equal(b.rhs_nonlinear_vjp(u, c * 2.0 ** k), one * 2.0 ** k), k
     b.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("shape", [(n, 12, 8) for n in SIZES] + [(96, 192, 96), (192, 96, 128)])
+def test_vanishing_w(shape, prec):
+    """A velocity without w beside a z vorticity, which share a complex sequence of the x kernels: max |w| is 0."""
+    from dnsbox_b200.ops import Box
+    nx, ny, nz = shape
+    b = Box(nx=nx, ny=ny, nz=nz, precision=prec, bandlim=False, tstep_fix=True, dt=1e-3)
+    g = O.Grid(O.Params(nx=nx, ny=ny, nz=nz, bandlim=False))
+    u = b.from_numpy(plane_flow(g, nx, ny, nz, seed=nx))
+    rec = b.step(u, 1)[0]
+    assert rec["umax"][2] == 0.0 and rec["umax"][0] > 0.0
+    assert not u[2].abs().max().item()
+    b.close()
