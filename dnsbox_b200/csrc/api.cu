@@ -673,7 +673,7 @@ static int run_rhs(dnsbox_ctx *c, const void *uin, int mode, void *out, void *st
   }
   x.tw = reinterpret_cast<const C *>(c->tw[0]);
   x.st = cfl ? c->st : nullptr;   // the CFL maxima, where they are used
-  x.lines_per_box = p.ny * p.nz;
+  x.lines_per_box = x.box_lines = p.ny * p.nz;
   x.nlines = c->nbatch * p.ny * p.nz;
   x.nxh = c->nxh;
   x.alpha_x = p.alpha_x;

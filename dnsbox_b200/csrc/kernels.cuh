@@ -506,7 +506,8 @@ template <typename T> struct XlineNLArgs {
   const C *tw;
   StepState *st;                       // per-box step state: umax[3] gets max |u_i| (true scale)
   int nlines, nxh;
-  int lines_per_box;                   // ny * nz
+  int lines_per_box;                   // ny * nz, of the planes of this launch
+  int box_lines;                       // ny * nz of the whole box
   int kxa;                             // pruning: only kx < kxa and kx = N/2 are read and written (0: all)
   int pin, pout;                       // row pitch (complex elements) of the inputs / outputs; 0: nxh
   int npad;                            // compact rows: slots after nyq that complete its 32-byte sector (written as 0)
@@ -1183,7 +1184,7 @@ __global__ void __launch_bounds__(XReg<T, N>::NT, XReg<T, N>::minb)
   }
 }
 
-// The fused x pass of 96- and 192-point lines: k_xline_nl_g with split plans
+// The fused x pass of 96- (FP32) and 192-point lines of large boxes: k_xline_nl_g with split plans
 // (SplitPlan), so that each transform exchanges once, not twice, through the
 // shared memory that bounds it.  A block of 8 lines: R1 lanes a line load,
 // form the sequences and run the inverse transforms' first stage; after one
@@ -1202,7 +1203,7 @@ template <typename T, int N> struct XSplit {
   static constexpr size_t smem = tw + (sizeof(T) == 4 ? buf + buf / 2 : 3 * buf);
   // 96 FP32: 18 warps by 96 registers (some spills) 258 us, 15 by 128 270, 21 by
   // 80 275 (32 boxes of 96^3); 192 FP32: 16 warps 65 us, 12 71 (192^3)
-  static constexpr int minb = sizeof(T) == 8 ? (N == 96 ? 3 : 2) : (N == 96 ? 6 : 4);
+  static constexpr int minb = sizeof(T) == 8 ? 2 : (N == 96 ? 6 : 4);
 };
 template <typename T, int N>
 __global__ void __launch_bounds__(XSplit<T, N>::NT, XSplit<T, N>::minb)

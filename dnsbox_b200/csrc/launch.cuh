@@ -168,15 +168,19 @@ template <typename T, int N>
 cudaError_t Launcher<T, N>::xline_nl(const XlineNLArgs<T> &a, int variant, cudaStream_t st) {
   using C = typename CT<T>::type;
   cudaError_t e;
-  if constexpr (SplitPlan<N>::on) {
-    // from two waves of blocks on: 32 boxes of 96^3 285 -> 250 us, 192^3 78 -> 64;
-    // with fewer lines its barriers cost more than they save (a 192 x 48 x 96
-    // step, 4608 lines, 92 -> 94 us, the 96^3 horizon gradient 5.66 -> 5.73 ms)
+  if constexpr (SplitPlan<N>::on && (sizeof(T) == 4 || N == 192)) {
+    // by the lines of one box, so that a box runs the same arithmetic whatever
+    // other boxes or ranks share its launch.  Split against equal shares, us:
+    // 192 points 9216 lines FP32 23.8 / 25.3, FP64 43.5 / 46.3, 36864 lines 68 / 77,
+    // 148 / 165; 96 points FP32 8192 lines 14.9 / 14.6, 18432 25.9 / 27.3, 36864
+    // 43.1 / 48.7, 32 boxes of 9216 255 / 290.  Below, its barriers cost more than
+    // they save (192 points, 4608 lines, FP32: 19.5 / 17.0); at 96 points in FP64
+    // it gains nothing (9216 lines 26.8 / 25.7, 36864 84.8 / 86.2).
     using SH = XSplit<T, N>;
-    const int blocks = (a.nlines + SH::L - 1) / SH::L;
-    if (blocks >= 2 * 148 * SH::minb) {
+    if (a.box_lines >= 8192) {
+      const unsigned blocks = (unsigned)((a.nlines + SH::L - 1) / SH::L);
       if ((e = set_smem(k_xline_nl_s<T, N>, SH::smem)) != cudaSuccess) return e;
-      return launch_pdl(k_xline_nl_s<T, N>, (unsigned)blocks, SH::NT, SH::smem, st, a);
+      return launch_pdl(k_xline_nl_s<T, N>, blocks, SH::NT, SH::smem, st, a);
     }
   }
   if constexpr (XReg<T, N>::on) {   // whatever the choice

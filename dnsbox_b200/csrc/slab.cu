@@ -387,6 +387,7 @@ int rhs_middle(dnsbox_slab *s, const void *recv5, double *umax, void *send3, cud
   x.tw = reinterpret_cast<const C *>(s->tw[0]);
   x.st = s->st;
   x.lines_per_box = s->ny * s->nzl;
+  x.box_lines = s->ny * s->nz;
   x.nlines = s->ny * s->nzl;
   x.nxh = s->nxh;
   x.alpha_x = s->p.alpha_x;

@@ -234,3 +234,42 @@ def test_vanishing_w(shape, prec):
     assert rec["umax"][2] == 0.0 and rec["umax"][0] > 0.0
     assert not u[2].abs().max().item()
     b.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("nx,ny,nz,nbatch", [(96, 96, 96, 2), (96, 48, 48, 8), (192, 48, 96, 3), (192, 192, 192, 2)])
+def test_a_box_alone_and_among_others(nx, ny, nz, nbatch, prec):
+    """The kernels of a box do not depend on the boxes that share its launch: bit for bit the box alone (the x pass of
+    96- and 192-point lines has two kernels)."""
+    from dnsbox_b200.ops import Box
+    kw = dict(nx=nx, ny=ny, nz=nz, precision=prec, nu=2e-3, bandlim=False, tstep_fix=True, dt=1e-3)
+    g = torch.Generator(device="cuda").manual_seed(nx)
+    one, batch = Box(**kw), Box(nbatch=nbatch, **kw)
+    u = batch.zeros()
+    for i in range(nbatch):
+        v = one.zeros()
+        for c in range(3):
+            v[c] = one.r2c(torch.randn(nz, ny, nx, generator=g, device="cuda", dtype=v.dtype.to_real()))
+        one.project(v)
+        one.dealias(v)
+        u[:, i] = v
+    first = u[:, 0].clone()
+    recs = batch.step(u, 2)
+    r = one.step(first, 2)
+    assert torch.equal(u[:, 0], first)
+    assert [s[0] for s in recs] == r
+    one.close()
+    batch.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("nx,ny,nz", [(96, 64, 96), (96, 64, 128), (192, 48, 128), (192, 64, 128)])
+def test_x_lines_at_the_split_rule(nx, ny, nz, prec):
+    """96- and 192-point lines of boxes of 6144 and of 8192 lines, where the x kernel changes, against the oracle."""
+    from dnsbox_b200.ops import Box
+    g = O.Grid(O.Params(nx=nx, ny=ny, nz=nz, bandlim=False))
+    uh = rough(g, nx, ny, nz, seed=nx + nz)
+    b = Box(nx=nx, ny=ny, nz=nz, precision=prec, bandlim=False)
+    got, _ = b.rhs_nonlinear(b.from_numpy(uh))
+    assert rel(got.cpu().numpy(), O.rhs_nonlinear(g, uh)) < TOL[prec]
+    b.close()

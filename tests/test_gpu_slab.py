@@ -336,3 +336,33 @@ def test_slab_heun_with_courant_control_matches_the_box(prec, tol):
     for s in slabs:
         s.close()
     box.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("shape,p", [((96, 96, 96), 2), ((192, 96, 128), 4)])
+def test_slab_rhs_of_split_x_lines(prec, shape, p):
+    """Grids whose x pass runs the split kernel: the slabs, each with a part of the box's lines, take the box's kernel and
+    agree with it bit for bit."""
+    from dnsbox_b200.ops import Box
+    from dnsbox_b200.slab import SlabFFT
+    nx, ny, nz = shape
+    kw = dict(nu=0.01, bandlim=False)
+    box = Box(nx=nx, ny=ny, nz=nz, precision=prec, **kw)
+    gen = torch.Generator(device="cuda").manual_seed(nx)
+    ub = box.zeros()
+    for c in range(3):
+        ub[c] = box.r2c(torch.randn(nz, ny, nx, generator=gen, device="cuda", dtype=ub.dtype.to_real()))
+    box.project(ub)
+    box.dealias(ub)
+    nb, _ = box.rhs_nonlinear(ub)
+    slabs = [SlabFFT(nx, ny, nz, precision=prec, rank=r, nranks=p) for r in range(p)]
+    for s in slabs:
+        s.setup_rhs(**kw)
+    nyl = ny // p
+    states = [ub[:, :, r * nyl:(r + 1) * nyl, :].contiguous() for r in range(p)]
+    outs = [torch.full(s.state_shape(), complex("nan"), dtype=s.cdtype, device="cuda") for s in slabs]
+    _emulate_rhs(slabs, states, outs)
+    assert torch.equal(torch.cat(outs, dim=2), nb)
+    for s in slabs:
+        s.close()
+    box.close()
