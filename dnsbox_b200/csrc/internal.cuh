@@ -157,7 +157,7 @@ struct Prof {
 // rhs_Eband (rhs.f90:137-168) over the precomputed band-mode list; optionally
 // resets the CFL maxima.  One block per box.
 template <typename C> __global__ void k_eband(BandArgs b, int nx, int reset_umax) {
-  __shared__ double red[32];
+  __shared__ double red[kBandRed];
   pdl_launch();
   pdl_wait();
   eband_block<C>(b, nx, blockIdx.x, reset_umax, red);

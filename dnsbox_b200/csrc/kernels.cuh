@@ -98,36 +98,51 @@ struct BandArgs {
   const void *u;    // the right-hand side's input, components nh apart, boxes bstride apart
   long long nh, bstride;
 };
-// rhs_Eband (rhs.f90:137-168) of box `box` by one block (red: 32 doubles);
-// optionally resets the CFL maxima.
+// rhs_Eband (rhs.f90:137-168) of box `box` by one block (red: kBandRed doubles);
+// optionally resets the CFL maxima.  256 partial sums (modes j, j + 256, ..) and
+// a fixed tree over them, whatever the number of threads: the band energy is
+// one number, of a block of its own and of a tail block of any pass A.
+constexpr int kBandRed = 256;
 template <typename C>
 __device__ __forceinline__ void eband_block(const BandArgs &b, int nx, int box, bool reset_umax, double *red) {
   const C *u = reinterpret_cast<const C *>(b.u) + (long long)box * b.bstride;
   StepState *st = b.st + box;
-  double acc = 0.0;
-#pragma unroll 4
-  for (int i = threadIdx.x; i < b.n; i += blockDim.x) {
+  auto energy = [&](int i) {
     const long long off = (long long)(unsigned)b.modes[3 * i] | ((long long)b.modes[3 * i + 1] << 32);
-    const int kx = b.modes[3 * i + 2];
-    const double w = (k_half(kx, nx, 1.0) == 0.0) ? 0.5 : 1.0;   // rhs.f90:151-155
+    const double w = (k_half(b.modes[3 * i + 2], nx, 1.0) == 0.0) ? 0.5 : 1.0;   // rhs.f90:151-155
     double e = 0.0;
+#pragma unroll
     for (int c = 0; c < 3; ++c) {
       const C v = u[c * b.nh + off];
-      e += ((double)v.x * v.x + (double)v.y * v.y) * w;
+      e = fma(fma((double)v.x, (double)v.x, __dmul_rn(v.y, v.y)), w, e);   // one rounding in every kernel
     }
-    acc += e;
+    return e;
+  };
+  // thread t of nt (a divisor of 256) owns the sums t, t + nt, ..; four modes in flight
+  const int nt = min((int)blockDim.x, kBandRed), t = threadIdx.x;
+  if (t < nt) {
+    for (int j = t; j < kBandRed; j += nt) red[j] = 0.0;
+    for (int i = t; i < b.n; i += 4 * nt) {
+      double e[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) e[m] = i + m * nt < b.n ? energy(i + m * nt) : 0.0;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) red[(i + m * nt) % kBandRed] += e[m];
+    }
   }
-  double v[1] = {acc};
-  if (blockDim.x < 32) {   // no whole warp to shuffle in
-    red[threadIdx.x] = acc;
+  __syncthreads();
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {   // each 32 sums
+    for (int j = threadIdx.x; j < kBandRed / 32 * o; j += blockDim.x) {
+      double *r = red + j / o * 32 + j % o;
+      r[0] += r[o];
+    }
     __syncthreads();
-    if (threadIdx.x == 0)
-      for (unsigned i = 1; i < blockDim.x; ++i) v[0] += red[i];
-  } else {
-    block_sum<1>(v, red);
   }
   if (threadIdx.x == 0) {
-    st->eband = v[0] * b.s2;
+    for (int o = kBandRed / 64; o; o >>= 1)
+      for (int j = 0; j < o; ++j) red[32 * j] += red[32 * (j + o)];
+    st->eband = red[0] * b.s2;
     if (reset_umax) st->umax[0] = st->umax[1] = st->umax[2] = 0.0;
   }
 }
@@ -235,7 +250,7 @@ template <typename T, int N> struct StridedShape {
   static constexpr size_t tile = PL::NST > 1 ? (size_t)N * W * 16 : 0;
   static constexpr size_t smem(bool inv) {   // tile, twiddles and (inverse) row multipliers
     const size_t n = tile + (size_t)vtw_size<PL>() * 16 + (inv ? 2 * N * sizeof(T) : 0);
-    return n < 256 ? 256 : n;   // 32 doubles for the band block
+    return n < kBandRed * sizeof(double) ? kBandRed * sizeof(double) : n;   // the band block's sums
   }
   // Resident CTAs asked of the register allocator: 16 warps per SM where a
   // thread holds 16 values (128 registers), 20 at 12 (96), 24 at 8 (80).  The

@@ -273,3 +273,23 @@ def test_x_lines_at_the_split_rule(nx, ny, nz, prec):
     got, _ = b.rhs_nonlinear(b.from_numpy(uh))
     assert rel(got.cpu().numpy(), O.rhs_nonlinear(g, uh)) < TOL[prec]
     b.close()
+
+
+@pytest.mark.parametrize("kcut", [2.5, 6.0, 9.5])
+@pytest.mark.parametrize("nz", [8, 12, 16, 24, 32, 48, 64, 96, 128, 192, 256])
+def test_band_energy_of_every_path(nz, kcut):
+    """One band energy: of the operator, the right-hand side and the step record, full and pruned, whatever block adds it
+    up (a tail block of pass A, whose threads depend on nz, or a launch of its own); narrow and wide bands."""
+    from dnsbox_b200.ops import Box
+    kw = dict(nx=24, ny=32, nz=nz, nu=2e-3, kCutOff=kcut, Pin=0.1, bandlim=True, tstep_fix=True, dt=1e-3)
+    g = O.Grid(O.Params(nx=24, ny=32, nz=nz, nu=2e-3, kCutOff=kcut, Pin=0.1, bandlim=True))
+    uh = rough(g, 24, 32, nz, seed=nz)
+    b, full = Box(**kw), Box(prune=False, **kw)
+    u, v = b.from_numpy(uh), b.from_numpy(uh)
+    want = b.eband(u)
+    assert abs(want / O.rhs_eband(g, uh) - 1) < 1e-13
+    assert b.rhs_nonlinear(u)[1] == want
+    assert b.step(u, 1)[0]["eband"] == want and b.step_pruned()
+    assert full.step(v, 1)[0]["eband"] == want and not full.step_pruned()
+    b.close()
+    full.close()

@@ -75,3 +75,23 @@ def test_state_with_cut_content_takes_the_full_path():
     uh[0, 5, 3, 13] = 1e-3 + 2e-3j          # kx = 13 >= 32/3 (not the Nyquist column 16): cut
     (up, _, pr), (uf, _, _) = run_pair((n, n, n), "fp64", 3, uh, **FORCED)
     assert not pr and torch.equal(up, uf)
+
+
+@pytest.mark.parametrize("tc", [(2, 1, 1), (1, 2, 2), (2, 2, 2)])
+def test_pruned_with_a_mixed_schedule_and_a_wide_band(tc):
+    """Tensor-core and SIMT passes side by side, and a band of more modes than a block has threads: where the band
+    energy is formed does not depend on pruning."""
+    from dnsbox_b200.ops import Box
+    n = 128
+    uh = ic.random_field(n, seed=5, k0=4.0)
+    out = []
+    for prune in (True, False):
+        b = Box(n, precision="tc_split", prune=prune, nu=2e-3, kCutOff=7.5, Pin=0.1, courant_min=0.5, courant_max=0.5)
+        b.set_schedule(tc)
+        u = b.from_numpy(uh)
+        recs = b.step(u, 4)
+        out.append((u.cpu(), recs))
+        assert b.step_pruned() == prune
+        b.close()
+    assert torch.equal(out[0][0], out[1][0])
+    assert out[0][1] == out[1][1]
