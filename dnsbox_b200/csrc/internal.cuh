@@ -220,6 +220,12 @@ template <typename T> struct Ops {
     switch (n) { DNSBOX_SIZES(DNSBOX_CASE_HASXW) }
     return false;
   }
+#define DNSBOX_CASE_STHR(NN) \
+  case NN: return Launcher<T, NN>::strided_threads();
+  static int strided_threads(int n) {
+    switch (n) { DNSBOX_SIZES(DNSBOX_CASE_STHR) }
+    return 0;
+  }
 #define DNSBOX_CASE_HASXV(NN) \
   case NN: return Launcher<T, NN>::has_xline_vjp();
   static bool has_xline_vjp(int n) {

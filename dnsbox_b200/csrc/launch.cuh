@@ -30,6 +30,7 @@ static inline cudaError_t launch_pdl(void (*kernel)(KA...), dim3 grid, dim3 bloc
 
 template <typename T, int N> struct Launcher {
   static cudaError_t strided(const StridedArgs<T> &a, bool inv, int ntiles, cudaStream_t st);
+  static int strided_threads();   // of a block
   // tensor-core split-precision form of `strided` (FP32, N = 128 .. 1024);
   // adft: the four DFT-64 operands, status: set to 1 if an MMA wait gave up
   static cudaError_t strided_tc(const StridedArgs<T> &a, bool inv, int nother, const void *adft, int *status,
@@ -88,6 +89,8 @@ cudaError_t Launcher<T, N>::strided(const StridedArgs<T> &a, bool inv, int ntile
   if (ws == 1) return strided_launch<T, N, false, ST_FROM_WS>(a, nb, st);
   return strided_launch<T, N, false, ST_ANY>(a, nb, st);
 }
+
+template <typename T, int N> int Launcher<T, N>::strided_threads() { return StridedShape<T, N>::NT; }
 
 template <typename T, int N> bool Launcher<T, N>::has_tc() {
   return std::is_same<T, float>::value && TcPlan<N>::on;
