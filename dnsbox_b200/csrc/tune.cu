@@ -13,8 +13,8 @@
 // E1) stay selectable by dnsbox_set_schedule but are not candidates: they
 // measured slower than both others at every size.  Each uniform candidate schedule advances a copy of the caller's
 // state for a few steps with pass timing on (CUDA events on the context's
-// stream); every pass keeps its fastest kernel; the chosen schedule is timed
-// once more.  The context's clock, time step and step history are restored,
+// stream); the schedule of every pass's fastest kernel is timed too, and the
+// fastest of them all is kept.  The context's clock, time step and step history are restored,
 // and the choice is cached per (device, precision, grid, boxes) so that later
 // contexts of the same shape start with it.
 #include <map>
@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "internal.cuh"
+#include "tune_pick.h"
 
 namespace {
 
@@ -203,14 +204,17 @@ extern "C" int dnsbox_autotune(dnsbox_ctx *ctx, const void *uh, int nsteps, dnsb
         if (r.s.x_kernel == xv) sum += r.pass[DNSBOX_PASS_X_NL], ++n;
       if (n && sum / n < bestx) bestx = sum / n, best.x_kernel = xv;
     }
-    best.ms_default = runs.empty() ? 0.0 : runs[0].step;   // cp.async passes, default x kernel
     double pass_tmp[DNSBOX_NPASS];
     rc = trial(ctx, best, uh, scratch, bytes, sv, nsteps, pass_tmp, &best.ms_tuned);
-    // keep the default when the combination measures slower than it
-    if (rc == DNSBOX_OK && best.ms_tuned > best.ms_default) {
-      const double mt = best.ms_default;
-      best = runs[0].s;
-      best.ms_default = best.ms_tuned = mt;
+    if (rc == DNSBOX_OK) {
+      std::vector<double> ms;
+      for (const Run &r : runs) ms.push_back(r.step);
+      const int k = fastest_schedule(ms.data(), (int)ms.size(), best.ms_tuned);
+      if (k >= 0) {
+        best = runs[k].s;
+        best.ms_tuned = ms[k];
+      }
+      best.ms_default = ms[0];   // cp.async passes, default x kernel
     }
     best.tuned = 1;
   }
