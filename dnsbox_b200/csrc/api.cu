@@ -902,7 +902,7 @@ int run_strided_tma(dnsbox_ctx *c, int axis, bool inv, const StridedArgs<float> 
                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return set_err(DNSBOX_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
   Prof pr(c, kind);
-  CK(Ops<float>::strided_tma(n, t, inv, c->adft, c->tc_status, c->tma_ctas_per_sm * c->nsm, c->stream));
+  CK(Ops<float>::strided_tma(n, t, inv, c->adft, c->tc_status, c->nsm, c->stream));
   return DNSBOX_OK;
 }
 
@@ -1148,11 +1148,6 @@ static int alloc_dft64(dnsbox_ctx *c) {
   const char *br = getenv("DNSBOX_TMA_BOX_ROWS");
   const int brv = br ? atoi(br) : 32;
   c->tma_box_rows = (brv == 8 || brv == 16 || brv == 32 || brv == 64) ? brv : 32;
-  // resident CTAs per SM of the TMA passes (DNSBOX_TMA_CTAS_PER_SM = 2 for
-  // two; one by default: with two per SM, repeated 256^3 pruned steps gave an
-  // occasional wrong result that one CTA per SM never showed)
-  const char *cps = getenv("DNSBOX_TMA_CTAS_PER_SM");
-  c->tma_ctas_per_sm = (cps && atoi(cps) == 2) ? 2 : 1;
   return DNSBOX_OK;
 }
 

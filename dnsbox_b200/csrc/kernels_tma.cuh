@@ -30,9 +30,10 @@
 // completes on an mbarrier; the next tile's loads are issued as soon as the
 // current tile's stage A has read the staging tile, so they land while its
 // DFT, split and MMAs run (a two-input job stages its second input after the
-// first).  Two 256-thread CTAs share an SM, each with its own staging tile, B
-// operand (MN-major 128-byte swizzle) and 128-column TMEM accumulator, so the
-// phases and waits of one overlap the work of the other; a tile's
+// first).  One 256-thread CTA per SM, with a staging tile, B operand (MN-major
+// 128-byte swizzle) and 128-column TMEM accumulator; its shared memory is asked
+// for so that a second one does not fit, since with two per SM repeated 256^3
+// pruned steps gave an occasional wrong result whose cause is not known; a tile's
 // accumulator is drained straight to HBM at the start of the next tile's
 // split, before the next MMAs are issued.  Per-tile column data (half-axis
 // index, wavenumber, unscale factor) is tabulated once in shared memory and
@@ -56,11 +57,11 @@ template <int N> struct TmaPlan {
   static constexpr int SPC = TCW + 2;            // staging row pitch (complex): the tile and a one-column shift
   static constexpr int STAGE = N * SPC * 8;      // bytes of the staged input tile
   static constexpr int THREADS = 256;            // 8 warps; 512 stage-A items (64 n1 x 8 column groups), 2 each
-  static constexpr int CTAS_PER_SM = 2;
   static constexpr int A_PART = 128 * 64 * 2;    // f16 128 x 64 operand
   static constexpr int B_PART = 64 * 128 * 2;    // f16 64 (K) x 128 (MN) operand
   static constexpr int TMEM_COLS = 128;          // one 128-column accumulator
-  static constexpr int SMEM = 1024 + 2 * A_PART + 2 * B_PART + STAGE;
+  static constexpr int USED = 1024 + 2 * A_PART + 2 * B_PART + STAGE;
+  static constexpr int SMEM = USED > 116 * 1024 ? USED : 116 * 1024;   // more than half an SM's 228 KB
 };
 
 constexpr int kTmaMaxBoxes = 64;   // boxes per staged tile (N / 8 at most)
@@ -153,7 +154,7 @@ __device__ __forceinline__ int tma_col(const TmaArgs &a, int kx) {
 }
 
 template <int N, bool INV>
-__global__ void __launch_bounds__(TmaPlan<N>::THREADS, TmaPlan<N>::CTAS_PER_SM)
+__global__ void __launch_bounds__(TmaPlan<N>::THREADS, 1)
     k_strided_tma(const __grid_constant__ TmaArgs a, const __half *__restrict__ Adft, int *status) {
   using C = float2;
   using PL = TmaPlan<N>;
