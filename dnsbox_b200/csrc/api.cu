@@ -1593,11 +1593,11 @@ extern "C" int dnsbox_eband(dnsbox_ctx *ctx, const void *uh, double *eband) {
 template <typename T> static int state_to_phys(dnsbox_ctx *ctx, const void *uh, double scale, void **phys) {
   const void *in[3];
   void *out[3];
-  // the c2r passes use W1 slots 0-2 and W2 slots 0-2; the physical output goes
-  // to W1 slots 3-5 (each real field needs half a complex field's bytes)
+  // the c2r passes use W1 and W2 slots 0-2; the physical output goes to W1 slots
+  // 3-5 (each real field needs half a complex field's bytes)
   for (int f = 0; f < 3; ++f) {
     in[f] = cfield(reinterpret_cast<const char *>(uh), ctx, f);
-    out[f] = field(ctx->W1, ctx, 3 + f);
+    out[f] = wfield(ctx->W1, ctx, 3 + f);
     phys[f] = out[f];
   }
   return c2r_fields<T>(ctx, 3, in, out, scale);
