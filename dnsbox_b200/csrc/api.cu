@@ -574,7 +574,6 @@ template <typename T> static FinishArgs<T> finish_base(const dnsbox_ctx *c) {
   FinishArgs<T> f;
   memset(&f, 0, sizeof(f));
   const dnsbox_params &p = c->p;
-  f.tw = reinterpret_cast<const typename CT<T>::type *>(c->tw[2]);
   f.nh = (long long)c->nh;
   f.nx = p.nx;
   f.ny = p.ny;
@@ -681,7 +680,6 @@ static int run_rhs(dnsbox_ctx *c, const void *uin, int mode, void *out, void *st
   x.lines_per_box = x.box_lines = p.ny * p.nz;
   x.nlines = c->nbatch * p.ny * p.nz;
   x.nxh = c->nxh;
-  x.alpha_x = p.alpha_x;
   x.s = s;
   if (pruned) x.kxa = c->keep[0].a;   // read only kept kx; write only kx the finish keeps
   {
@@ -739,7 +737,6 @@ static int run_rhs(dnsbox_ctx *c, const void *uin, int mode, void *out, void *st
   e.nu_box = c->d_nu;
   e.nh = (long long)c->fstride;
   e.bstride = (long long)c->nh;
-  e.mode = mode;
   e.kx = pruned ? c->keep[0] : AxisKeep{0, p.nx, 0};
   e.ky = pruned ? c->keep[1] : AxisKeep{0, p.ny, 1};
   e.kz = pruned ? c->keep[2] : AxisKeep{0, p.nz, 1};

@@ -75,7 +75,6 @@ struct dnsbox_ctx {
   int *band = nullptr;                   // band-mode index triples
   int nband = 0;
   dnsbox_diag *ddiag = nullptr;          // device per-step records
-  int ddiag_cap = 0;
   double *hstage = nullptr;              // pinned host staging (8 doubles)
   int nspec = 0;
   int ab2_started = 0;
@@ -314,15 +313,6 @@ static inline int ensure_red(dnsbox_ctx *c, size_t ndoubles) {
   c->red = nullptr;
   CK(cudaMalloc(&c->red, ndoubles * sizeof(double)));
   c->red_cap = ndoubles;
-  return DNSBOX_OK;
-}
-
-static inline int ensure_diag(dnsbox_ctx *c, int n) {
-  if (n <= c->ddiag_cap) return DNSBOX_OK;
-  if (c->ddiag) cudaFree(c->ddiag);
-  c->ddiag = nullptr;
-  CK(cudaMalloc(&c->ddiag, (size_t)n * sizeof(dnsbox_diag)));
-  c->ddiag_cap = n;
   return DNSBOX_OK;
 }
 

@@ -527,7 +527,6 @@ template <typename T> struct XlineNLArgs {
   int pin, pout;                       // row pitch (complex elements) of the inputs / outputs; 0: nxh
   int npad;                            // compact rows: slots after nyq that complete its 32-byte sector (written as 0)
   int nyq;                             // slot of the Nyquist column in a row (kxa in compact workspace rows); 0: N/2
-  double alpha_x;
   double s;                            // scalemodes
 };
 
@@ -1798,7 +1797,6 @@ template <typename T> struct FinishArgs {
   const StepState *st;     // per-box step state (blockIdx.y)
   const double *nu_box;    // per-box viscosity or null (use nu)
   double *partials;        // per-CTA (E, D) of the new state, or null; gridDim.x pairs per box
-  const C *tw;
   long long nh;            // elements between components (all boxes of one component)
   long long bstride;       // elements between boxes
   int nx, ny, nz, nxh;
@@ -1806,7 +1804,7 @@ template <typename T> struct FinishArgs {
   double nu, Q, Pin;
   double kcut2;            // largest k.k whose root is at most kCutOff (kcut2_of)
   double cutx, cuty, cutz, sph2;
-  int bandlim, spherical, mode, ab2_standard;
+  int bandlim, spherical, ab2_standard;
   double s;                // scalemodes
   AxisKeep kx, ky, kz;     // pruning: only kept (kz, ky) rows and kept kx modes are visited
   // layout of n3 when it is a padded workspace field: row pitch, elements

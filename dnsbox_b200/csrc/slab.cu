@@ -390,7 +390,6 @@ int rhs_middle(dnsbox_slab *s, const void *recv5, double *umax, void *send3, cud
   x.box_lines = s->ny * s->nz;
   x.nlines = s->ny * s->nzl;
   x.nxh = s->nxh;
-  x.alpha_x = s->p.alpha_x;
   x.s = sc;
   cudaError_t e = Ops<T>::xline_nl(s->nx, x, 0, st);
   if (e != cudaSuccess) return set_err(DNSBOX_ERR_CUDA, "slab x pass: %s", cudaGetErrorString(e));
@@ -427,7 +426,6 @@ int rhs_finish(dnsbox_slab *s, const void *recv3, const void *uh, const double *
   f.state = reinterpret_cast<C *>(state);
   f.partials = rows;
   f.st = s->st;
-  f.tw = reinterpret_cast<const C *>(s->tw[2]);
   f.nh = (long long)slab_field(s);
   f.nx = s->nx;
   f.ny = s->nyl;
@@ -449,7 +447,6 @@ int rhs_finish(dnsbox_slab *s, const void *recv3, const void *uh, const double *
   f.bandlim = p.bandlim;
   f.spherical = p.spherical;
   f.s = 1.0 / ((double)s->nx * s->ny * s->nz);
-  f.mode = mode;
   f.kx = AxisKeep{0, s->nx, 0};
   f.ky = AxisKeep{0, s->nyl, 1};
   f.kz = AxisKeep{0, s->nz, 1};
