@@ -18,7 +18,7 @@ of writing a file.  Its functions then produce, on seeded fields:
 Outputs are stored as half spectra in the [kz, ky, kx] layout.  Run in this
 container only (it reads the reference tree); the .npz files are committed.
 
-    python tests/golden/make_golden.py /root/reference/python/dnsbox.py
+    python tests/golden/make_golden.py <path to the reference's python/dnsbox.py>
 """
 from __future__ import annotations
 
