@@ -612,16 +612,18 @@ static int run_rhs(dnsbox_ctx *c, const void *uin, int mode, void *out, void *st
   const bool compact = pruned && strided_simt<T>(c);
   const int wp = ws_pitch(c, compact);
   // rhs_Eband (rhs.f90:22-24): a block of pass A where that runs the SIMT
-  // kernel on workspace rows and has a thread for every eight modes of the band,
-  // else a launch of 256 threads of its own.  Step, us, in pass A / launched: 32^3
-  // FP32 (32 threads) 112 modes 41.9 / 45.9, 208 45.0 / 45.9, 500 54 / 47, 2952 128 /
-  // 59; 64^3 FP64 (64) 500 modes 65.7 / 67.3, 1136 76 / 71; 256^3 FP32 (128) 1136 845 /
-  // 845, 2952 874 / 860; 64 x 64 x 8 (8) 44 modes 47.5 / 47.2, 112 54 / 47, 1532 201 / 53.
+  // kernel on workspace rows with whole warps and has a thread for every 16 modes
+  // of the band, else a launch of 256 threads of its own.  Step, us, in pass A /
+  // launched: 32^3 FP32 (32 threads) 112 modes 40.2 / 42.9, 500 43.3 / 47.1, 1136 50.2 /
+  // 49.6, 2952 69 / 58; 64^3 FP64 (64) 500 modes 61.2 / 67.7, 2952 78 / 79; 256^3 FP32
+  // (128) 112 modes 829.6 / 834.9, 1136 843 / 844, 2952 873 / 860; 64 x 64 x 8 (8
+  // threads) 44 modes 45.7 / 45.6, 112 49 / 45, 1532 129 / 53.
   auto simt = [&](int i, int n) {
     return (!c->tc || !Ops<T>::has_tc(n) || c->sched_tc[i] == 2) && (!pruned || compact);
   };
   const bool band = p.bandlim && c->nband;
-  const bool band_in_a = band && simt(0, p.nz) && c->nband <= 8 * Ops<T>::strided_threads(p.nz);
+  const int bthreads = Ops<T>::strided_threads(p.nz);
+  const bool band_in_a = band && simt(0, p.nz) && bthreads >= 32 && c->nband <= 16 * bthreads;
   if (band && !band_in_a) {
     Prof pr(c, DNSBOX_PASS_SMALL);
     CK(launch_pdl(k_eband<C>, c->nbatch, 256, 0, c->stream, band_args(c, uin), p.nx, 0));

@@ -153,12 +153,12 @@ struct Prof {
 
 // ------------------------------------------------------------ shared kernels
 // rhs_Eband (rhs.f90:137-168) over the precomputed band-mode list; optionally
-// resets the CFL maxima.  One block per box.
+// resets the CFL maxima.  One block of 256 threads per box.
 template <typename C> __global__ void k_eband(BandArgs b, int nx, int reset_umax) {
-  __shared__ double red[kBandRed];
+  __shared__ double red[kBandRed / 32];
   pdl_launch();
   pdl_wait();
-  eband_block<C>(b, nx, blockIdx.x, reset_umax, red);
+  eband_block<C, 256>(b, nx, blockIdx.x, reset_umax, red);
 }
 
 // Sum of n doubles in a fixed order (one block).

@@ -98,12 +98,13 @@ struct BandArgs {
   const void *u;    // the right-hand side's input, components nh apart, boxes bstride apart
   long long nh, bstride;
 };
-// rhs_Eband (rhs.f90:137-168) of box `box` by one block (red: kBandRed doubles);
-// optionally resets the CFL maxima.  256 partial sums (modes j, j + 256, ..) and
-// a fixed tree over them, whatever the number of threads: the band energy is
-// one number, of a block of its own and of a tail block of any pass A.
+// rhs_Eband (rhs.f90:137-168) of box `box` by a block of NT threads, a power of
+// two from 32 on (red: a double per 32 sums); optionally resets the CFL maxima.  256 partial
+// sums (modes j, j + 256, ..) and a fixed tree over them, whatever the number of
+// threads: the band energy is one number, of a block of its own and of a tail
+// block of any pass A.
 constexpr int kBandRed = 256;
-template <typename C>
+template <typename C, int NT>
 __device__ __forceinline__ void eband_block(const BandArgs &b, int nx, int box, bool reset_umax, double *red) {
   const C *u = reinterpret_cast<const C *>(b.u) + (long long)box * b.bstride;
   StepState *st = b.st + box;
@@ -118,30 +119,37 @@ __device__ __forceinline__ void eband_block(const BandArgs &b, int nx, int box, 
     }
     return e;
   };
-  // thread t of nt (a divisor of 256) owns the sums t, t + nt, ..; four modes in flight
-  const int nt = min((int)blockDim.x, kBandRed), t = threadIdx.x;
-  if (t < nt) {
-    for (int j = t; j < kBandRed; j += nt) red[j] = 0.0;
-    for (int i = t; i < b.n; i += 4 * nt) {
-      double e[4];
+  // thread t of P owns the sums t, t + P, .., in registers; a warp's shuffles add
+  // 32 neighbouring ones
+  constexpr int P = NT < kBandRed ? NT : kBandRed, M = kBandRed / P, Q = M < 4 ? M : 4;   // Q modes in flight
+  static_assert(P >= 32 && kBandRed % P == 0, "whole warps");
+  const int t = threadIdx.x;
+  if (t < P) {
+    double s[M];
 #pragma unroll
-      for (int m = 0; m < 4; ++m) e[m] = i + m * nt < b.n ? energy(i + m * nt) : 0.0;
+    for (int m = 0; m < M; ++m) s[m] = 0.0;
+    for (int i = t; i < b.n; i += kBandRed)
 #pragma unroll
-      for (int m = 0; m < 4; ++m) red[(i + m * nt) % kBandRed] += e[m];
+      for (int q = 0; q < M; q += Q) {
+        if (i - t + q * P >= b.n) break;
+        double e[Q];
+#pragma unroll
+        for (int m = 0; m < Q; ++m) e[m] = energy(min(i + (q + m) * P, b.n - 1));
+#pragma unroll
+        for (int m = 0; m < Q; ++m)
+          if (i + (q + m) * P < b.n) s[q + m] += e[m];
+      }
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const int g = t / 32 + m * (P / 32);
+      if (32 * g < b.n) s[m] = warp_sum(s[m]);   // else zeros
+      if (t % 32 == 0) red[g] = s[m];
     }
   }
   __syncthreads();
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {   // each 32 sums
-    for (int j = threadIdx.x; j < kBandRed / 32 * o; j += blockDim.x) {
-      double *r = red + j / o * 32 + j % o;
-      r[0] += r[o];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
+  if (t == 0) {
     for (int o = kBandRed / 64; o; o >>= 1)
-      for (int j = 0; j < o; ++j) red[32 * j] += red[32 * (j + o)];
+      for (int j = 0; j < o; ++j) red[j] += red[j + o];
     st->eband = red[0] * b.s2;
     if (reset_umax) st->umax[0] = st->umax[1] = st->umax[2] = 0.0;
   }
@@ -250,7 +258,7 @@ template <typename T, int N> struct StridedShape {
   static constexpr size_t tile = PL::NST > 1 ? (size_t)N * W * 16 : 0;
   static constexpr size_t smem(bool inv) {   // tile, twiddles and (inverse) row multipliers
     const size_t n = tile + (size_t)vtw_size<PL>() * 16 + (inv ? 2 * N * sizeof(T) : 0);
-    return n < kBandRed * sizeof(double) ? kBandRed * sizeof(double) : n;   // the band block's sums
+    return n < kBandRed / 32 * sizeof(double) ? kBandRed / 32 * sizeof(double) : n;   // the band block's sums
   }
   // Resident CTAs asked of the register allocator: 16 warps per SM where a
   // thread holds 16 values (128 registers), 20 at 12 (96), 24 at 8 (80).  The
@@ -390,10 +398,10 @@ __global__ void __launch_bounds__(StridedShape<T, N>::NT, StridedShape<T, N>::mi
   V *twt = reinterpret_cast<V *>(smem_raw + SH::tile);
   T *bks = reinterpret_cast<T *>(smem_raw + SH::tile + (size_t)vtw_size<PL>() * 16);
   pdl_launch();
-  if constexpr (INV && MODE == ST_TO_WS) {
+  if constexpr (INV && MODE == ST_TO_WS && SH::NT >= 32) {
     if (a.band.n && blockIdx.x == gridDim.x - 1) {
       pdl_wait();
-      eband_block<C>(a.band, a.nx, blockIdx.y, false, reinterpret_cast<double *>(smem_raw));
+      eband_block<C, SH::NT>(a.band, a.nx, blockIdx.y, false, reinterpret_cast<double *>(smem_raw));
       return;
     }
   }

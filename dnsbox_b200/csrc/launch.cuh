@@ -79,7 +79,7 @@ cudaError_t Launcher<T, N>::strided(const StridedArgs<T> &a, bool inv, int ntile
   // workspace to workspace, forward: workspace to either); pruned columns need
   // the compact workspace
   const int ws = a.kcol.a && !a.compact ? 0 : a.ws;
-  if ((a.band.n && !(inv && ws == 2)) || (a.cfl.on && (inv || ws != 3))) return cudaErrorInvalidValue;
+  if ((a.band.n && !(inv && ws == 2 && strided_threads() >= 32)) || (a.cfl.on && (inv || ws != 3))) return cudaErrorInvalidValue;
   if (inv) {
     if (ws == 3) return strided_launch<T, N, true, ST_WS>(a, nb, st);
     if (ws == 2) return strided_launch<T, N, true, ST_TO_WS>(a, nb, st);
