@@ -163,6 +163,17 @@ cudaError_t Launcher<T, N>::strided_tma(const TmaArgs &a, bool inv, const void *
 
 template <typename T, int N> bool Launcher<T, N>::has_xline_warp() { return XlineWarp<T, N>::on; }
 
+// Threads of an x-line block of up to nt, P to a sequence: smaller blocks where
+// the sequences are few, so that each of the 148 SMs gets four, for sequences of
+// up to 8 threads.  Halved against not, us: step 32^3 FP32 39.1 / 40.2, 48^3 57.0 / 58.7;
+// transposed term 48^3 35.6 / 37.2, 64^3 FP64 38.6 / 38.7; C2R 24^3 5.6 / 6.4, 64^3 6.4 /
+// 7.0.  With 16 and 32 threads a sequence it loses: step 256 x 16 x 16 48.4 / 45.6,
+// 128 x 32 x 32 FP64 59.1 / 58.4, 512 x 16 x 16 57.2 / 56.4.
+static inline int xline_threads(int P, int nt, long long sequences) {
+  while (P <= 8 && nt > 32 && sequences * P < 148LL * 4 * nt) nt >>= 1;
+  return nt;
+}
+
 template <typename T, int N>
 cudaError_t Launcher<T, N>::xline_nl(const XlineNLArgs<T> &a, int variant, cudaStream_t st) {
   using C = typename CT<T>::type;
@@ -184,9 +195,7 @@ cudaError_t Launcher<T, N>::xline_nl(const XlineNLArgs<T> &a, int variant, cudaS
   }
   if constexpr (XReg<T, N>::on) {   // whatever the choice
     using SH = XReg<T, N>;
-    // few lines: smaller blocks, so that every SM gets some
-    int nt = SH::NT;
-    while (nt > 32 && (long long)a.nlines * SH::PL::P < 148LL * 4 * nt) nt >>= 1;
+    const int nt = xline_threads(SH::PL::P, SH::NT, a.nlines);
     const int lpb = nt / SH::PL::P;
     if ((e = set_smem(k_xline_nl_g<T, N>, SH::smem(nt))) != cudaSuccess) return e;
     return launch_pdl(k_xline_nl_g<T, N>, (unsigned)((a.nlines + lpb - 1) / lpb), nt, SH::smem(nt), st, a);
@@ -216,8 +225,7 @@ template <typename T, int N>
 cudaError_t Launcher<T, N>::xline_vjp(const XlineVjpArgs<T> &a, cudaStream_t st) {
   if constexpr (XReg<T, N>::on) {
     using SH = XReg<T, N>;
-    int nt = SH::NT;   // pairs of lines: at least two in a block
-    while (nt > 32 && nt > 2 * SH::PL::P && (long long)a.nlines * SH::PL::P < 148LL * 4 * nt) nt >>= 1;
+    const int nt = xline_threads(SH::PL::P, SH::NT, a.nlines);   // an even number of lines
     const int lpb = nt / SH::PL::P;
     const cudaError_t e = set_smem(k_xline_vjp<T, N>, SH::smem(nt));
     if (e != cudaSuccess) return e;
@@ -228,17 +236,10 @@ cudaError_t Launcher<T, N>::xline_vjp(const XlineVjpArgs<T> &a, cudaStream_t st)
   }
 }
 
-// Threads of a plain x-line block: smaller blocks where the lines are few.
-template <typename T, int N> static int xplain_threads(const XlineArgs<T> &a, int nf) {
-  int nt = XPlain<T, N>::NT;
-  while (nt > 32 && (long long)nf * a.nlines * XPlain<T, N>::PL::P < 2 * 148LL * 4 * nt) nt >>= 1;
-  return nt;
-}
-
 template <typename T, int N>
 cudaError_t Launcher<T, N>::xline_c2r(const XlineArgs<T> &a, int nf, cudaStream_t st) {
   using SH = XPlain<T, N>;
-  const int nt = xplain_threads<T, N>(a, nf), lpb = 2 * (nt / SH::PL::P);
+  const int nt = xline_threads(SH::PL::P, SH::NT, (long long)nf * a.nlines / 2), lpb = 2 * (nt / SH::PL::P);
   const cudaError_t e = set_smem(k_xline_c2r<T, N>, SH::smem(nt));
   if (e != cudaSuccess) return e;
   return launch_pdl(k_xline_c2r<T, N>, dim3((unsigned)((a.nlines + lpb - 1) / lpb), (unsigned)nf), nt, SH::smem(nt), st, a);
@@ -247,7 +248,7 @@ cudaError_t Launcher<T, N>::xline_c2r(const XlineArgs<T> &a, int nf, cudaStream_
 template <typename T, int N>
 cudaError_t Launcher<T, N>::xline_r2c(const XlineArgs<T> &a, int nf, cudaStream_t st) {
   using SH = XPlain<T, N>;
-  const int nt = xplain_threads<T, N>(a, nf), lpb = 2 * (nt / SH::PL::P);
+  const int nt = xline_threads(SH::PL::P, SH::NT, (long long)nf * a.nlines / 2), lpb = 2 * (nt / SH::PL::P);
   const cudaError_t e = set_smem(k_xline_r2c<T, N>, SH::smem(nt));
   if (e != cudaSuccess) return e;
   return launch_pdl(k_xline_r2c<T, N>, dim3((unsigned)((a.nlines + lpb - 1) / lpb), (unsigned)nf), nt, SH::smem(nt), st, a);
