@@ -293,3 +293,19 @@ def test_band_energy_of_every_path(nz, kcut):
     assert full.step(v, 1)[0]["eband"] == want and not full.step_pruned()
     b.close()
     full.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("ny,nz", [(8, 8), (12, 96), (96, 128)])
+@pytest.mark.parametrize("nx", [8, 12])
+def test_transforms_of_short_lines(nx, ny, nz, prec):
+    """R2C and C2R whose x lines are two lanes wide, against pocketfft (the round-off bars of the slab transforms)."""
+    from dnsbox_b200.ops import Box
+    g = O.Grid(O.Params(nx=nx, ny=ny, nz=nz))
+    f = np.random.default_rng(nx).standard_normal((nz, ny, nx))
+    b = Box(nx=nx, ny=ny, nz=nz, precision=prec)
+    tol = 1e-13 if prec == "fp64" else 8e-7
+    spec = b.r2c(torch.from_numpy(f).to("cuda", b.zeros().dtype.to_real()))
+    assert rel(spec.cpu().numpy(), g.r2c(f)) < tol
+    assert rel(b.c2r(spec).cpu().numpy(), f * (nx * ny * nz)) < tol
+    b.close()
