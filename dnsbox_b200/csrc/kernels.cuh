@@ -378,8 +378,8 @@ enum StridedMode : int {
 // FFT the same loads and stores take 67 / 125 / 56 / 35 us (A, B, D, E1,
 // 256^3 FP32, padded rows with the kept columns first) and the pass takes
 // 76 / 135 / 57 / 39; compact rows, written in whole sectors, bring it to
-// 63 / 111 / 48 / 32 (one 8-byte column per thread: 77 / 148 / 63 / 43), FP64
-// from 111 / 248 / 94 / 67 to 101 / 197 / 75 / 54.
+// 61 / 109 / 45 / 31 (one 8-byte column per thread: 77 / 148 / 63 / 43), FP64
+// from 111 / 248 / 94 / 67 to 99 / 191 / 74 / 54.
 template <typename T, int N, bool INV, int MODE>
 __global__ void __launch_bounds__(StridedShape<T, N>::NT, StridedShape<T, N>::minb)
     k_strided(const __grid_constant__ StridedArgs<T> a) {
@@ -1007,9 +1007,9 @@ template <typename T, int N> struct XReg {
 // Hermitian mirror's, which goes to the lane that holds row N - n by shuffle.
 // Against the block kernel (fields in shared memory, bank conflicts) and the
 // warp kernels it replaces, us: 32 boxes of 64^3 FP32 150 -> 73, of 32^3 29 -> 17,
-// 128^3 56 -> 25, 256^3 162 -> 130 (FP64 397 -> 325), 512^3 1698 -> 1285.  At 256 in
-// FP32 it is balanced: issue 57-60%, FMA pipe 50%, L1 61-65%, 12 warps by registers;
-// FP64 is bound by L1 (82-87%), the exchanges.  All loads of a line up front (the
+// 128^3 56 -> 25, 256^3 162 -> 131 (FP64 397 -> 326), 512^3 1698 -> 1285.  At 256 in
+// FP32 it is balanced: issue 57-60%, FMA pipe 50%, L1 60-64%, 12 warps by registers;
+// FP64 is bound by L1 (82-88%), the exchanges.  All loads of a line up front (the
 // third sequence's during the pair's transform) brought 179 -> 140 at 256.
 template <typename T, int N>
 __global__ void __launch_bounds__(XReg<T, N>::NT, XReg<T, N>::minb)
@@ -1214,8 +1214,8 @@ __global__ void __launch_bounds__(XReg<T, N>::NT, XReg<T, N>::minb)
 // forward transforms' first stage; R1 lanes a line finish and store.  The tile
 // rows are skewed by row / R of the stage that writes them (16-byte accesses
 // of every stage free of bank conflicts at the pitches of SplitPlan).  Against
-// k_xline_nl_g, us: 32 boxes of 96^3 FP32 285 -> 250 (L1 87% -> 67-75%, now bound by
-// load latency and the block's barriers), 192^3 FP32 78 -> 64, FP64 156 -> 144.
+// k_xline_nl_g, us: 32 boxes of 96^3 FP32 285 -> 253 (L1 87% -> 67-75%, now bound by
+// load latency and the block's barriers), 192^3 FP32 77 -> 68, FP64 165 -> 148.
 template <typename T, int N> struct XSplit {
   using SP = SplitPlan<N>;
   static constexpr int L = 8, PO = SP::R1, PI = SP::R0, NT = L * (PO > PI ? PO : PI);

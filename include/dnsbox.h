@@ -332,7 +332,9 @@ int dnsbox_adjoint_descent(dnsbox_ctx *ctx, void *uhat3_dev, int niter, double *
 int dnsbox_heun_step_vjp(dnsbox_ctx *ctx, const void *uhat3_dev, const void *g3_dev, void *out3_dev);
 /* g0 = (S^nsteps)'(u0)^T gT, with the states recomputed per segment from
  * checkpoints taken every `every` steps (device memory: nsteps/every + every + 2
- * states, held by the context).  uT3_dev (may be NULL) receives u(T). */
+ * states, held by the context).  uT3_dev (may be NULL) receives u(T).  The clock
+ * and the step records (dnsbox_diag_read) count the nsteps forward steps, then each
+ * segment's recomputed ones, the last segment first. */
 int dnsbox_heun_steps_vjp(dnsbox_ctx *ctx, const void *u0_3_dev, int nsteps, int every, const void *gT3_dev,
                           void *g0_3_dev, void *uT3_dev);
 /* J = 1/2 <|u(T) - u0|^2> (mean square over the physical grid, FP64) with
