@@ -99,10 +99,10 @@ struct BandArgs {
   long long nh, bstride;
 };
 // rhs_Eband (rhs.f90:137-168) of box `box` by a block of NT threads, a power of
-// two from 32 on (red: a double per 32 sums); optionally resets the CFL maxima.  256 partial
-// sums (modes j, j + 256, ..) and a fixed tree over them, whatever the number of
-// threads: the band energy is one number, of a block of its own and of a tail
-// block of any pass A.
+// two from 32 on (red: a double per 32 sums); optionally resets the CFL maxima.
+// 256 partial sums (modes j, j + 256, ..) and a fixed tree over them, whatever the
+// number of threads: the band energy is one number, of a block of its own and of
+// a tail block of any pass A.
 constexpr int kBandRed = 256;
 template <typename C, int NT>
 __device__ __forceinline__ void eband_block(const BandArgs &b, int nx, int box, bool reset_umax, double *red) {
@@ -1206,8 +1206,8 @@ __global__ void __launch_bounds__(XReg<T, N>::NT, XReg<T, N>::minb)
   }
 }
 
-// The fused x pass of 96- (FP32) and 192-point lines of large boxes: k_xline_nl_g with split plans
-// (SplitPlan), so that each transform exchanges once, not twice, through the
+// The fused x pass of 96- (FP32) and 192-point lines of large boxes (the rule
+// stands at the launch): k_xline_nl_g with split plans (SplitPlan), so that each transform exchanges once, not twice, through the
 // shared memory that bounds it.  A block of 8 lines: R1 lanes a line load,
 // form the sequences and run the inverse transforms' first stage; after one
 // barrier R0 lanes a line run the second stage, form the products and run the
@@ -1936,7 +1936,7 @@ __global__ void __launch_bounds__(256, FinishMinB<T, MODE>::v)
       const int kx = column(s0 + 32 * h, unused);
       const long long idx = rowbase + kx;
       const double kxr = k_half(kx, a.nx, a.ax);
-    const double wk = (kxr == 0.0) ? 0.5 : 1.0;   // state.f90:436-440
+      const double wk = (kxr == 0.0) ? 0.5 : 1.0;   // state.f90:436-440
       const double k2 = kxr * kxr + kyr * kyr + kzr * kzr;
       const bool zero = (kxr == 0.0) && (kyr == 0.0) && (kzr == 0.0);
       const bool cut = (a.spherical && k2 >= a.sph2) || fabs(kxr) >= a.cutx || rowcut || zero;
